@@ -607,7 +607,7 @@ __device__ __forceinline__ void strip_state(const MP& m, const Grid& g, int side
       double Yi[NR];
 #pragma unroll
       for (int k = 0; k < NR; ++k) Yi[k] = g.Yinj[k * g.nx + pos];
-      injector_state(m, q, gamma, T, Yi, g.inj_block_p, gs);
+      injector_state<false>(m, q, gamma, T, Yi, g.inj_block_p, gs);
       return;
     }
   }

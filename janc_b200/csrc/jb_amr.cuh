@@ -85,11 +85,19 @@ __device__ __forceinline__ void amr_eYR(const MP& m, const double* Ub, long long
                                         double* Yf, double& R) {
   constexpr int nY = 4;
   const double rho = Ub[c];
+  double Y8[NR];
+#if JB_FAST
+  const double ri = 1.0 / rho;
+  const double u = Ub[nc + c] * ri, v = Ub[2 * nc + c] * ri;
+  e = Ub[3 * nc + c] * ri - 0.5 * (u * u + v * v);
+#pragma unroll
+  for (int k = 0; k < NR; ++k) Y8[k] = Ub[(nY + k) * nc + c] * ri;
+#else
   const double u = Ub[nc + c] / rho, v = Ub[2 * nc + c] / rho;
   e = Ub[3 * nc + c] / rho - 0.5 * (u * u + v * v);
-  double Y8[NR];
 #pragma unroll
   for (int k = 0; k < NR; ++k) Y8[k] = Ub[(nY + k) * nc + c] / rho;
+#endif
   fill_Y(Y8, Yf);
   R = get_R(m, Yf);
 }
@@ -218,9 +226,17 @@ __global__ void __launch_bounds__(AMR_NT, JB_AMR_MINB) k_amr_stage(MP m, Grid g,
         const long long gc = (long long)bxp * PY + byp;
         const bool in = bxp < PX && byp < PY;
         const double qf = in ? gU[f * nc + gc] : 1.0;
+        const double al = dir == 0 ? ax : ay;
+#if JB_FAST
+        // F = vel q + pressure terms: the reference's LF flux regrouped
+        const double vel = sP[(1 + dir) * AQ + c];
+        double F = vel * qf;
+        if (f == 1 + dir) F += sP[3 * AQ + c];
+        if (f == 3) F += vel * sP[3 * AQ + c];
+#else
         const double E = in ? gU[3 * nc + gc] : 1.0;
         const double F = lf_flux<2>(f, dir, qf, sP[c], sP[AQ + c], sP[2 * AQ + c], sP[3 * AQ + c], E);
-        const double al = dir == 0 ? ax : ay;
+#endif
         const double hp = 0.5 * (F + al * qf), hm = 0.5 * (F - al * qf);
         if (dir == 0) { sHxp[px * TY + (py - 3)] = hp; sHxm[px * TY + (py - 3)] = hm; }
         else { sHyp[(px - 3) * APY + py] = hp; sHym[(px - 3) * APY + py] = hm; }
@@ -281,28 +297,106 @@ __global__ void __launch_bounds__(AMR_NT, JB_AMR_MINB) k_amr_stage(MP m, Grid g,
     }
   }
   if (!(ax == ax) || !(ay == ay)) st |= JB_ERR_NONFINITE;
+#if !JB_FAST
   if (STAGE > 0) {
     __syncthreads();
-    // ---- update_aux of the padded block from G's temperatures
+    // ---- update_aux of the padded block from G's temperatures (the fast
+    // variants' launcher runs k_amr_update_cells on the result instead)
     amr_update_block(m, oU, gA + nc, io.oA + b * io.osA, nc, st);
   }
+#endif
   st = amr_block_or(st);
   if (tid == 0 && st) atomicOr(&slots->status, st);
 }
 
 // update_aux of every block (vmap(update_aux), set_simulator.py:41) with
 // each block's own stop: U [nb][nv][X][Y] (field stride nc, block stride
-// su), aux_in / aux_out [nb][2][X][Y] (block stride sa).
+// su), aux_in / aux_out [nb][2][X][Y] (block strides sai, sao).
 template <int UNUSED>
 __global__ void __launch_bounds__(AMR_NT) k_amr_update(MP m, long long nc, const double* U, long long su,
-                                                     const double* aux_in, double* aux_out, long long sa,
-                                                     Slots* slots) {
+                                                     const double* aux_in, long long sai, double* aux_out,
+                                                     long long sao, Slots* slots) {
   const long long b = blockIdx.x;
   unsigned st = 0;
-  amr_update_block(m, U + b * su, aux_in + b * sa + nc, aux_out + b * sa, nc, st);
+  amr_update_block(m, U + b * su, aux_in + b * sai + nc, aux_out + b * sao, nc, st);
   st = amr_block_or(st);
   if (threadIdx.x == 0 && st) atomicOr(&slots->status, st);
 }
+
+#if JB_FAST
+// The same with each thread's CPT cells held in registers across the rounds:
+// energy, gas constant, temperature and the six coefficients of the mixture
+// enthalpy (mix_h; every species switches NASA7 ranges at the same
+// temperature), so a round is one Horner pass and one block-wide vote
+// instead of the species sums over a state read again.  676-cell padded
+// blocks (20 x 20 + ghosts), 300 of them: half of the stage's 160 us before.
+constexpr int AMR_UNT = 512, AMR_UCPT = 4;  // blocks of up to 2048 cells
+template <int CPT>
+__global__ void __launch_bounds__(AMR_UNT) k_amr_update_cells(MP m, long long nc, const double* U, long long su,
+                                                           const double* aux_in, long long sai, double* aux_out,
+                                                           long long sao, Slots* slots) {
+  const long long b = blockIdx.x;
+  const double* Ub = U + b * su;
+  const double* T0 = aux_in + b * sai + nc;
+  double* Ab = aux_out + b * sao;
+  const double Tcr = m.Tcr[0];
+  double T[CPT], e[CPT], R[CPT], H[CPT][6], cp[CPT];
+  unsigned lo = 0, st = 0;
+  auto cell = [&](int k) { return (long long)threadIdx.x + (long long)k * blockDim.x; };
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) {
+    const long long c = cell(k);
+    if (c < nc) {
+      double Yf[NS];
+      amr_eYR(m, Ub, nc, c, e[k], Yf, R[k]);
+      T[k] = T0[c];
+      if (T[k] < Tcr) lo |= 1u << k;
+      mix_h(m, Yf, T[k] < Tcr, H[k]);
+    }
+  }
+  for (int i = 0;; ++i) {
+    double Tn[CPT];
+    unsigned bits = 0;
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      if (cell(k) < nc) {
+        double h, dcp;
+        poly6_d2(H[k], T[k], h, cp[k], dcp);
+        const double res = (h - R[k] * T[k]) - e[k], d1 = cp[k] - R[k];
+        if (fabs(res) > HALLEY_TOL) bits |= 1u;
+        if (res != res) bits |= 2u;
+        Tn[k] = T[k] + ((-2.0 * res) * d1) / ((2.0 * (d1 * d1)) - res * dcp);
+      }
+    }
+    const int go = __syncthreads_or(bits & 1u), bad = __syncthreads_or(bits & 2u);
+    if (!go || bad || i == HALLEY_MAX) break;
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      const long long c = cell(k);
+      if (c < nc) {
+        T[k] = Tn[k];
+        if ((T[k] < Tcr) != (bool)((lo >> k) & 1u)) {  // the iterate crossed the range boundary (rare)
+          lo ^= 1u << k;
+          double ek, Yf[NS], Rk;
+          amr_eYR(m, Ub, nc, c, ek, Yf, Rk);
+          mix_h(m, Yf, T[k] < Tcr, H[k]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) {
+    const long long c = cell(k);
+    if (c < nc) {
+      Ab[c] = cp[k] / (cp[k] - R[k]);
+      Ab[nc + c] = T[k];
+      if (!(T[k] == T[k])) st |= JB_ERR_NONFINITE;
+    }
+  }
+  st = amr_block_or(st);
+  if (threadIdx.x == 0 && st) atomicOr(&slots->status, st);
+}
+#endif
 
 // Chemistry of every cell of nb unpadded blocks (the vmapped
 // reaction_source_terms of set_simulator.py:109-111): out = U + S(U, T, dt),

@@ -40,7 +40,7 @@ struct jb_handle {
   // adjoint support
   double base_A[JB_NREAC_MAX];  // pre-exponential factors as created (jb_set_log_A_offset)
   int probe[4];                 // x0, y0, wx, wy of the pressure probe (wx*wy = 0: none)
-  void* fwork;                  // mixed 2D flux scratch (float32 primitives, x flux differences)
+  void* fwork;                  // 2D flux scratch (primitives, x flux differences: sweep_work)
   jb_transport tr;              // laminar transport model (viscous fluxes when grid.visc is set)
   double* vbuf;                 // viscous node planes and node fluxes
   double* vcell;                // viscous rhs of the current stage state (nv x ncell)
@@ -181,9 +181,12 @@ int jb_create(const jb_mech_params* mech, int dim, int nx, int ny, double dx, do
   if (e == cudaSuccess) e = cudaMalloc(&h->slots, sizeof(jb_slots));
   if (e == cudaSuccess) e = cudaMemset(h->strips, 0, bytes_strip);
   if (e == cudaSuccess) e = cudaMemset(h->slots, 0, sizeof(jb_slots));
-  // mixed 2D: float32 primitives of the stage state and of the state being
-  // written (two buffers used in turn), then the x flux differences
-  const size_t bytes_fwork = precision == JB_PREC_MIXED && dim == 2 ? sizeof(float) * 18 * nc : 0;
+  // 2D sweeps (jb_sweep.cuh): the primitives of the stage state (mixed: and
+  // of the state being written, two buffers used in turn), then the x flux
+  // differences; float32 in mixed, float64 in fp64
+  const size_t bytes_fwork = dim != 2 || precision == JB_PREC_STRICT ? 0
+                             : precision == JB_PREC_MIXED            ? sizeof(float) * 18 * nc
+                                                                     : sizeof(double) * 15 * nc;
   if (e == cudaSuccess && bytes_fwork) e = cudaMalloc(&h->fwork, bytes_fwork);
   if (e != cudaSuccess) {
     jb_destroy(h);
@@ -291,6 +294,23 @@ int jb_set_ghost_cells(jb_handle* h, double* sendx, double* halox, double* sendy
   return JB_OK;
 }
 
+// Parts of the handle's 2D sweep scratch: the stage state's primitives, the
+// buffer of the next state's (mixed) and the x flux differences; null where
+// the handle's flux options take the tile kernels.
+struct sweep_work {
+  void *prims, *prims_next, *dfx;
+};
+static sweep_work sweep_parts(const jb_handle* h) {
+  const jb_grid& g = h->grid;
+  if (!h->fwork || g.scheme != JB_FLUX_LF || g.recon != JB_RECON_WENO5) return {nullptr, nullptr, nullptr};
+  if (h->precision == JB_PREC_MIXED) {
+    float* b = static_cast<float*>(h->fwork);
+    return {b, b + 3 * g.ncell, b + 6 * g.ncell};
+  }
+  double* b = static_cast<double*>(h->fwork);
+  return {b, b, b + 3 * g.ncell};
+}
+
 int jb_flux_func(jb_handle* h, const double* U, const double* aux, double dt, double* rhs,
                  void* stream) {
   if (!h || !U || !aux || !rhs) return set_err(h, JB_ERR_ARG, "null pointer");
@@ -298,14 +318,15 @@ int jb_flux_func(jb_handle* h, const double* U, const double* aux, double dt, do
   cudaStream_t st = (cudaStream_t)stream;
   const jb::Ops& o = *h->ops;
   JB_TRY(o.slots_reset(h->slots, st), "slots_reset");
+  const sweep_work sw = sweep_parts(h);
   JB_TRY(o.select(h->dim, false, true, false, h->mech, h->grid, U, aux, nullptr, nullptr, h->strips,
-                  h->slots, -1, 3, nullptr, st),
+                  h->slots, -1, 3, sw.prims, st),
          "alpha");
   if (int rc = exchange(h, U, aux, JB_XCH_HALO, 3, st)) return rc;
   if (h->grid.visc)
     JB_TRY(o.visc(h->dim, h->mech, h->grid, h->tr, U, aux, h->strips, h->vbuf, h->vcell, st), "viscous");
   JB_TRY(o.flux(h->dim, 0, h->mech, h->grid, U, aux, nullptr, rhs, h->strips, h->slots, 3, jb_fin_cand(nullptr, -1),
-                nullptr, nullptr, dt, st),
+                sw.prims, sw.dfx, dt, st),
          "flux");
   return JB_OK;
 }
@@ -388,13 +409,15 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
   // iterates and a select pass after each picks the reference's iteration
   // count.
   const bool pc = o.per_cell && (d == 2 || g.scheme == JB_FLUX_LF || g.scheme == JB_FLUX_SW);
-  // mixed 2D: float32 u, v, p of the current state (pin) and the buffer the
-  // next kernel writes (pout), swapped after each writer
-  float* pin = h->fwork ? static_cast<float*>(h->fwork) : nullptr;
-  float* pout = pin ? pin + 3 * g.ncell : nullptr;
-  void* dfx = pin ? static_cast<void*>(pin + 6 * g.ncell) : nullptr;
+  // 2D sweeps: u, v, p of the current state (pin); mixed: and the buffer the
+  // next kernel writes (pout), swapped after each writer (fp64: the select
+  // pass rewrites pin between the stages)
+  const sweep_work sw = sweep_parts(h);
+  void* pin = sw.prims;
+  float* pout = static_cast<float*>(pc ? sw.prims_next : nullptr);
+  void* dfx = sw.dfx;
   auto swap_prims = [&]() {
-    float* t = pin;
+    float* t = static_cast<float*>(pin);
     pin = pout;
     pout = t;
   };

@@ -125,8 +125,8 @@ struct Shape {
 
 template <class R, int NT>
 __host__ __device__ constexpr size_t ens_smem_bytes() {
-  return smem1d_bytes<R, NT>(12) > sizeof(double) * CHEM_SH * NT ? smem1d_bytes<R, NT>(12)
-                                                                  : sizeof(double) * CHEM_SH * NT;
+  return line_smem<R, NT - ENS_HALO>() > sizeof(double) * CHEM_SH * NT ? line_smem<R, NT - ENS_HALO>()
+                                                                        : sizeof(double) * CHEM_SH * NT;
 }
 
 // The mechanism of the running ensemble.  Each launch copies it here from
@@ -185,9 +185,9 @@ __device__ __noinline__ void flux_pass(const jb_ens_inst& I, int rank, const dou
   unsigned bits = 0;
   double amx = 0.0, dtm = __longlong_as_double(0x7ff0000000000000LL);
   for (int t = rank; t < I.ntiles; t += I.ncta)
-    bits |= flux1d_tile<STAGE, R, NT>(c_mech, I.g, Uk, auxk, I.U, out, fin, I.strips, alpha, dt, t * (NT - 1),
-                                      smraw, amx, dtm, s);
-  if (fin.aux && fin.aidx >= 0) ens_strips(I, rank, NT - 1, I.ntiles, out, fin.aux, amx);
+    bits |= line_tile<STAGE, R, NT, NT - ENS_HALO>(c_mech, I.g, Uk, auxk, I.U, out, fin, I.strips, alpha, dt,
+                                                   t * (NT - ENS_HALO), smraw, amx, dtm, s);
+  if (fin.aux && fin.aidx >= 0) ens_strips(I, rank, NT - ENS_HALO, I.ntiles, out, fin.aux, amx);
   finish_reduce(fin, amx, 0.0, dtm, bits, s);
 }
 
@@ -498,7 +498,7 @@ int configure(jb_ensemble* e, int block, int bpsm) {
     jb_ens_inst& I = e->host_insts[i];
     I.cta0 = c;
     I.ncta = ncta[i];
-    I.ntiles = (e->nx[i] + block - 2) / (block - 1);
+    I.ntiles = (e->nx[i] + block - ENS_HALO - 1) / (block - ENS_HALO);
     I.nchunks = (e->nx[i] + block - 1) / block;
     for (int j = 0; j < ncta[i]; ++j) cta_inst[c++] = i;
   }

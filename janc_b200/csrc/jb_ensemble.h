@@ -4,6 +4,10 @@
 
 #include "jb_types.h"
 
+// A flux tile's padded cells are one per thread of its block: block - ENS_HALO
+// cells and the 3 + 3 halo cells.
+#define ENS_HALO 6
+
 // One instance (a detonation tube).  Every pointer is device memory owned by
 // the ensemble; the state U / aux is advanced in place.
 typedef struct jb_ens_inst {
@@ -22,7 +26,7 @@ typedef struct jb_ens_inst {
   double cfl;           // > 0: CFL time step
   double dt;            // fixed time step when cfl <= 0
   int cta0, ncta;       // the CTAs [cta0, cta0 + ncta) serve this instance
-  int ntiles;           // flux tiles of (block - 1) cells
+  int ntiles;           // flux tiles of (block - ENS_HALO) cells
   int nchunks;          // cell chunks of block cells (select / chemistry)
 } jb_ens_inst;
 

@@ -50,21 +50,23 @@ __device__ __forceinline__ double bitsd(unsigned long long b) {
 // ---------------------------------------------------------------------------
 // block reductions
 // ---------------------------------------------------------------------------
+// Non-negative doubles (and +inf) order as their bit patterns, so a warp's
+// maximum or minimum is two 32-bit redux instructions, the high words first
+// and then the low words of the lanes that hold the extreme high word
+// (a shuffle tree took five rounds of two shuffles and a compare each).
 __device__ __forceinline__ double warp_max(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  const unsigned long long b = dbits(v);
+  const unsigned hi = (unsigned)(b >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
+  return bitsd(((unsigned long long)mh << 32) | ml);
 }
 __device__ __forceinline__ double warp_min(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  const unsigned long long b = dbits(v);
+  const unsigned hi = (unsigned)(b >> 32), mh = __reduce_min_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_min_sync(0xffffffffu, hi == mh ? (unsigned)b : 0xffffffffu);
+  return bitsd(((unsigned long long)mh << 32) | ml);
 }
-__device__ __forceinline__ unsigned warp_or(unsigned v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
+__device__ __forceinline__ unsigned warp_or(unsigned v) { return __reduce_or_sync(0xffffffffu, v); }
 
 // All threads of the block must call; returns the result in thread 0.
 __device__ __forceinline__ void block_reduce_store(double ax, double ay, double dtm,
@@ -569,10 +571,49 @@ __device__ void pressure_outlet_state(const MP& m, const double* q, double gamma
   out[nv + 1] = T_c;
 }
 
+// One evaluation of the injector's throat condition at Mach number M
+// (inj_model): whether the flow chokes below (up: P2 >= P1, dn: P2 < P1; a
+// NaN is neither), the mass flux and the injection velocity.
+__device__ __forceinline__ void injector_eval(double M, double P3, double Ri, double C0, bool& up, bool& dn,
+                                              double& MFC, double& V3) {
+  const double gam = 1.29, A1 = 1.0, A3 = 5.0, A2 = 4.0;
+  const double gh = (gam - 1.0) / 2.0;
+  const double e2 = -(gam + 1.0) / 2.0 / (gam - 1.0);
+  const double gg = gam / (gam - 1.0);
+  double base = 1.0 + gh * (M * M);
+#if JB_FAST
+  // -gam / (gam - 1) = e2 - 1/2: one power and one square root for the
+  // reference's three powers
+  const double pw = pow(base, e2), rs = 1.0 / sqrt(base);
+  double P1 = pw * rs;
+  double V1 = M * rs * C0;
+  MFC = 1.0 * sqrt(gam / Ri) * M * pw;
+#else
+  const double e1 = -gam / (gam - 1.0);
+  double P1 = 1.0 * pow(base, e1);
+  double V1 = M * pow(base, -0.5) * C0;
+  MFC = 1.0 * sqrt(gam / Ri) * M * pow(base, e2);
+#endif
+  double B = gg * P3 * A3 / MFC;
+  double C = -gam / (gam - 1.0) * Ri * 1.0;
+  V3 = (-B + sqrt(B * B - 2.0 * C)) / 1.0;
+  double P2 = (MFC * (V3 - V1) - P1 * A1 + P3 * A3) / A2;
+  up = P2 >= P1;
+  dn = P2 < P1;
+}
+
 // Rotating-detonation injector of examples/janc_basic_example2.ipynb
 // (bottom_boundary + inj_model, after Fievisohn et al. 2017): bisection on
 // the throat Mach number of a choked injector fed at nondimensional total
 // pressure 1 and temperature 1; blocked (slip-like) when p_in >= 1.
+// WARP: the 32 lanes of a warp call it together on one boundary cell.  The 20
+// bisections then are 4 rounds of 5: each lane evaluates one of the 31 nodes
+// of the five-level tree below the current interval (the midpoints the
+// sequential bisection can meet, formed by the same operations), and every
+// lane walks the tree by the ballots, so the result is the sequential one.
+// Four dependent evaluations instead of 20: 35.6 us a launch at 1600
+// positions before, 12 us now.
+template <bool WARP>
 __device__ void injector_state(const MP& m, const double* q, double gamma, double T,
                                const double* Yinj8, double block_p, double* out) {
   constexpr int nY = 4;
@@ -590,27 +631,42 @@ __device__ void injector_state(const MP& m, const double* q, double gamma, doubl
   double Yi[NS];
   fill_Y(Yinj8, Yi);
   double Ri = get_R(m, Yi);
-  const double gam = 1.29;
-  const double A1 = 1.0, A3 = 5.0, A2 = 4.0;
-  const double C0 = sqrt(gam * Ri * 1.0);
-  const double gh = (gam - 1.0) / 2.0;
-  const double e1 = -gam / (gam - 1.0);
-  const double e2 = -(gam + 1.0) / 2.0 / (gam - 1.0);
-  const double gg = gam / (gam - 1.0);
+  const double A3 = 5.0;
+  const double C0 = sqrt(1.29 * Ri * 1.0);
   const double P3 = p;
   double M1 = 0.0, M2 = 1.0, MFC = 0.0, V3 = 0.0;
-  for (int it = 0; it < 20; ++it) {
-    double M = 0.5 * (M1 + M2);
-    double base = 1.0 + gh * (M * M);
-    double P1 = 1.0 * pow(base, e1);
-    double V1 = M * pow(base, -0.5) * C0;
-    MFC = 1.0 * sqrt(gam / Ri) * M * pow(base, e2);
-    double B = gg * P3 * A3 / MFC;
-    double C = -gam / (gam - 1.0) * Ri * 1.0;
-    V3 = (-B + sqrt(B * B - 2.0 * C)) / 1.0;
-    double P2 = (MFC * (V3 - V1) - P1 * A1 + P3 * A3) / A2;
-    M2 = (P2 >= P1) ? M : M2;
-    M1 = (P2 < P1) ? M : M1;
+  bool up, dn;
+  if (WARP) {
+    const int lane = threadIdx.x & 31, node = lane ? lane : 1;
+#pragma unroll 1
+    for (int round = 0; round < 4; ++round) {
+      double lo = M1, hi = M2;
+      for (int bit = 30 - __clz(node); bit >= 0; --bit) {  // the path to this lane's node
+        const double M = 0.5 * (lo + hi);
+        if ((node >> bit) & 1) lo = M;
+        else hi = M;
+      }
+      double mf, v3;
+      injector_eval(0.5 * (lo + hi), P3, Ri, C0, up, dn, mf, v3);
+      const unsigned ups = __ballot_sync(0xffffffffu, up), dns = __ballot_sync(0xffffffffu, dn);
+      int n = 1, last = 1;
+      for (int d = 0; d < 5; ++d) {
+        const double M = 0.5 * (M1 + M2);
+        last = n;
+        if ((ups >> n) & 1u) { M2 = M; n = 2 * n; }
+        else if ((dns >> n) & 1u) { M1 = M; n = 2 * n + 1; }
+        else break;  // neither: the interval stays, and so does every later midpoint
+      }
+      MFC = __shfl_sync(0xffffffffu, mf, last);
+      V3 = __shfl_sync(0xffffffffu, v3, last);
+    }
+  } else {
+    for (int it = 0; it < 20; ++it) {
+      double M = 0.5 * (M1 + M2);
+      injector_eval(M, P3, Ri, C0, up, dn, MFC, V3);
+      M2 = up ? M : M2;
+      M1 = dn ? M : M1;
+    }
   }
   double rho_i = MFC / V3 / A3;
   double T_i = P3 / (Ri * rho_i);
@@ -651,41 +707,60 @@ constexpr double W_13 = 1.0 / 3.0, W_76 = 7.0 / 6.0, W_116 = 11.0 / 6.0;
 constexpr double W_m16 = -1.0 / 6.0, W_56 = 5.0 / 6.0, W_16 = 1.0 / 6.0;
 
 #if JB_FAST
-// Same weights with one division: alpha_k = C_k / d_k^2 is scaled by
-// d_1^2 d_2^2 d_3^2, so w_k = C_k prod_{j!=k} d_j^2 / sum.  (The float64
-// range covers the squared products of the smoothness indicators met here.)
-__device__ __forceinline__ double weno_combine(double IS1, double IS2, double IS3, double q1, double q2,
-                                               double q3) {
-  const double e1 = W_EPS + IS1, e2 = W_EPS + IS2, e3 = W_EPS + IS3;
-  const double s1 = e1 * e1, s2 = e2 * e2, s3 = e3 * e3;
-  const double a1 = W_C1 * (s2 * s3), a2 = W_C2 * (s1 * s3), a3 = W_C3 * (s1 * s2);
-  return (a1 * q1 + a2 * q2 + a3 * q3) / (a1 + a2 + a3);
+// 1 / x of a float64 x > 0 away from the ends of the range: the hardware's
+// approximate reciprocal refined by one third-order step of the Newton
+// family, r (1 + e + e^2) with e = 1 - x r (its error e^3 is below half an
+// ulp).  No range fix-up and no branch, so that several of them interleave.
+__device__ __forceinline__ double rcp_pos(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 }
 
+// Weighted correction of a WENO5-JS value (reconstruction/WENO5_JS.py) at the
+// face behind cell j, value = f_j + num / (6 den), from the four differences
+// around it, dmm = f_{j-1} - f_{j-2}, dm = f_j - f_{j-1}, dp = f_{j+1} - f_j,
+// dpp = f_{j+2} - f_{j+1}, and the curvature terms D_i = 13/3 (d_{i+1/2} -
+// d_{i-1/2})^2 + 16 eps of cells j-1, j, j+1.  With t1 = 3 dm - dmm, t2 = dm +
+// dp, t3 = 3 dp - dpp the candidates relative to f_j are (2 t1 - dm) / 6,
+// (t2 + dp) / 6 and (t3 + dp) / 6, and the linear weights are 1 : 6 : 3.  The
+// inputs are split fluxes without the 1/2 (H' = F +- alpha q = 2 H), so t^2 +
+// D is 16 times eps + IS, which leaves every weight as the reference's in
+// real arithmetic (plain values take D with 4 eps).
+//
+// float64: alpha_k = C_k / e_k^2 scaled by (e_1 e_2 e_3)^2, one reciprocal.
+__device__ __forceinline__ void weno_side(double dmm, double dm, double dp, double dpp, double Da, double Db,
+                                          double Dc, double& num, double& den) {
+  const double t1 = fma(3.0, dm, -dmm), t2 = dm + dp, t3 = fma(3.0, dp, -dpp);
+  const double e1 = fma(t1, t1, Da), e2 = fma(t2, t2, Db), e3 = fma(t3, t3, Dc);
+  const double p1 = e2 * e3, p2 = e1 * e3, p3 = e1 * e2;
+  const double a1 = p1 * p1, a2 = 6.0 * (p2 * p2), a3 = 3.0 * (p3 * p3);
+  num = fma(a3, t3 + dp, fma(a2, t2 + dp, a1 * fma(2.0, t1, -dm)));
+  den = (a1 + a2) + a3;
+}
+
+
+// curvature term of two neighbouring differences, 13/3 s^2 + eps
+__device__ __forceinline__ double weno_curv(double da, double db, double eps) {
+  const double s = db - da;
+  return fma((13.0 / 3.0) * s, s, eps);
+}
+
+// Left-biased value at j+1/2 from cells j-2..j+2 (interface_L_*), as f_j plus
+// the weighted correction of its differences: 38 operations with one
+// reciprocal (the candidate polynomials and smoothness sums taken term by
+// term with a division took 55).
 __device__ __forceinline__ double weno_L(double fjm2, double fjm1, double fj, double fjp1, double fjp2) {
-  double t1 = fjm2 - 4.0 * fjm1 + 3.0 * fj, s1 = fjm2 - 2.0 * fjm1 + fj;
-  double t2 = fjm1 - fjp1, s2 = fjm1 - 2.0 * fj + fjp1;
-  double t3 = 3.0 * fj - 4.0 * fjp1 + fjp2, s3 = fj - 2.0 * fjp1 + fjp2;
-  double IS1 = W_Q * (t1 * t1) + W_D * (s1 * s1);
-  double IS2 = W_Q * (t2 * t2) + W_D * (s2 * s2);
-  double IS3 = W_Q * (t3 * t3) + W_D * (s3 * s3);
-  double q1 = W_13 * fjm2 - W_76 * fjm1 + W_116 * fj;
-  double q2 = W_m16 * fjm1 + W_56 * fj + W_13 * fjp1;
-  double q3 = W_13 * fj + W_56 * fjp1 - W_16 * fjp2;
-  return weno_combine(IS1, IS2, IS3, q1, q2, q3);
+  const double dmm = fjm1 - fjm2, dm = fj - fjm1, dp = fjp1 - fj, dpp = fjp2 - fjp1;
+  double num, den;
+  weno_side(dmm, dm, dp, dpp, weno_curv(dmm, dm, 4 * W_EPS), weno_curv(dm, dp, 4 * W_EPS),
+            weno_curv(dp, dpp, 4 * W_EPS), num, den);
+  return fma(1.0 / 6.0, num * rcp_pos(den), fj);
 }
-
+// right-biased value at j-1/2 (interface_R_*): the mirrored stencil
 __device__ __forceinline__ double weno_R(double fjm2, double fjm1, double fj, double fjp1, double fjp2) {
-  double t1 = fjp2 - 4.0 * fjp1 + 3.0 * fj, s1 = fjp2 - 2.0 * fjp1 + fj;
-  double t2 = fjp1 - fjm1, s2 = fjp1 - 2.0 * fj + fjm1;
-  double t3 = 3.0 * fj - 4.0 * fjm1 + fjm2, s3 = fj - 2.0 * fjm1 + fjm2;
-  double IS1 = W_Q * (t1 * t1) + W_D * (s1 * s1);
-  double IS2 = W_Q * (t2 * t2) + W_D * (s2 * s2);
-  double IS3 = W_Q * (t3 * t3) + W_D * (s3 * s3);
-  double q1 = W_13 * fjp2 - W_76 * fjp1 + W_116 * fj;
-  double q2 = W_m16 * fjp1 + W_56 * fj + W_13 * fjm1;
-  double q3 = W_13 * fj + W_56 * fjm1 - W_16 * fjm2;
-  return weno_combine(IS1, IS2, IS3, q1, q2, q3);
+  return weno_L(fjp2, fjp1, fj, fjm1, fjm2);
 }
 #else
 // left-biased value at j+1/2 from cells j-2..j+2 (interface_L_*)
@@ -895,10 +970,6 @@ __device__ __forceinline__ void sw_split(int f, int dir, R qf, R rho, R u, R v, 
 // ---------------------------------------------------------------------------
 // float32 flux arithmetic of the mixed-precision variant
 // ---------------------------------------------------------------------------
-// The reference's epsilon is absolute (1e-6) while SI flux magnitudes reach
-// ~1e11, so (eps + IS)^2 overflows float32.  The weights are formed as ratios
-// to the smallest (eps + IS_k), alpha_k ~ C_k (min/(eps + IS_k))^2, which is
-// the same normalised weight in real arithmetic and cannot overflow.
 // One approximate reciprocal (MUFU.RCP, ~1 ulp).  The WENO weights' operands
 // are at least eps (smoothness sums eps + IS) or the smallest linear weight
 // (weight sums, where one ratio is 1), never denormal or huge, so no range
@@ -909,43 +980,39 @@ __device__ __forceinline__ float rcp_fast(float x) {
   return r;
 }
 
-__device__ __forceinline__ float weno_combine32(float IS1, float IS2, float IS3, float q1, float q2,
-                                                float q3, float eps) {
-  const float e1 = eps + IS1, e2 = eps + IS2, e3 = eps + IS3;
-  const float mn = fminf(e1, fminf(e2, e3));
-  const float r1 = mn * rcp_fast(e1), r2 = mn * rcp_fast(e2), r3 = mn * rcp_fast(e3);
-  const float a1 = 0.1f * (r1 * r1), a2 = 0.6f * (r2 * r2), a3 = 0.3f * (r3 * r3);
-  return (a1 * q1 + a2 * q2 + a3 * q3) * rcp_fast(a1 + a2 + a3);
+// The correction num / (6 den) of the float64 form in float32: squares of
+// e_k ~ (SI flux 1e12)^2 overflow, so the weights are taken relative to the
+// central stencil's, (e_2 / e_k)^2, the ratio bounded by 6.5e4.  e_2 <= 8/3
+// (e_1 + e_3) for any data (e_1 >= 13/4 dm^2, e_3 >= 13/4 dp^2, e_2 <= 26/3
+// (dm^2 + dp^2), each + eps), so at most one side's ratio reaches the bound,
+// and there the other weights are below 1e-8 of its own: the bound changes
+// no float32 weight.
+__device__ __forceinline__ void weno_side(float dmm, float dm, float dp, float dpp, float Da, float Db, float Dc,
+                                          float& num, float& den) {
+  const float t1 = fmaf(3.f, dm, -dmm), t2 = dm + dp, t3 = fmaf(3.f, dp, -dpp);
+  const float e1 = fmaf(t1, t1, Da), e2 = fmaf(t2, t2, Db), e3 = fmaf(t3, t3, Dc);
+  const float r1 = fminf(e2 * rcp_fast(e1), 6.5e4f), r3 = fminf(e2 * rcp_fast(e3), 6.5e4f);
+  const float a1 = r1 * r1, a3 = 3.f * (r3 * r3);
+  num = fmaf(a3, t3 + dp, fmaf(a1, fmaf(2.f, t1, -dm), 6.f * (t2 + dp)));
+  den = (a1 + 6.f) + a3;
+}
+__device__ __forceinline__ float weno_curv(float da, float db, float eps) {
+  const float s = db - da;
+  return fmaf((13.f / 3.f) * s, s, eps);
 }
 
-// Left/right-biased float32 values.  The ratio form of the weights never
-// squares (eps + IS), so only IS itself must stay in range: |f| below ~1e18
-// (SI fluxes stay below ~1e12).  Tiny fields give IS << eps and the linear
-// weights, as the reference's absolute eps does.
+// Left/right-biased float32 values.  Only e itself must stay in range: |f|
+// below ~1e18 (SI fluxes stay below ~1e12).  Tiny fields give IS << eps and
+// the linear weights, as the reference's absolute eps does.
 __device__ __forceinline__ float weno_L(float fjm2, float fjm1, float fj, float fjp1, float fjp2) {
-  const float t1 = fjm2 - 4.f * fjm1 + 3.f * fj, s1 = fjm2 - 2.f * fjm1 + fj;
-  const float t2 = fjm1 - fjp1, s2 = fjm1 - 2.f * fj + fjp1;
-  const float t3 = 3.f * fj - 4.f * fjp1 + fjp2, s3 = fj - 2.f * fjp1 + fjp2;
-  const float IS1 = 0.25f * (t1 * t1) + (13.f / 12.f) * (s1 * s1);
-  const float IS2 = 0.25f * (t2 * t2) + (13.f / 12.f) * (s2 * s2);
-  const float IS3 = 0.25f * (t3 * t3) + (13.f / 12.f) * (s3 * s3);
-  const float q1 = (1.f / 3.f) * fjm2 - (7.f / 6.f) * fjm1 + (11.f / 6.f) * fj;
-  const float q2 = (-1.f / 6.f) * fjm1 + (5.f / 6.f) * fj + (1.f / 3.f) * fjp1;
-  const float q3 = (1.f / 3.f) * fj + (5.f / 6.f) * fjp1 - (1.f / 6.f) * fjp2;
-  return weno_combine32(IS1, IS2, IS3, q1, q2, q3, 1e-6f);
+  const float dmm = fjm1 - fjm2, dm = fj - fjm1, dp = fjp1 - fj, dpp = fjp2 - fjp1;
+  float num, den;
+  weno_side(dmm, dm, dp, dpp, weno_curv(dmm, dm, 4e-6f), weno_curv(dm, dp, 4e-6f), weno_curv(dp, dpp, 4e-6f), num,
+            den);
+  return fmaf(1.f / 6.f, num * rcp_fast(den), fj);
 }
-
 __device__ __forceinline__ float weno_R(float fjm2, float fjm1, float fj, float fjp1, float fjp2) {
-  const float t1 = fjp2 - 4.f * fjp1 + 3.f * fj, s1 = fjp2 - 2.f * fjp1 + fj;
-  const float t2 = fjp1 - fjm1, s2 = fjp1 - 2.f * fj + fjm1;
-  const float t3 = 3.f * fj - 4.f * fjm1 + fjm2, s3 = fj - 2.f * fjm1 + fjm2;
-  const float IS1 = 0.25f * (t1 * t1) + (13.f / 12.f) * (s1 * s1);
-  const float IS2 = 0.25f * (t2 * t2) + (13.f / 12.f) * (s2 * s2);
-  const float IS3 = 0.25f * (t3 * t3) + (13.f / 12.f) * (s3 * s3);
-  const float q1 = (1.f / 3.f) * fjp2 - (7.f / 6.f) * fjp1 + (11.f / 6.f) * fj;
-  const float q2 = (-1.f / 6.f) * fjp1 + (5.f / 6.f) * fj + (1.f / 3.f) * fjm1;
-  const float q3 = (1.f / 3.f) * fj + (5.f / 6.f) * fjm1 - (1.f / 6.f) * fjm2;
-  return weno_combine32(IS1, IS2, IS3, q1, q2, q3, 1e-6f);
+  return weno_L(fjp2, fjp1, fj, fjm1, fjm2);
 }
 
 template <int DIM>
@@ -1321,322 +1388,8 @@ __global__ void __launch_bounds__(NT2, sizeof(R) == 4 ? 3 : 2) k_flux2d(MP m, Gr
 }
 
 #if JB_FAST
-// ---------------------------------------------------------------------------
-// mixed-precision 2D RK stage as an x-line sweep plus y runs (STAGE 1..3)
-// ---------------------------------------------------------------------------
-// float32 LF splitting and WENO5-JS on float32 primitives, float64 RK
-// combination and temperature solve:
-//   k_sweep_x    one thread per (y line, x segment of seg cells, field
-//                pair; seg chosen by the host for whole waves): a register
-//                window of the split fluxes walks the
-//                segment's faces and writes the x flux difference
-//                F_{i+1/2} - F_{i-1/2} of each cell
-//   k_flux_y_rk  one block per segment of S cells of a column (S = 32 x
-//                warps, up to 256, one cell per thread): split fluxes of all
-//                fields on the segment and its 3 + 3 halo cells in shared
-//                memory, the S + 1 y faces and the differences, then the
-//                RK combination with the x part and the temperature solve
-//                of the new state
-// Fields are handled in pairs (rho, rho u), (rho v, rho E), (rho Y_1, rho
-// Y_2), ... with sm_100's paired float32 instructions (FFMA2 / FADD2 /
-// FMUL2), which issue two float32 operations at once.  The x differences are
-// stored as float2 pairs: dfx[6][ncell][2].  The stage state's float32 u, v,
-// p come from the kernel that wrote that state (prims[3][ncell]).
-constexpr int SX_NT = 128;
-#ifndef JB_YR_W
-#define JB_YR_W 4
+#include "jb_sweep.cuh"
 #endif
-constexpr int YR_W = JB_YR_W, YR_NT = 32 * YR_W;  // most warps of a y-run block
-// shared memory of a y-run block of S cells: H+ and H- of the S + 6 window
-// cells and the S + 1 face values, six field pairs each
-__host__ __device__ constexpr size_t yr_smem(int S) {
-  return sizeof(float2) * (2 * 6 * (size_t)(S + 6) + 6 * (size_t)(S + 1));
-}
-
-typedef float2 f2;
-__device__ __forceinline__ f2 f2s(float a) { return make_float2(a, a); }
-__device__ __forceinline__ f2 f2add(f2 a, f2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ f2 f2mul(f2 a, f2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ f2 f2fma(f2 a, f2 b, f2 c) { return __ffma2_rn(a, b, c); }
-
-// WENO5-JS (reconstruction/WENO5_JS.py) of two fields at once: the
-// left-biased value at the face between c and d from cells a..e (the
-// right-biased value at the face between b and c is weno2(e, d, c, b, a)).
-// The inputs are split fluxes without the 1/2 (H' = F +- alpha q = 2 H), so
-// the smoothness indicators are formed as t^2 + 13/3 s^2 (16 IS) with eps
-// scaled by 16, which leaves every weight exactly as the reference's in real
-// arithmetic; the caller halves the face value.  Weights in the ratio form
-// to the smallest eps + IS (no float32 overflow for SI fluxes ~1e11), with
-// the linear weights C_k folded into the candidate polynomials.
-__device__ __forceinline__ f2 weno2(f2 a, f2 b, f2 c, f2 d, f2 e) {
-  const f2 t1 = f2fma(c, f2s(3.f), f2fma(b, f2s(-4.f), a));
-  const f2 s1 = f2add(f2fma(b, f2s(-2.f), a), c);
-  const f2 t2 = f2fma(d, f2s(-1.f), b);
-  const f2 s2 = f2add(f2fma(c, f2s(-2.f), b), d);
-  const f2 t3 = f2fma(c, f2s(3.f), f2fma(d, f2s(-4.f), e));
-  const f2 s3 = f2add(f2fma(d, f2s(-2.f), c), e);
-  const f2 e16 = f2s(16e-6f), k13 = f2s(13.f / 3.f);
-  const f2 e1 = f2fma(t1, t1, f2fma(f2mul(s1, k13), s1, e16));
-  const f2 e2 = f2fma(t2, t2, f2fma(f2mul(s2, k13), s2, e16));
-  const f2 e3 = f2fma(t3, t3, f2fma(f2mul(s3, k13), s3, e16));
-  const f2 mn = make_float2(fminf(e1.x, fminf(e2.x, e3.x)), fminf(e1.y, fminf(e2.y, e3.y)));
-  const f2 r1 = f2mul(mn, make_float2(rcp_fast(e1.x), rcp_fast(e1.y)));
-  const f2 r2 = f2mul(mn, make_float2(rcp_fast(e2.x), rcp_fast(e2.y)));
-  const f2 r3 = f2mul(mn, make_float2(rcp_fast(e3.x), rcp_fast(e3.y)));
-  const f2 w1 = f2mul(r1, r1), w2 = f2mul(r2, r2), w3 = f2mul(r3, r3);
-  // C_k times the candidate values (C = 1/10, 6/10, 3/10)
-  const f2 q1 = f2fma(c, f2s(11.f / 60.f), f2fma(b, f2s(-7.f / 60.f), f2mul(a, f2s(1.f / 30.f))));
-  const f2 q2 = f2fma(d, f2s(0.2f), f2fma(c, f2s(0.5f), f2mul(b, f2s(-0.1f))));
-  const f2 q3 = f2fma(e, f2s(-0.05f), f2fma(d, f2s(0.25f), f2mul(c, f2s(0.1f))));
-  const f2 num = f2fma(w3, q3, f2fma(w2, q2, f2mul(w1, q1)));
-  const f2 den = f2fma(w3, f2s(0.3f), f2fma(w2, f2s(0.6f), f2mul(w1, f2s(0.1f))));
-  return f2mul(num, make_float2(rcp_fast(den.x), rcp_fast(den.y)));
-}
-
-// Doubled split fluxes of field pair j at one cell for direction dir:
-// F = vel q (+ p in the normal momentum, + vel p in rho E), H' = F +- alpha q.
-__device__ __forceinline__ void split2(int j, int dir, f2 q, float vel, float p, float al, f2& hp, f2& hm) {
-  // pair 0 = (rho, rho u), pair 1 = (rho v, rho E)
-  f2 c = make_float2(0.f, 0.f);
-  if (j == 0 && dir == 0) c.y = p;
-  if (j == 1) {
-    if (dir == 1) c.x = p;
-    c.y = vel * p;
-  }
-  const f2 F = f2fma(f2s(vel), q, c);
-  hp = f2fma(f2s(al), q, F);
-  hm = f2fma(f2s(-al), q, F);
-}
-
-// Field pair j (or all 12 fields for DIR 1, as six pairs), the normal
-// velocity and the pressure of padded cell (x, y): interior and copied ghosts
-// from the state and the primitives, outlet / injector ghosts and ghost
-// layers from their buffers.  DIR 0: x sweep; DIR 1, 2: y run (2: one pair).
-template <int DIR>
-__device__ __forceinline__ void win_load2(const MP& m, const Grid& g, const double* __restrict__ Uk,
-                                          const float* __restrict__ prims, const double* __restrict__ strips, int x,
-                                          int y, int j, f2* q, float& vel, float& p) {
-  constexpr int NP = DIR == 1 ? 6 : 1;
-  const long long nc = g.ncell;
-  const Src s = map_cell<2>(g, x, y);
-  if (s.kind == 0) {
-    const long long src = (long long)s.xs * g.ny + s.ys;
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const int f = 2 * (DIR == 1 ? i : j);
-      const double v0 = Uk[f * nc + src], v1 = Uk[(f + 1) * nc + src];
-      q[i] = make_float2((float)(((s.flip >> f) & 1) ? -v0 : v0), (float)(((s.flip >> (f + 1)) & 1) ? -v1 : v1));
-    }
-    vel = prims[(DIR == 0 ? 0 : nc) + src];
-    if (s.flip & (DIR == 0 ? 2 : 4)) vel = -vel;
-    p = prims[2 * nc + src];
-  } else if (s.kind == 1) {
-    float qa[12];
-#pragma unroll
-    for (int i = 0; i < 12; ++i) qa[i] = (float)ghost(g, strips, s, i);
-    float rho, u, v;
-    flux_prims<2>(m, qa, (float)ghost(g, strips, s, 13), rho, u, v, p);
-    vel = DIR == 0 ? u : v;
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const int f = 2 * (DIR == 1 ? i : j);
-      q[i] = make_float2(qa[f], qa[f + 1]);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < NP; ++i) q[i] = make_float2(1.f, 1.f);
-    vel = 1.f;
-    p = 1.f;
-  }
-}
-
-#ifndef JB_SX_MINB
-#define JB_SX_MINB 7  // 72 registers: the paired window and WENO still fit without spills
-#endif
-#ifndef JB_SX_PF
-#define JB_SX_PF 1  // cells fetched ahead of the window (a divisor of 6)
-#endif
-__global__ void __launch_bounds__(SX_NT, JB_SX_MINB) k_sweep_x(MP m, Grid g, const double* __restrict__ Uk,
-                                                   const float* __restrict__ prims,
-                                                   const double* __restrict__ strips, const Slots* slots, int aidx,
-                                                   float2* __restrict__ dfx, int nlb, int seg_len) {
-  const int j = blockIdx.x % 6;
-  const int rest = blockIdx.x / 6;
-  const int y = (rest % nlb) * SX_NT + threadIdx.x, seg = rest / nlb;
-  if (y >= g.ny) return;
-  const long long nc = g.ncell;
-  const double* u0 = Uk + 2 * j * nc;
-  const double* u1 = u0 + nc;
-  const float al = (float)bitsd(slots->ax[aidx]);
-  const int a0 = seg * seg_len, a1 = min(a0 + seg_len, g.nx);  // cells [a0, a1), faces a0 .. a1
-  f2 Hp[6], Hm[6];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    f2 q;
-    float vel, p;
-    win_load2<0>(m, g, Uk, prims, strips, a0 - 3 + k, y, j, &q, vel, p);
-    split2(j, 0, q, vel, p, al, Hp[k], Hm[k]);
-  }
-  // The hi-side ghost cells nx .. nx+2 of the line (the last segment's
-  // window reaches them) go to this thread's column of shared memory first,
-  // so that the face loop's fetch is a plain load: the ghost mapping stays
-  // out of the unrolled loop body.
-  __shared__ float gh[3][4][SX_NT];
-  if (a1 + 2 >= g.nx) {
-#pragma unroll 1
-    for (int k = 0; k < 3; ++k) {
-      f2 q;
-      float vel, p;
-      win_load2<0>(m, g, Uk, prims, strips, g.nx + k, y, j, &q, vel, p);
-      gh[k][0][threadIdx.x] = q.x;
-      gh[k][1][threadIdx.x] = q.y;
-      gh[k][2][threadIdx.x] = vel;
-      gh[k][3][threadIdx.x] = p;
-    }
-  }
-  // the cells about to enter the window, fetched JB_SX_PF faces ahead into
-  // buffer (c - a0) % JB_SX_PF and left untouched until then so that their
-  // loads overlap the WENO arithmetic (a >= a0 + 2 >= 0 here)
-  double n0[JB_SX_PF], n1[JB_SX_PF];
-  float nv[JB_SX_PF], np[JB_SX_PF];
-  auto fetch = [&](int a, int b) {
-    if (a < g.nx) {
-      const long long src = (long long)a * g.ny + y;
-      n0[b] = u0[src];
-      n1[b] = u1[src];
-      nv[b] = prims[src];
-      np[b] = prims[2 * nc + src];
-    } else {
-      const int k = a - g.nx;
-      n0[b] = gh[k][0][threadIdx.x];
-      n1[b] = gh[k][1][threadIdx.x];
-      nv[b] = gh[k][2][threadIdx.x];
-      np[b] = gh[k][3][threadIdx.x];
-    }
-  };
-#pragma unroll
-  for (int k = 0; k < JB_SX_PF; ++k) fetch(a0 + 2 + k, (2 + k) % JB_SX_PF);
-  float2* out = dfx + (long long)j * nc + y;
-  f2 Fprev = make_float2(0.f, 0.f);
-  // cell c lives in window slot (c - a0 + 3) % 6: the face loop is unrolled
-  // over the window's period so that the window rotates by renaming
-#pragma unroll 1
-  for (int fb = a0; fb <= a1; fb += 6) {
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-      const int fa = fb + r;
-      if (fa > a1) break;
-      const int bc = (r + 2) % JB_SX_PF;  // buffer of cell fa + 2 ((fb - a0) is a multiple of 6)
-      split2(j, 0, make_float2((float)n0[bc], (float)n1[bc]), nv[bc], np[bc], al, Hp[(r + 5) % 6],
-             Hm[(r + 5) % 6]);  // cell fa+2
-      if (fa + JB_SX_PF <= a1) fetch(fa + 2 + JB_SX_PF, bc);
-      // face fa (cells fa-1 | fa): H+ of cells fa-3 .. fa+1, H- of fa-2 .. fa+2
-      const f2 F = f2mul(f2s(0.5f), f2add(weno2(Hp[r % 6], Hp[(r + 1) % 6], Hp[(r + 2) % 6], Hp[(r + 3) % 6],
-                                                Hp[(r + 4) % 6]),
-                                          weno2(Hm[(r + 5) % 6], Hm[(r + 4) % 6], Hm[(r + 3) % 6],
-                                                Hm[(r + 2) % 6], Hm[(r + 1) % 6])));
-      if (fa > a0) out[(long long)(fa - 1) * g.ny] = f2fma(Fprev, f2s(-1.f), F);
-      Fprev = F;
-    }
-  }
-}
-
-#ifndef JB_YR_MINB
-#define JB_YR_MINB (32 / JB_YR_W)  // 64 registers (64 B of spills)
-#endif
-template <int STAGE, bool VISC>
-__global__ void __launch_bounds__(YR_NT, JB_YR_MINB) k_flux_y_rk(MP m, Grid g, const double* __restrict__ Uk,
-                                                       const double* __restrict__ auxk,
-                                                       const double* __restrict__ Un, const float* __restrict__ prims,
-                                                       const double* __restrict__ strips,
-                                                       const float2* __restrict__ dfx, double* __restrict__ out,
-                                                       Slots* slots, int aidx, jb_fin fin, int nsy) {
-  extern __shared__ __align__(128) unsigned char smraw[];
-  const int S = blockDim.x, t = threadIdx.x;
-  const int C = S + 6, NF = S + 1;
-  f2* sHp = reinterpret_cast<f2*>(smraw);  // [6][C]: cell y0 - 3 + j in slot j
-  f2* sHm = sHp + 6 * C;
-  f2* sF = sHm + 6 * C;  // [6][NF]: face y0 + k (cells y0+k-1 | y0+k)
-  const long long nc = g.ncell;
-  const int x = blockIdx.x / nsy, y0 = (blockIdx.x % nsy) * S;
-  const float al = (float)bitsd(slots->ay[aidx]);
-  // ---- split fluxes on the window: the segment's own cells one per
-  // thread, the 3 + 3 halo cells as 36 (cell, pair) items
-  {
-    const int jj = t + 3;
-    f2 q[6];
-    float vel, p;
-    if (y0 + t < g.ny) {
-      const long long cell = (long long)x * g.ny + y0 + t;
-#pragma unroll
-      for (int i = 0; i < 6; ++i)
-        q[i] = make_float2((float)Uk[2 * i * nc + cell], (float)Uk[(2 * i + 1) * nc + cell]);
-      vel = prims[nc + cell];
-      p = prims[2 * nc + cell];
-    } else {
-      win_load2<1>(m, g, Uk, prims, strips, x, y0 + t, 0, q, vel, p);
-    }
-#pragma unroll
-    for (int i = 0; i < 6; ++i) split2(i, 1, q[i], vel, p, al, sHp[i * C + jj], sHm[i * C + jj]);
-  }
-#pragma unroll 1
-  for (int i = t; i < 36; i += S) {
-    const int h = i / 6, pr = i % 6;
-    const int jj = h < 3 ? h : S + h;
-    f2 q;
-    float vel, p;
-    win_load2<2>(m, g, Uk, prims, strips, x, y0 - 3 + jj, pr, &q, vel, p);
-    split2(pr, 1, q, vel, p, al, sHp[pr * C + jj], sHm[pr * C + jj]);
-  }
-  __syncthreads();
-  // ---- faces: face y0 + t of every pair, and face y0 + S by threads 0..5
-  // (one pair each)
-#pragma unroll 1
-  for (int i = 0; i < 6; ++i) {
-    const f2* hp = sHp + i * C + t;
-    const f2* hm = sHm + i * C + t;
-    sF[i * NF + t] = f2mul(f2s(0.5f), f2add(weno2(hp[0], hp[1], hp[2], hp[3], hp[4]),
-                                             weno2(hm[5], hm[4], hm[3], hm[2], hm[1])));
-  }
-  if (t < 6) {
-    const f2* hp = sHp + t * C + S;
-    const f2* hm = sHm + t * C + S;
-    sF[t * NF + S] = f2mul(f2s(0.5f), f2add(weno2(hp[0], hp[1], hp[2], hp[3], hp[4]),
-                                             weno2(hm[5], hm[4], hm[3], hm[2], hm[1])));
-  }
-  __syncthreads();
-  // ---- RK combination (float64) and update_aux of the new state
-  const int y = y0 + t;
-  const bool live = y < g.ny;
-  unsigned bits = 0;
-  double amx = 0.0, amy = 0.0, dtm = __longlong_as_double(0x7ff0000000000000LL);
-  if (live) {
-    const long long cell = (long long)x * g.ny + y;
-    const double dt = slots->dt;
-    double q[12];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const float2 dF = dfx[i * nc + cell];
-      const f2 dG = f2fma(sF[i * NF + t], f2s(-1.f), sF[i * NF + t + 1]);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int f = 2 * i + h;
-        const double rhs = dt * visc_add<VISC>(g, f, cell, -((double)(h ? dF.y : dF.x) * g.idx +
-                                                            (double)(h ? dG.y : dG.x) * g.idy));
-        const double uk = Uk[f * nc + cell];  // read again (L1): no registers held across the WENO
-        double r;
-        if (STAGE == 1) r = uk + rhs;
-        else if (STAGE == 2) r = 3.0 / 4.0 * Un[f * nc + cell] + 1.0 / 4.0 * (uk + rhs);
-        else r = 1.0 / 3.0 * Un[f * nc + cell] + 2.0 / 3.0 * (uk + rhs);
-        out[f * nc + cell] = r;
-        q[f] = r;
-      }
-    }
-    bits = finish_state<2, true>(m, g, fin, q, auxk[nc + cell], cell, amx, amy, dtm, slots);
-  }
-  finish_reduce(fin, amx, amy, dtm, bits, slots);
-}
-#endif  // JB_FAST
 
 // 1D: a block of NT threads handles a tile of NT-1 cells, so its NT faces
 // map one-to-one onto threads.
@@ -1834,12 +1587,12 @@ __global__ void k_halley(MP m, Grid g, const double* __restrict__ U, const doubl
 // being finished (SELECT); slots: where a NaN CFL candidate is flagged.
 // STRIPS: a boundary cell of a pressure-outlet / injector side also builds
 // its ghost state here (k_select leaves that to k_strips).
-template <int DIM, bool SELECT, bool ALPHA, bool CFL, bool STRIPS = true>
+template <int DIM, bool SELECT, bool ALPHA, bool CFL, bool STRIPS = true, class PT = float>
 __device__ __forceinline__ void select_cell(const MP& m, const Grid& g, const double* U, const double* aux_in,
                                             const double* cand, double* aux_out, double* strips,
                                             Slots* slots, unsigned mask, long long c, double& amx,
                                             double& amy, double& dtm, unsigned& st,
-                                            float* prims = nullptr) {
+                                            PT* prims = nullptr) {
   constexpr int nY = DIM == 1 ? 3 : 4;
   constexpr int nv = nY + NR;
   const long long nc = g.ncell;
@@ -1872,10 +1625,10 @@ __device__ __forceinline__ void select_cell(const MP& m, const Grid& g, const do
     }
     if (ALPHA || CFL) {
       Prim<DIM> pr = u_to_prim<DIM>(m, q, gamma, T);
-      if (DIM == 2 && prims) {  // float32 primitives for the next mixed-precision flux stage
-        prims[c] = (float)pr.u;
-        prims[nc + c] = (float)pr.v;
-        prims[2 * nc + c] = (float)pr.p;
+      if (DIM == 2 && prims) {  // primitives for the next flux stage's sweeps
+        prims[c] = (PT)pr.u;
+        prims[nc + c] = (PT)pr.v;
+        prims[2 * nc + c] = (PT)pr.p;
       }
       double sx = fabs(pr.u) + pr.a;
       double sy = fabs(pr.v) + pr.a;
@@ -1900,21 +1653,14 @@ __device__ __forceinline__ void select_cell(const MP& m, const Grid& g, const do
         int y = DIM == 1 ? 0 : (int)(c % g.ny);
         for (int side = 0; side < 2 * DIM; ++side) {
           int kind = g.bc[side];
-          if (kind != JB_BC_PRESSURE_OUTLET && kind != JB_BC_RDC_INJECTOR) continue;
+          if (kind != JB_BC_PRESSURE_OUTLET) continue;
           bool on = side == 0 ? x == 0 : side == 1 ? x == g.nx - 1 : side == 2 ? y == 0 : y == g.ny - 1;
           if (!on) continue;
           double gs[nv + 2];
-          if (kind == JB_BC_PRESSURE_OUTLET) {
-            double un = side < 2 ? q[1] / q[0] : q[2] / q[0];
-            if (side == 0 || side == 2) un = -un;
-            pressure_outlet_state<DIM>(m, q, gamma, T, un, g.Pb, gs);
-          } else {
-            if (DIM == 2) {
-              double Yi[NR];
-              for (int k = 0; k < NR; ++k) Yi[k] = g.Yinj[k * g.nx + x];
-              injector_state(m, q, gamma, T, Yi, g.inj_block_p, gs);
-            }
-          }
+          static_assert(!STRIPS || DIM == 1, "the 2D sides' strips are k_strips'");
+          double un = q[1] / q[0];
+          if (side == 0) un = -un;
+          pressure_outlet_state<DIM>(m, q, gamma, T, un, g.Pb, gs);
           int pos = side < 2 ? y : x;
           for (int f = 0; f < nv + 2; ++f) strips[strip_idx(g, side, f, pos)] = gs[f];
           Prim<DIM> pg = u_to_prim<DIM>(m, gs, gs[nv], gs[nv + 1]);
@@ -1927,24 +1673,25 @@ __device__ __forceinline__ void select_cell(const MP& m, const Grid& g, const do
   }
 }
 
-template <int DIM, bool SELECT, bool ALPHA, bool CFL>
+template <int DIM, bool SELECT, bool ALPHA, bool CFL, class PT>
 __global__ void __launch_bounds__(256, 4) k_select(MP m, Grid g, const double* __restrict__ U, const double* __restrict__ aux_in,
                          const double* __restrict__ cand, double* __restrict__ aux_out,
                          double* __restrict__ strips, Slots* slots, int midx, int aidx,
-                         float* __restrict__ prims) {
+                         PT* __restrict__ prims) {
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double amx = 0.0, amy = 0.0, dtm = __longlong_as_double(0x7ff0000000000000LL);
   unsigned st = 0;
   if (c < g.ncell)
-    select_cell<DIM, SELECT, ALPHA, CFL, false>(m, g, U, aux_in, cand, aux_out, strips, slots,
+    select_cell<DIM, SELECT, ALPHA, CFL, false, PT>(m, g, U, aux_in, cand, aux_out, strips, slots,
                                                 SELECT ? slots->mask[midx] : 0u, c, amx, amy, dtm, st,
-                                                ALPHA ? prims : nullptr);
+                                                ALPHA ? prims : (PT*)nullptr);
   if (ALPHA || CFL) block_reduce_store(amx, amy, dtm, st << 16, slots, aidx, ALPHA, CFL, -1);
 }
 
 // The ghost state of an outlet / injector side at boundary position pos from
 // the boundary cell's (U, gamma, T) into the strip, and its wave speeds
-// folded into amx, amy (nothing for other sides).
+// folded into amx, amy (nothing for other sides).  An injector side's
+// positions are a warp each (injector_state<true>), an outlet's a thread.
 template <int DIM>
 __device__ __forceinline__ void strip_one(const MP& m, const Grid& g, const double* U, const double* aux,
                                           double* strips, int side, int pos, double& amx, double& amy) {
@@ -1969,7 +1716,7 @@ __device__ __forceinline__ void strip_one(const MP& m, const Grid& g, const doub
       if (DIM == 2) {
         double Yi[NR];
         for (int k = 0; k < NR; ++k) Yi[k] = g.Yinj[k * g.nx + x];
-        injector_state(m, q, gamma, T, Yi, g.inj_block_p, gs);
+        injector_state<true>(m, q, gamma, T, Yi, g.inj_block_p, gs);
       }
     }
     for (int f = 0; f < nv + 2; ++f) strips[strip_idx(g, side, f, pos)] = gs[f];
@@ -1981,20 +1728,28 @@ __device__ __forceinline__ void strip_one(const MP& m, const Grid& g, const doub
 
 // Ghost strips of the pressure-outlet and injector sides (the padded grid's
 // entries that are not copies of interior cells) and their wave speeds into
-// the alpha maxima: one thread per boundary position, after the pass that
-// wrote the boundary cells' (gamma, T) into aux.  Positions: side 0 and 1
-// (x = 0, nx-1) ny each, then sides 2 and 3 (y = 0, ny-1) nx each.
+// the alpha maxima, after the pass that wrote the boundary cells' (gamma, T)
+// into aux.  Work items are the positions of the sides of those kinds in side
+// order, 32 threads (one warp) per position of an injector side; first[s] is
+// the first thread of side s (multiples of 32), first[4] their number.
+struct StripSides {
+  int first[5];
+};
 template <int DIM>
 __global__ void __launch_bounds__(128) k_strips(MP m, Grid g, const double* __restrict__ U,
                                                 const double* __restrict__ aux, double* __restrict__ strips,
-                                                Slots* slots, int aidx) {
+                                                Slots* slots, int aidx, StripSides ss) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ns = DIM == 1 ? 1 : g.ny;
   double amx = 0.0, amy = 0.0;
-  int side = -1, pos = 0;
-  if (t < 2 * ns) { side = t / ns; pos = t % ns; }
-  else if (DIM == 2 && t < 2 * ns + 2 * g.nx) { side = 2 + (t - 2 * ns) / g.nx; pos = (t - 2 * ns) % g.nx; }
-  strip_one<DIM>(m, g, U, aux, strips, side, pos, amx, amy);
+  if (t < ss.first[4]) {
+    int side = 0;
+#pragma unroll
+    for (int s = 1; s < 4; ++s)
+      if (t >= ss.first[s]) side = s;
+    const int i = t - ss.first[side], len = DIM == 1 ? 1 : side < 2 ? g.ny : g.nx;
+    const int pos = g.bc[side] == JB_BC_RDC_INJECTOR ? i >> 5 : i;
+    if (pos < len) strip_one<DIM>(m, g, U, aux, strips, side, pos, amx, amy);
+  }
   block_reduce_store(amx, amy, 0.0, 0u, slots, aidx, true, false, -1);
 }
 
@@ -2474,8 +2229,8 @@ __global__ void __launch_bounds__(128) k_halo_alpha_y(MP m, Grid g, Slots* slots
 #pragma unroll
       for (int f = 0; f < nv + 2; ++f) q[f] = g.haloy[haloy_idx(g, side, l, f, x)];
       Prim<2> pr = u_to_prim<2>(m, q, q[nv], q[nv + 1]);
-      amx = fabs(pr.u) + pr.a;
-      amy = fabs(pr.v) + pr.a;
+      amx = fmax(0.0, fabs(pr.u) + pr.a);  // NaN is skipped, as nanmax skips it
+      amy = fmax(0.0, fabs(pr.v) + pr.a);
     }
   }
   block_reduce_store(amx, amy, 0.0, 0u, slots, aidx, true, false, -1);
@@ -2502,8 +2257,8 @@ __global__ void __launch_bounds__(128) k_halo_alpha(MP m, Grid g, Slots* slots, 
 #pragma unroll
       for (int f = 0; f < nv + 2; ++f) q[f] = g.halo[halo_idx(g, side, l, f, y)];
       Prim<DIM> pr = u_to_prim<DIM>(m, q, q[nv], q[nv + 1]);
-      amx = fabs(pr.u) + pr.a;
-      amy = fabs(pr.v) + pr.a;
+      amx = fmax(0.0, fabs(pr.u) + pr.a);  // NaN is skipped, as nanmax skips it
+      amy = fmax(0.0, fabs(pr.v) + pr.a);
     }
   }
   block_reduce_store(amx, amy, 0.0, 0u, slots, aidx, true, false, -1);

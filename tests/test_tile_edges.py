@@ -1,0 +1,115 @@
+"""The fp64 and mixed builds' own flux kernels (2D x sweep + y runs, 1D line
+tiles) and the register form of the block temperature solve against the
+strict build's general kernels, at the edges of their tiles and segments:
+axes below, at and above the 128-cell y segments, the sweep segments, the 26-
+and 122-cell line tiles, and the 512-cell register slots of a block.
+
+The flux bound is relative to dt/dx max(|F| + alpha |U|) of each field, the
+size of the terms whose difference is taken: about 100 roundings of float64
+(1e-13) and of float32 (2e-5) per face value, weights included."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+ND = {"P0": 10 * 101325, "T0": 300, "R0": 369, "x0": 0.08}
+KEYS = ("left_boundary", "right_boundary", "bottom_boundary", "top_boundary")
+BCS = {"walls": ("slip_wall", "zero_gradient", "slip_wall", "no_slip_wall"),
+       "outlets": ("pressure_outlet", "no_slip_wall", "zero_gradient", "pressure_outlet"),
+       "ring": ("periodic", "periodic", "periodic", "periodic"),
+       "injector": ("periodic", "periodic", "rdc_injector", "pressure_outlet")}
+
+
+def _state(s, shape, nd=False, seed=5):
+    """A jump in the middle of every axis, waves and 1 % of noise."""
+    rng = np.random.default_rng(seed)
+    full = (1,) + shape
+    ax = np.meshgrid(*[np.arange(n) / n for n in shape], indexing="ij")
+    hot = sum(a > 0.45 for a in ax) / len(shape)
+    wave = 0.05 * sum(np.sin(5 * a + k) for k, a in enumerate(ax))
+    P = (1.0 + 8.0 * hot + wave) * (1 + 0.01 * rng.uniform(-1, 1, shape))
+    T = (1.2 + 5.0 * hot + wave) * (1 + 0.01 * rng.uniform(-1, 1, shape))
+    if nd:
+        P, T = P * 0.08, T
+    else:
+        P, T = P * 101325.0, T * 300.0
+    Y = rng.uniform(0.0, 0.1, (8,) + shape)
+    cu = lambda a: torch.as_tensor(np.ascontiguousarray(a), device="cuda")  # noqa: E731
+    c = 1.0 if nd else 300.0
+    vel = [cu((c * (0.4 * hot + rng.uniform(-0.2, 0.2, shape))).reshape(full)) for _ in shape]
+    return s.state_from_PTY(cu(P.reshape(full)), cu(T.reshape(full)), cu(Y), vel)
+
+
+def _pair(dim, nx, ny, bc, prec, nd, d):
+    from janc_b200 import mechanism as jm
+    from janc_b200.solver import Solver
+    mech = jm.load(jm.DEFAULT_MECHANISM, ND if nd else None)
+    b = dict(zip(KEYS[: 2 * dim], BCS[bc]))
+    mk = lambda p: Solver(dim, nx, ny if dim == 2 else None, d, d if dim == 2 else None, b, mech,  # noqa: E731
+                          precision=p)
+    return mk("fp64_strict"), mk(prec)
+
+
+def _check_flux(s0, s1, U, aux, theta, d, prec):
+    dt = 1e-8
+    a, b = s0.flux_func(U, aux, dt=dt, theta=theta), s1.flux_func(U, aux, dt=dt, theta=theta)
+    prim = s0.u_to_prim(U, aux)
+    p, c = prim[-2], prim[-1]
+    speed = sum(v.abs() for v in prim[1:1 + s0.dim]) + c
+    tol = 1e-13 if prec == "fp64" else 2e-5
+    for f in range(s0.nv):
+        scale = float((speed * (U[f:f + 1].abs())).max())
+        if f <= s0.dim:
+            scale += float(p.max())
+        if f == s0.dim + 1:
+            scale += float((speed * p).max())
+        assert float((a[f] - b[f]).abs().max()) <= tol * dt / d * scale, f
+    assert s1.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx,ny,bc", [(4, 4, "walls"), (7, 31, "outlets"), (13, 127, "ring"), (6, 128, "walls"),
+                                      (9, 129, "injector"), (5, 131, "outlets"), (50, 257, "walls"),
+                                      (97, 6, "injector"), (61, 255, "ring")])
+def test_sweep_flux_matches_the_strict_tiles(nx, ny, bc, prec):
+    nd = bc == "injector"
+    d = 0.0025 if nd else 1e-4
+    s0, s1 = _pair(2, nx, ny, bc, prec, nd, d)
+    U, aux = _state(s0, (nx, ny), nd)
+    theta = {"Pb": 0.1 if nd else 101325.0}
+    if nd:
+        theta["Yinj"] = np.concatenate([[0.028, 0.22], 1e-20 * np.ones(6)])
+    _check_flux(s0, s1, U, aux, theta if bc in ("outlets", "injector") else None, d, prec)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx,bc", [(4, "ring"), (25, "walls"), (26, "outlets"), (27, "ring"), (53, "walls"),
+                                   (15392, "outlets"), (15393, "walls"), (15494, "ring"), (15495, "outlets")])
+def test_line_flux_matches_the_strict_tiles(nx, bc, prec):
+    s0, s1 = _pair(1, nx, 1, bc, prec, False, 5e-5)
+    U, aux = _state(s0, (nx,))
+    _check_flux(s0, s1, U, aux, {"Pb": 101325.0} if bc == "outlets" else None, 5e-5, prec)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("X,Y", [(7, 7), (16, 32), (19, 27), (32, 32), (41, 25), (44, 35), (45, 45), (46, 46)])
+def test_block_update_matches_the_strict_loop(X, Y):
+    """update_aux of blocks of 49 .. 2116 cells (one to four cells a thread,
+    and the general loop above), guesses 20 % off.  Both stop when the block's
+    largest residual is within 5e-9 J/kg, so T agrees within 2 * 5e-9 / cv and
+    its rounding: 1e-12 relative."""
+    from janc_b200.solver import Solver
+    d = 1e-4
+    s0 = Solver(2, 32, 32, d, d, precision="fp64_strict")
+    s1 = Solver(2, 32, 32, d, d, precision="fp64")
+    U, aux = _state(s0, (3 * X, Y))
+    rng = np.random.default_rng(2)
+    blk = lambda a: a.reshape(a.shape[0], 3, X, Y).transpose(0, 1).contiguous()  # noqa: E731
+    Ub, ab = blk(U), blk(aux)
+    guess = ab.clone()
+    guess[:, 1] *= torch.as_tensor(rng.uniform(0.8, 1.2, (3, X, Y)), device="cuda")
+    r0, r1 = s0.amr_update_aux(Ub, guess), s1.amr_update_aux(Ub, guess)
+    assert float(((r1 - r0).abs() / r0.abs()).max()) <= 1e-12
+    assert s1.status() == 0

@@ -21,7 +21,7 @@ OBJ = os.path.join(HERE, "_objs")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 # the slowest units first: they start before the pool fills
-UNITS = [("jb_ensemble.cu", ["-fmad=true"]), ("jb_fast_flux32.cu", ["-fmad=true"]),
+UNITS = [("jb_ensemble.cu", ["-fmad=true"]), ("jb_fast_run.cu", ["-fmad=true"]), ("jb_fast_flux32.cu", ["-fmad=true"]),
          ("jb_fast_god32.cu", ["-fmad=true"]), ("jb_fast_flux64.cu", ["-fmad=true"]),
          ("jb_fast_god64.cu", ["-fmad=true"]), ("jb_fast.cu", ["-fmad=true"]),
          ("jb_strict_flux.cu", ["-fmad=false"]), ("jb_strict_god.cu", ["-fmad=false"]),

@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(AMR_UNT) k_amr_update_cells(MP m, long long nc
         const double res = (h - R[k] * T[k]) - e[k], d1 = cp[k] - R[k];
         if (fabs(res) > HALLEY_TOL) bits |= 1u;
         if (res != res) bits |= 2u;
-        Tn[k] = T[k] + ((-2.0 * res) * d1) / ((2.0 * (d1 * d1)) - res * dcp);
+        Tn[k] = T[k] + ((-2.0 * res) * d1) * rcp_nr((2.0 * (d1 * d1)) - res * dcp);
       }
     }
     const int go = __syncthreads_or(bits & 1u), bad = __syncthreads_or(bits & 2u);
@@ -417,12 +417,15 @@ __global__ void __launch_bounds__(128, 3) k_amr_chem(MP m, AmrBlocks B, const do
     const double T = Ib[(nv + 1) * nc + c];
     const double rho = Ib[c];
     double Y8[NR], S[NR];
-#pragma unroll
-    for (int k = 0; k < NR; ++k) Y8[k] = Ib[(nY + k) * nc + c] / rho;
 #if JB_FAST
+    const double ri = 1.0 / rho;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) Y8[k] = Ib[(nY + k) * nc + c] * ri;
     if (GEN) chem_cell_gen(m, rho, Y8, T, dt, S, st, shc + threadIdx.x, blockDim.x);
     else chem_cell(m, rho, Y8, T, dt, S, st);
 #else
+#pragma unroll
+    for (int k = 0; k < NR; ++k) Y8[k] = Ib[(nY + k) * nc + c] / rho;
     chem_cell(m, rho, Y8, T, dt, S, st);
 #endif
 #pragma unroll

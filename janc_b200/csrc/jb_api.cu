@@ -28,7 +28,7 @@ struct jb_handle {
   double* auxw[2];     // stage aux [2][ncell]
   double* cand;        // Halley iterates [6][ncell]
   double* strips;      // ghost strips [4][nv+2][lstrip]
-  jb_slots* slots;
+  jb_slots* slots;     // the step's slots, then two more sets and 16 barrier words (1D runs)
   long long ws_bytes;
   // optional per-kernel timing of jb_advance (jb_set_kernel_timing)
   int timing;
@@ -178,9 +178,16 @@ int jb_create(const jb_mech_params* mech, int dim, int nx, int ny, double dx, do
   for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&h->auxw[i], bytes_aux);
   if (e == cudaSuccess) e = cudaMalloc(&h->cand, bytes_cand);
   if (e == cudaSuccess) e = cudaMalloc(&h->strips, bytes_strip);
-  if (e == cudaSuccess) e = cudaMalloc(&h->slots, sizeof(jb_slots));
+  const size_t bytes_slots = 3 * sizeof(jb_slots) + 16 * sizeof(unsigned);
+  if (e == cudaSuccess) e = cudaMalloc(&h->slots, bytes_slots);
   if (e == cudaSuccess) e = cudaMemset(h->strips, 0, bytes_strip);
-  if (e == cudaSuccess) e = cudaMemset(h->slots, 0, sizeof(jb_slots));
+  if (e == cudaSuccess) e = cudaMemset(h->slots, 0, bytes_slots);
+  for (int i = 1; i < 3 && e == cudaSuccess; ++i) {  // as a run's last block leaves them
+    jb_slots clear;
+    std::memset(&clear, 0, sizeof(clear));
+    clear.dtmin_next = 0x7ff0000000000000ull;
+    e = cudaMemcpy(h->slots + i, &clear, sizeof(clear), cudaMemcpyHostToDevice);
+  }
   // 2D sweeps (jb_sweep.cuh): the primitives of the stage state (mixed: and
   // of the state being written, two buffers used in turn), then the x flux
   // differences; float32 in mixed, float64 in fp64
@@ -192,7 +199,7 @@ int jb_create(const jb_mech_params* mech, int dim, int nx, int ny, double dx, do
     jb_destroy(h);
     return JB_ERR_CUDA;
   }
-  h->ws_bytes = (long long)(2 * bytes_W + 2 * bytes_aux + bytes_cand + bytes_strip + sizeof(jb_slots) + bytes_fwork);
+  h->ws_bytes = (long long)(2 * bytes_W + 2 * bytes_aux + bytes_cand + bytes_strip + bytes_slots + bytes_fwork);
   *out = h;
   return JB_OK;
 }
@@ -408,6 +415,16 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
   // and fp64, and the mixed 1D Godunov path): the kernels write the Halley
   // iterates and a select pass after each picks the reference's iteration
   // count.
+  // short 1D LF / WENO5-JS lines: the whole run as one launch
+  if (d == 1 && o.line_run && chemistry && !rec && !probe_p && !h->xch && !g.visc && !h->timing &&
+      g.scheme == JB_FLUX_LF && g.recon == JB_RECON_WENO5) {
+    const jb::jb_line_io io = {U,          aux,      U_out,   aux_out,  h->W[0],
+                               h->W[1],    h->auxw[0], h->auxw[1], h->cand, h->strips,
+                               h->slots,   reinterpret_cast<unsigned*>(h->slots + 3), dt_fixed, use_cfl ? cfl : 0.0,
+                               nsteps,     dt_hist};
+    cudaError_t e = cudaSuccess;
+    if (o.line_run(m, g, io, st, e)) return check_cuda(h, e, "line run");
+  }
   const bool pc = o.per_cell && (d == 2 || g.scheme == JB_FLUX_LF || g.scheme == JB_FLUX_SW);
   // 2D sweeps: u, v, p of the current state (pin); mixed: and the buffer the
   // next kernel writes (pout), swapped after each writer (fp64: the select

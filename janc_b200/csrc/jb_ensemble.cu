@@ -27,13 +27,14 @@
 // whose instances keep the reference's global stop of the temperature
 // solve).  The mixed variant solves each cell's temperature where its new
 // state is written (as its single-case step does), so no select pass
-// follows and a step has four phases:
+// follows and a step has three phases:
 //   stage 1  U, aux      -> W0, A0      (alpha 1)
 //   stage 2  W0, A0, U   -> W1, A1      (alpha 2)
-//   stage 3  W1, A1, U   -> W0, A0
-//   chem     W0, A0      -> U, aux      (alpha of the next stage 1, CFL
+//   stage 3  W1, A1, U   -> W0, A0, then each CTA's chemistry of its own
+//            cells W0, A0 -> U, aux     (alpha of the next stage 1, CFL
 //                                        minimum of the next dt)
-// each also writing the outlet ghost strips of its new state.  Slot sets
+// each also writing the outlet ghost strips of its new state, into three
+// buffers in turn: the U^n, U1 and U2 ghosts.  Slot sets
 // alternate between even and odd steps, so clearing one never races with
 // reading the other.
 #define JB_NS ens
@@ -160,7 +161,7 @@ __device__ __noinline__ void select_pass(const jb_ens_inst& I, int rank, const d
 // visible to its own threads after a block barrier), their wave speeds
 // folded into amx.  chunk: cells per work item of the pass that wrote them.
 __device__ __forceinline__ void ens_strips(const jb_ens_inst& I, int rank, int chunk, int nitems,
-                                           const double* U, const double* aux, double& amx) {
+                                           const double* U, const double* aux, double* strips, double& amx) {
   __syncthreads();
   if (threadIdx.x < 2) {
     const int side = threadIdx.x;
@@ -169,7 +170,7 @@ __device__ __forceinline__ void ens_strips(const jb_ens_inst& I, int rank, int c
     if ((kind == JB_BC_PRESSURE_OUTLET || kind == JB_BC_RDC_INJECTOR) && (x / chunk) % I.ncta == rank &&
         x / chunk < nitems) {
       double amy = 0.0;
-      strip_one<1>(c_mech, I.g, U, aux, I.strips, side, 0, amx, amy);
+      strip_one<1>(c_mech, I.g, U, aux, strips, side, 0, amx, amy);
     }
   }
 }
@@ -177,39 +178,44 @@ __device__ __forceinline__ void ens_strips(const jb_ens_inst& I, int rank, int c
 // One RK stage over this CTA's tiles.  Global-stop mode (float64 tiles):
 // Halley mask into s->mask[STAGE - 1]; per-cell mode (float tiles of the
 // mixed variant): each cell's temperature solve into fin.aux, and the new
-// state's alpha (with the outlet strips) into s->ax[fin.aidx].
+// state's alpha (with the outlet strips) into s->ax[fin.aidx].  sin, sout:
+// the ghost strip buffers of the input and of the new state (a neighbour may
+// still read the former while the boundary CTA writes the latter).
 template <int STAGE, class R, int NT>
 __device__ __noinline__ void flux_pass(const jb_ens_inst& I, int rank, const double* Uk, const double* auxk,
                                        double* out, double alpha, double dt, Slots* s, unsigned char* smraw,
-                                       const jb_fin& fin) {
+                                       const jb_fin& fin, int sin, int sout) {
   unsigned bits = 0;
   double amx = 0.0, dtm = __longlong_as_double(0x7ff0000000000000LL);
   for (int t = rank; t < I.ntiles; t += I.ncta)
-    bits |= line_tile<STAGE, R, NT, NT - ENS_HALO>(c_mech, I.g, Uk, auxk, I.U, out, fin, I.strips, alpha, dt,
+    bits |= line_tile<STAGE, R, NT, NT - ENS_HALO>(c_mech, I.g, Uk, auxk, I.U, out, fin, I.strips + sin, alpha, dt,
                                                    t * (NT - ENS_HALO), smraw, amx, dtm, s);
-  if (fin.aux && fin.aidx >= 0) ens_strips(I, rank, NT - ENS_HALO, I.ntiles, out, fin.aux, amx);
+  if (fin.aux && fin.aidx >= 0) ens_strips(I, rank, NT - ENS_HALO, I.ntiles, out, fin.aux, I.strips + sout, amx);
   finish_reduce(fin, amx, 0.0, dtm, bits, s);
 }
 
-// Per-cell mode: chemistry of this CTA's cells at the stage-3 temperature
-// in A0, then each cell's temperature solve into aux, the new state's alpha
-// (with the outlet strips) into s->ax[3] and its CFL minimum.
+// Per-cell mode: chemistry of the cells of this CTA's own flux tiles at the
+// stage-3 temperature in A0 (each thread takes the cells it finished there,
+// so no barrier separates it from stage 3), then each cell's temperature
+// solve into aux, the new state's alpha (with the outlet strips) into
+// s->ax[3] and its CFL minimum.
 template <int NT>
 __device__ __noinline__ void chem_pass_cell(const jb_ens_inst& I, int rank, double dt, Slots* s,
                                             unsigned char* smraw) {
+  constexpr int S = NT - ENS_HALO;
   const Grid& g = I.g;
   const long long nc = g.ncell;
   double* sh = reinterpret_cast<double*>(smraw) + threadIdx.x;
   const jb_fin fin = jb_fin_cell(I.aux, nullptr, 3, 1);
   unsigned bits = 0, st = 0;
   double amx = 0.0, amy = 0.0, dtm = __longlong_as_double(0x7ff0000000000000LL);
-  for (int j = rank; j < I.nchunks; j += I.ncta) {
-    long long c = (long long)j * NT + threadIdx.x;
-    if (c < nc)
+  for (int t = rank; t < I.ntiles; t += I.ncta) {
+    const long long c = (long long)t * S + threadIdx.x;
+    if (threadIdx.x < S && c < nc)
       chem_cell_step<1, false, true, true>(c_mech, g, I.W0, I.A0[nc + c], I.U, fin, c, dt, sh, bits, st, amx, amy,
                                            dtm, s);
   }
-  ens_strips(I, rank, NT, I.nchunks, I.U, I.aux, amx);
+  ens_strips(I, rank, S, I.ntiles, I.U, I.aux, I.strips, amx);
   finish_reduce(fin, amx, 0.0, dtm, bits | (st << 16), s);
 }
 
@@ -271,40 +277,39 @@ __global__ void __launch_bounds__(NT, Shape<NT>::MINB)
                                   : I.dt;
     if (dt_hist && rank == 0 && tid == 0) dt_hist[(long long)ii * nsteps + step] = dt;
     if constexpr (sizeof(R) == sizeof(float)) {
-      // mixed variant, per-cell temperature solves: four phases a step
+      // mixed variant, per-cell temperature solves: three phases a step
       // stage 1: U1 = U + L(U), (gamma, T)_1 and alpha 1
       flux_pass<1, R, NT>(I, rank, I.U, I.aux, I.W0, bitsd(__ldcg(&prv->ax[3])), dt, cur, smraw,
-                          jb_fin_cell(I.A0, nullptr, 1, 0));
+                          jb_fin_cell(I.A0, nullptr, 1, 0), 0, 1);
       JB_ENS_SYNC();
       if (rank == 0 && tid == 0) slots_clear(prv);  // every CTA has read it
       // stage 2: U2 = 3/4 U + 1/4 (U1 + L(U1))
       flux_pass<2, R, NT>(I, rank, I.W0, I.A0, I.W1, bitsd(__ldcg(&cur->ax[1])), dt, cur, smraw,
-                          jb_fin_cell(I.A1, nullptr, 2, 0));
+                          jb_fin_cell(I.A1, nullptr, 2, 0), 1, 2);
       JB_ENS_SYNC();
       // stage 3: U3 = 1/3 U + 2/3 (U2 + L(U2)), T3 into A0
       flux_pass<3, R, NT>(I, rank, I.W1, I.A1, I.W0, bitsd(__ldcg(&cur->ax[2])), dt, cur, smraw,
-                          jb_fin_cell(I.A0, nullptr, -1, 0));
-      JB_ENS_SYNC();
-      // chemistry, the final solve, alpha and CFL minimum of the next step
+                          jb_fin_cell(I.A0, nullptr, -1, 0), 2, 2);
+      // chemistry of the own cells, the final solve, alpha and CFL minimum of the next step
       chem_pass_cell<NT>(I, rank, dt, cur, smraw);
       JB_ENS_SYNC();
     } else {
     // stage 1: U1 = U + L(U)
     flux_pass<1, R, NT>(I, rank, I.U, I.aux, I.W0, bitsd(__ldcg(&prv->ax[3])), dt, cur, smraw,
-                        jb_fin_cand(I.cand, 0));
+                        jb_fin_cand(I.cand, 0), 0, 0);
     JB_ENS_SYNC();
     if (rank == 0 && tid == 0) slots_clear(prv);  // every CTA has read it
     select_pass<true, false, NT>(I, rank, I.W0, nullptr, I.A0, __ldcg(&cur->mask[0]), cur, 1);
     JB_ENS_SYNC();
     // stage 2: U2 = 3/4 U + 1/4 (U1 + L(U1))
     flux_pass<2, R, NT>(I, rank, I.W0, I.A0, I.W1, bitsd(__ldcg(&cur->ax[1])), dt, cur, smraw,
-                        jb_fin_cand(I.cand, 1));
+                        jb_fin_cand(I.cand, 1), 0, 0);
     JB_ENS_SYNC();
     select_pass<true, false, NT>(I, rank, I.W1, nullptr, I.A1, __ldcg(&cur->mask[1]), cur, 2);
     JB_ENS_SYNC();
     // stage 3: U3 = 1/3 U + 2/3 (U2 + L(U2))
     flux_pass<3, R, NT>(I, rank, I.W1, I.A1, I.W0, bitsd(__ldcg(&cur->ax[2])), dt, cur, smraw,
-                        jb_fin_cand(I.cand, 2));
+                        jb_fin_cand(I.cand, 2), 0, 0);
     JB_ENS_SYNC();
     chem_pass<NT>(I, rank, halley_count(__ldcg(&cur->mask[2])), dt, cur, smraw);
     JB_ENS_SYNC();
@@ -396,7 +401,7 @@ struct jb_ensemble {
   std::vector<jb_ens_inst> host_insts;
   double* state;                // per instance: U [11][nx] then aux [2][nx]
   double* work;                 // per instance: W0, W1 [11][nx], A0, A1 [2][nx], cand [6][nx]
-  double* strips;               // [n][4][13]
+  double* strips;               // [n][4][13][3]
   jb_slots* slots;              // [n][2]
   unsigned* sync;               // [n] barrier counters, then a jb_ens_ctl
   jb_ens_ctl* ctl;
@@ -456,7 +461,7 @@ bool assign(const std::vector<int>& nx, int block, int total, std::vector<int>& 
   std::vector<int> tiles(n);
   int tmax = 0;
   for (int i = 0; i < n; ++i) {
-    tiles[i] = (nx[i] + block - 2) / (block - 1);
+    tiles[i] = (nx[i] + block - ENS_HALO - 1) / (block - ENS_HALO);
     tmax = std::max(tmax, tiles[i]);
   }
   if (total < n) return false;
@@ -571,14 +576,14 @@ int jb_ens_create(const jb_mech_params* mech, int n, const int* nx, const double
   e->cells_alloc = o;
   cudaError_t ce = cudaMalloc(&e->state, sizeof(double) * 13 * (size_t)o);
   if (ce == cudaSuccess) ce = cudaMalloc(&e->work, sizeof(double) * 32 * (size_t)o);
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->strips, sizeof(double) * 52 * (size_t)n);
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->strips, sizeof(double) * ENS_STRIP * (size_t)n);
   if (ce == cudaSuccess) ce = cudaMalloc(&e->slots, sizeof(jb_slots) * 2 * (size_t)n);
   if (ce == cudaSuccess) ce = cudaMalloc(&e->sync, sync_bytes(n));
   if (ce == cudaSuccess) ce = cudaMalloc(&e->d_insts, sizeof(jb_ens_inst) * (size_t)n);
   if (ce == cudaSuccess) ce = cudaMalloc(&e->d_mech, sizeof(jb_mech_params));
   if (ce == cudaSuccess) ce = cudaMemcpy(e->d_mech, &e->mech, sizeof(jb_mech_params), cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMemset(e->state, 0, sizeof(double) * 13 * (size_t)o);
-  if (ce == cudaSuccess) ce = cudaMemset(e->strips, 0, sizeof(double) * 52 * (size_t)n);
+  if (ce == cudaSuccess) ce = cudaMemset(e->strips, 0, sizeof(double) * ENS_STRIP * (size_t)n);
   if (ce == cudaSuccess) ce = cudaMemset(e->slots, 0, sizeof(jb_slots) * 2 * (size_t)n);
   if (ce == cudaSuccess) ce = cudaMemset(e->sync, 0, sync_bytes(n));
   if (ce != cudaSuccess) {
@@ -606,7 +611,7 @@ int jb_ens_create(const jb_mech_params* mech, int n, const int* nx, const double
     g.Pb = 0.0;
     g.Yinj = nullptr;
     g.inj_block_p = 1.0;
-    g.lstrip = 1;
+    g.lstrip = ENS_STRIP / 52;  // strip buffers
     const size_t c = (size_t)nx[i];
     I.U = e->state + 13 * (size_t)e->off[i];
     I.aux = I.U + 11 * c;
@@ -616,7 +621,7 @@ int jb_ens_create(const jb_mech_params* mech, int n, const int* nx, const double
     I.A0 = w + 22 * c;
     I.A1 = w + 24 * c;
     I.cand = w + 26 * c;
-    I.strips = e->strips + 52 * (size_t)i;
+    I.strips = e->strips + ENS_STRIP * (size_t)i;
     I.slots = e->slots + 2 * (size_t)i;
     I.bar = e->sync + i;
     I.dt_hist = nullptr;

@@ -7,11 +7,13 @@
 // A flux tile's padded cells are one per thread of its block: block - ENS_HALO
 // cells and the 3 + 3 halo cells.
 #define ENS_HALO 6
+// Doubles of an instance's ghost strips [4][13][3]: sides, fields, buffers
+#define ENS_STRIP 156
 
 // One instance (a detonation tube).  Every pointer is device memory owned by
 // the ensemble; the state U / aux is advanced in place.
 typedef struct jb_ens_inst {
-  jb_grid g;            // nx = cells, ny = 1, ncell = nx, lstrip = 1
+  jb_grid g;            // nx = cells, ny = 1, ncell = nx, lstrip = 3 (strip buffers)
   double* U;            // [11][nx] conserved state
   double* aux;          // [2][nx]  gamma, T
   double* W0;           // [11][nx] RK stage buffers
@@ -19,7 +21,7 @@ typedef struct jb_ens_inst {
   double* A0;           // [2][nx]  aux of the RK stages
   double* A1;
   double* cand;         // [6][nx]  Halley iterates
-  double* strips;       // [4][13][1] ghost states of outlet sides
+  double* strips;       // [4][13][3] ghost states of outlet sides
   jb_slots* slots;      // [2]: even / odd steps
   unsigned* bar;        // arrival counter of this instance's CTA group
   double* dt_hist;      // [max steps] time steps of the last run, or null

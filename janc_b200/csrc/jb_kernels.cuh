@@ -47,6 +47,21 @@ __device__ __forceinline__ double bitsd(unsigned long long b) {
   return __longlong_as_double((long long)b);
 }
 
+#if JB_FAST
+// 1 / x of a float64 x whose size and reciprocal are normal numbers: the
+// hardware's approximate reciprocal refined by one third-order step of the
+// Newton family, r (1 + e + e^2) with e = 1 - x r (measured: e below 1e-6, so
+// the step's error e^3 is below half an ulp; the result within 2 ulp).  No
+// range fix-up and no branch, so that several of them interleave.  0 and
+// infinity give NaN.
+__device__ __forceinline__ double rcp_nr(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+#endif
+
 // ---------------------------------------------------------------------------
 // block reductions
 // ---------------------------------------------------------------------------
@@ -275,7 +290,7 @@ __device__ __forceinline__ unsigned halley_iterates_fast(const MP& m, double e, 
     const double d1 = cp - R;
     if (fabs(res) > HALLEY_TOL) bits |= 1u << i;
     if (res != res) bits |= 1u << (8 + i);
-    const double dT = ((-2.0 * res) * d1) / ((2.0 * (d1 * d1)) - res * d2);
+    const double dT = ((-2.0 * res) * d1) * rcp_nr((2.0 * (d1 * d1)) - res * d2);
     T = T + dT;
     cand[i + 1] = T;
   }
@@ -411,7 +426,7 @@ __device__ __forceinline__ double halley_cell(const MP& m, double e, const doubl
 #pragma unroll 1
     for (int i = 0; i < HALLEY_MAX && halley_go(res, polished); ++i) {
       const double d1 = cp - R;
-      T = T + ((-2.0 * res) * d1) / ((2.0 * (d1 * d1)) - res * d2);
+      T = T + ((-2.0 * res) * d1) * rcp_nr((2.0 * (d1 * d1)) - res * d2);
       const bool lo_i = T < Tcr;
       if (lo_i != lo) {  // the iterate crossed the range boundary (rare)
         lo = lo_i;
@@ -612,7 +627,7 @@ __device__ __forceinline__ void injector_eval(double M, double P3, double Ri, do
 // sequential bisection can meet, formed by the same operations), and every
 // lane walks the tree by the ballots, so the result is the sequential one.
 // Four dependent evaluations instead of 20: 35.6 us a launch at 1600
-// positions before, 12 us now.
+// positions before, 11 us now.
 template <bool WARP>
 __device__ void injector_state(const MP& m, const double* q, double gamma, double T,
                                const double* Yinj8, double block_p, double* out) {
@@ -707,17 +722,6 @@ constexpr double W_13 = 1.0 / 3.0, W_76 = 7.0 / 6.0, W_116 = 11.0 / 6.0;
 constexpr double W_m16 = -1.0 / 6.0, W_56 = 5.0 / 6.0, W_16 = 1.0 / 6.0;
 
 #if JB_FAST
-// 1 / x of a float64 x > 0 away from the ends of the range: the hardware's
-// approximate reciprocal refined by one third-order step of the Newton
-// family, r (1 + e + e^2) with e = 1 - x r (its error e^3 is below half an
-// ulp).  No range fix-up and no branch, so that several of them interleave.
-__device__ __forceinline__ double rcp_pos(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 // Weighted correction of a WENO5-JS value (reconstruction/WENO5_JS.py) at the
 // face behind cell j, value = f_j + num / (6 den), from the four differences
 // around it, dmm = f_{j-1} - f_{j-2}, dm = f_j - f_{j-1}, dp = f_{j+1} - f_j,
@@ -756,7 +760,7 @@ __device__ __forceinline__ double weno_L(double fjm2, double fjm1, double fj, do
   double num, den;
   weno_side(dmm, dm, dp, dpp, weno_curv(dmm, dm, 4 * W_EPS), weno_curv(dm, dp, 4 * W_EPS),
             weno_curv(dp, dpp, 4 * W_EPS), num, den);
-  return fma(1.0 / 6.0, num * rcp_pos(den), fj);
+  return fma(1.0 / 6.0, num * rcp_nr(den), fj);
 }
 // right-biased value at j-1/2 (interface_R_*): the mirrored stencil
 __device__ __forceinline__ double weno_R(double fjm2, double fjm1, double fj, double fjp1, double fjp2) {
@@ -1812,7 +1816,7 @@ __device__ __forceinline__ void lu_solve(double (&J)[NR][NR], double (&b)[NR], d
     if (J[c][c] == 0.0) st |= JB_ERR_SINGULAR;
 #if JB_FAST
     // one reciprocal per pivot (kept for the back substitution)
-    ipv[c] = 1.0 / J[c][c];
+    ipv[c] = rcp_nr(J[c][c]);
 #endif
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
@@ -1997,17 +2001,34 @@ __device__ __forceinline__ void chem_cell_gen(const MP& m, double rho, const dou
   for (int k = 0; k < NR; ++k) {
     const double xc = X[k] < 1e-50 ? 1e-50 : X[k];
     Xc[k] = xc;
-    rMX[k] = m.invM[k] / xc;
+    rMX[k] = m.invM[k] * rcp_nr(xc);
   }
   const double lT = log(T), invT = 1.0 / T, lT0T = lT + m.lnT0;
-  // get_gibbs (reaction_model.py:78-89): g = s/R - h/(R T); E = exp(g)
+  // get_gibbs (reaction_model.py:78-89): g = s/R - h/(R T); E = exp(g).  One
+  // branch where all species switch ranges at the same temperature, so that
+  // one range's coefficients are read straight from the parameter bank.
+  double gk[NR];
+  if (m.tcr_uniform) {
+    if (T < m.Tcr[0]) {
+#pragma unroll
+      for (int k = 0; k < NR; ++k) gk[k] = poly5(m.s_lo[k], T) + m.lg_lo[k] * lT0T - poly6(m.hc_lo[k], T) * invT;
+    } else {
+#pragma unroll
+      for (int k = 0; k < NR; ++k) gk[k] = poly5(m.s_hi[k], T) + m.lg_hi[k] * lT0T - poly6(m.hc_hi[k], T) * invT;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const bool lo = T < m.Tcr[k];
+      const double h = lo ? poly6(m.hc_lo[k], T) : poly6(m.hc_hi[k], T);
+      const double s = lo ? poly5(m.s_lo[k], T) + m.lg_lo[k] * lT0T : poly5(m.s_hi[k], T) + m.lg_hi[k] * lT0T;
+      gk[k] = s - h * invT;
+    }
+  }
 #pragma unroll
   for (int k = 0; k < NR; ++k) {
-    const bool lo = T < m.Tcr[k];
-    const double h = lo ? poly6(m.hc_lo[k], T) : poly6(m.hc_hi[k], T);
-    const double s = lo ? poly5(m.s_lo[k], T) + m.lg_lo[k] * lT0T : poly5(m.s_hi[k], T) + m.lg_hi[k] * lT0T;
-    E[k] = exp(s - h * invT);
-    iE[k] = 1.0 / E[k];
+    E[k] = exp(gk[k]);
+    iE[k] = rcp_nr(fmin(fmax(E[k], 1e-300), 1e300));  // finite where E over- or underflows
   }
   chem_rates_gen(m, lT, invT, T / m.pref, m.pref * invT, X, Xc, E, iE, sh, stride, w);
   double J[NR][NR];
@@ -2044,8 +2065,14 @@ __device__ __forceinline__ void chem_cell_step(const MP& m, const Grid& g, const
 #endif
     double rho = q[0];
     double Y8[NR], S[NR];
+#if JB_FAST
+    const double ri = 1.0 / rho;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] * ri;
+#else
 #pragma unroll
     for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] / rho;
+#endif
 #if JB_FAST
     if (GEN) chem_cell_gen(m, rho, Y8, T, dt, S, st, sh, blockDim.x);
     else chem_cell(m, rho, Y8, T, dt, S, st);

@@ -23,6 +23,19 @@ struct jb_amr_io {
   long long osU, osA;
 };
 
+// A run of nsteps 1D steps with chemistry (advance_impl's sequence): the
+// step's buffers, the handle's slots followed by two more sets, and the three
+// barrier words of the persistent launch (zero between launches).
+struct jb_line_io {
+  const double *U, *aux;
+  double *U_out, *aux_out, *W0, *W1, *A0, *A1, *cand, *strips;
+  jb_slots* slots;
+  unsigned* bar;
+  double dt_fixed, cfl;
+  int nsteps;
+  double* dt_hist;
+};
+
 struct Ops {
   const char* name;
   // stepping (jb_advance) solves each new state's temperature per cell
@@ -94,6 +107,10 @@ struct Ops {
                             double* aux_out, jb_slots* slots, cudaStream_t st);
   cudaError_t (*amr_chem)(const jb_mech_params& m, int nb, int bx, int by, const double* blk, double* out,
                           jb_slots* slots, double dt, cudaStream_t st);
+  // 1D LF / WENO5-JS runs as one persistent launch: false (nothing launched)
+  // where that does not apply; null in the strict build
+  bool (*line_run)(const jb_mech_params& m, const jb_grid& g, const jb_line_io& io, cudaStream_t st,
+                   cudaError_t& err);
 };
 
 // Doubles of the viscous scratch (node planes and node fluxes) of a grid.

@@ -80,7 +80,7 @@ __device__ __forceinline__ void weno_side(f2 dmm, f2 dm, f2 dp, f2 dpp, f2 Da, f
 // divergence.
 __device__ __forceinline__ double face_value(double bl, double nl, double dl, double br, double nr, double dr) {
   // each side's value rounded by itself, as the reference rounds L and R
-  return fma(1.0 / 6.0, nl * rcp_pos(dl), bl) + fma(-1.0 / 6.0, nr * rcp_pos(dr), br);
+  return fma(1.0 / 6.0, nl * rcp_nr(dl), bl) + fma(-1.0 / 6.0, nr * rcp_nr(dr), br);
 }
 __device__ __forceinline__ float face_value(float bl, float nl, float dl, float br, float nr, float dr) {
   return fmaf(1.f / 6.f, fmaf(nl, dr, -(nr * dl)) * rcp_fast(dl * dr), bl + br);

@@ -113,3 +113,30 @@ def test_block_update_matches_the_strict_loop(X, Y):
     r0, r1 = s0.amr_update_aux(Ub, guess), s1.amr_update_aux(Ub, guess)
     assert float(((r1 - r0).abs() / r0.abs()).max()) <= 1e-12
     assert s1.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx,bc", [(4, "ring"), (26, "outlets"), (27, "outlets"), (54, "outlets"), (131, "walls"),
+                                   (1301, "ring"), (11544, "walls"), (11545, "outlets"), (25753, "outlets"),
+                                   (54169, "walls")])
+def test_line_run_is_the_separate_launches(nx, bc, prec):
+    """advance of a 1D line as one persistent launch, bitwise the same steps
+    as one launch per phase (the form that per-kernel timing takes): last
+    tiles of one and two cells beside an outlet, one block, the tile sizes'
+    limits, CFL and fixed steps, the launch repeated on its own workspace."""
+    from janc_b200 import mechanism as jm
+    from janc_b200.solver import Solver
+    b = dict(zip(KEYS[:2], BCS[bc]))
+    if bc == "outlets":
+        b["right_boundary"] = "pressure_outlet"
+    one, sep = [Solver(1, nx, dx=5e-5, boundary_config=b, mechanism=jm.load(), precision=prec) for _ in range(2)]
+    sep.set_kernel_timing(True)
+    U, aux = _state(one, (nx,))
+    theta = {"Pb": 101325.0} if bc == "outlets" else None
+    for how in ({"cfl": 0.05}, {"dt": 1e-9}, {"cfl": 0.02}):
+        a = one.advance(U, aux, 3, theta=theta, **how)
+        r = sep.advance(U, aux, 3, theta=theta, **how)
+        for x, y in zip(a, r):
+            assert torch.equal(x, y) and bool(torch.isfinite(x).all())
+    assert one.status() == sep.status() == 0

@@ -53,6 +53,7 @@ def generate(path=None):
     w(f"#define JB_GEN_NREAC {nreac}")
     w(f"#define JB_GEN_NR {nr}")
     w(f"#define JB_GEN_NS {ns}")
+    w(f"#define JB_GEN_ROWS {3 * nreac + int((is_tb != 0).sum())}  // staged values of the split form")
     w("// structure signature (compared with the loaded mechanism by jb_create)")
     w("static const signed char JB_GEN_VF[%d][%d] = {%s};" % (
         nreac, nr, ", ".join("{" + ", ".join(str(int(x)) for x in row) + "}" for row in vf)))
@@ -72,12 +73,22 @@ def generate(path=None):
     w("// F_i = M_i kf and B_i = M_i kb to shared memory (layout [i][3][stride])")
     w("// and accumulates w_k = sum_i dv_ik M_i q_i.  Xc: clipped concentrations;")
     w("// E, iE: exp(g_k) and 1 / exp(g_k); Tp = T / pref, pT = pref / T.")
+    w("// G < 0: every reaction; G = 0..3: the reactions i = G mod 4, which also")
+    w("// write M_i q_i of the third-body reactions to rows 57.. (w_k is not formed).")
+    w("// Products that enter a sum are written as fma or as rounded products, so that")
+    w("// both forms round alike.")
+    w("template <int G>")
     w("__device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double invT, double Tp, double pT,")
     w("    const double* X, const double* Xc, const double* E, const double* iE, double* sh, int stride,")
     w("    double* wk) {")
+    w("  if constexpr (G < 0) {")
     for k in range(nr):
-        w(f"  wk[{k}] = 0.0;")
+        w(f"    wk[{k}] = 0.0;")
+    w("  }")
+    tb_row = {}
     for i in range(nreac):
+        if is_tb[i]:
+            tb_row[i] = 3 * nreac + len(tb_row)
         reac = [(k, int(vf[i, k])) for k in range(nr) if vf[i, k] != 0]
         prod = [(k, int(vb[i, k])) for k in range(nr) if vb[i, k] != 0]
         dv = [(k, int(vb[i, k] - vf[i, k])) for k in range(nr) if vb[i, k] != vf[i, k]]
@@ -86,11 +97,14 @@ def generate(path=None):
             # prod arr[k]^c as repeated products (c a small positive integer)
             return [f"{arr}[{k}]" for k, c in terms for _ in range(c)]
 
-        w(f"  {{  // reaction {i}")
-        w(f"    const double k0 = exp(m.lnA[{i}] + m.B[{i}] * lT - m.EaR[{i}] * invT);")
+        w(f"  if constexpr (G < 0 || G == {i % 4}) {{  // reaction {i}")
+        w(f"    const double k0 = exp(fma(-m.EaR[{i}], invT, fma(m.B[{i}], lT, m.lnA[{i}])));")
         if is_tb[i]:
-            terms = [f"m.tb[{i}][{j}] * X[{j}]" for j in range(ns) if tb[i, j] != 0]
-            w(f"    const double Mi = {' + '.join(terms)};")
+            js = [j for j in range(ns) if tb[i, j] != 0]
+            expr = f"m.tb[{i}][{js[0]}] * X[{js[0]}]"
+            for j in js[1:]:
+                expr = f"fma(m.tb[{i}][{j}], X[{j}], {expr})"
+            w(f"    const double Mi = {expr};")
         else:
             w("    const double Mi = 1.0;")
         fac_f = powers(reac, "Xc")
@@ -99,24 +113,44 @@ def generate(path=None):
         vs = int(vsum[i])
         pw = ["Tp"] * vs if vs > 0 else ["pT"] * (-vs)
         fac_b = eg + pw + powers(prod, "Xc")
-        w(f"    const double kf = {' * '.join(['k0'] + fac_f)};")
-        w(f"    const double kb = {' * '.join(['k0'] + fac_b)};")
+        w(f"    const double kf = __dmul_rn({' * '.join(['k0'] + fac_f[:-1])}, {fac_f[-1]});")
+        w(f"    const double kb = __dmul_rn({' * '.join(['k0'] + fac_b[:-1])}, {fac_b[-1]});")
         w("    const double q = kf - kb;")
-        w("    const double Mq = Mi * q;")
+        w("    const double Mq = __dmul_rn(Mi, q);" if is_tb[i] else "    const double Mq = q;")
+        w("    if constexpr (G < 0) {")
         for k, c in dv:
-            if c == 1:
-                w(f"    wk[{k}] += Mq;")
-            elif c == -1:
-                w(f"    wk[{k}] -= Mq;")
-            else:
-                w(f"    wk[{k}] += {_num(c)} * Mq;")
+            w(f"      wk[{k}] {'+' if c > 0 else '-'}= Mq;" if abs(c) == 1 else
+              f"      wk[{k}] = fma({_num(c)}, Mq, wk[{k}]);")
+        if is_tb[i]:
+            w("    } else {")
+            w(f"      sh[{tb_row[i]} * stride] = Mq;")
+        w("    }")
         w(f"    sh[({3 * i} + 0) * stride] = q;")
         w(f"    sh[({3 * i} + 1) * stride] = Mi * kf;")
         w(f"    sh[({3 * i} + 2) * stride] = Mi * kb;")
         w("  }")
     w("}")
     w("")
-    w("// Phase B: the analytic Jacobian J[k][n] (without the M_k row factor).")
+    w("// w_k of the species 2 G and 2 G + 1 from the rows the groups wrote, in the")
+    w("// order of the full sum.")
+    w("template <int G>")
+    w("__device__ __forceinline__ void chem_w_gen(const double* sh, int stride, double* wk) {")
+    for k in range(nr):
+        w(f"  if constexpr (G == {k // 2}) {{")
+        w("    double s = 0.0;")
+        for i in range(nreac):
+            c = int(vb[i, k] - vf[i, k])
+            if c == 0:
+                continue
+            row = f"sh[{tb_row[i] if is_tb[i] else 3 * i} * stride]"
+            w(f"    s {'+' if c > 0 else '-'}= {row};" if abs(c) == 1 else f"    s = fma({_num(c)}, {row}, s);")
+        w(f"    wk[{k % 2}] = s;")
+        w("  }")
+    w("}")
+    w("")
+    w("// Phase B: the analytic Jacobian J[k][n] (without the M_k row factor); G = 0..3:")
+    w("// its columns 2 G and 2 G + 1 alone.")
+    w("template <int G>")
     w("__device__ __forceinline__ void chem_jac_gen(const MP& m, const double* rMX, const double* sh,")
     w("    int stride, double (&J)[8][8]) {")
     w("#pragma unroll")
@@ -144,17 +178,17 @@ def generate(path=None):
                 if b:
                     inner.append(("- B" if b == 1 else f"- {_num(b)} * B"))
                 expr = " ".join(inner) if a else inner[0].replace("- ", "-", 1)
-                parts.append(f"({expr}) * rMX[{n}]")
+                parts.append(f"__dmul_rn({expr}, rMX[{n}])")
             if not parts:
                 continue
-            w(f"    {{ const double c = {' + '.join(parts)};")
+            q = f"q, m.tbinvM[{i}][{n}]"
+            expr = f"fma({q}, {parts[1]})" if len(parts) == 2 else \
+                (f"__dmul_rn({q})" if tb[i, n] != 0 else parts[0])
+            w(f"    if constexpr (G < 0 || G == {n // 2}) {{")
+            w(f"      const double c = {expr};")
             for k, c in dv:
-                if c == 1:
-                    w(f"      J[{k}][{n}] += c;")
-                elif c == -1:
-                    w(f"      J[{k}][{n}] -= c;")
-                else:
-                    w(f"      J[{k}][{n}] += {_num(c)} * c;")
+                w(f"      J[{k}][{n}] {'+' if c > 0 else '-'}= c;" if abs(c) == 1 else
+                  f"      J[{k}][{n}] = fma({_num(c)}, c, J[{k}][{n}]);")
             w("    }")
         w("  }")
     w("}")

@@ -523,11 +523,19 @@ __device__ __forceinline__ unsigned finish_state(const MP& m, const Grid& g, con
 #endif
   {
     (void)amx; (void)amy; (void)dtm; (void)slots;
+    double Y8[NR], Yf[NS];
+#if JB_FAST
+    const double ri = 1.0 / rho;
+    const double u = q[1] * ri, v = DIM == 2 ? q[2] * ri : 0.0;
+    const double e = q[nY - 1] * ri - 0.5 * (u * u + v * v);
+#pragma unroll
+    for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] * ri;
+#else
     const double u = q[1] / rho, v = DIM == 2 ? q[2] / rho : 0.0;
     const double e = q[nY - 1] / rho - 0.5 * (u * u + v * v);
-    double Y8[NR], Yf[NS];
 #pragma unroll
     for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] / rho;
+#endif
     fill_Y(Y8, Yf);
     const double R = get_R(m, Yf);
     double cnd[JB_NCAND];
@@ -1900,7 +1908,11 @@ __device__ __forceinline__ void chem_solve(const MP& m, double (&J)[NR][NR], con
     double lo = -Y8[k], hi = 1.0 - Y8[k];
     dY = dY < lo ? lo : dY;
     dY = dY > hi ? hi : dY;
+#if JB_FAST
+    S[k] = __dmul_rn(rho, dY);  // rounded here in every form of the chemistry, not fused into U + S
+#else
     S[k] = rho * dY;
+#endif
   }
 }
 
@@ -1985,6 +1997,36 @@ __device__ void chem_cell(const MP& m, double rho, const double* Y8, double T, d
 #if JB_FAST
 constexpr int CHEM_SH = 3 * NREAC;  // per-cell shared doubles of the specialised path
 
+// Concentrations X of one cell, those clipped at 1e-50, and the powers of T
+// that the rates take.
+struct ChemIn {
+  double X[NS], Xc[NR], lT, invT, lT0T, Tp, pT;
+};
+__device__ __forceinline__ void chem_in(const MP& m, double rho, const double* Y8, double T, ChemIn& in) {
+  double Yf[NS];
+  fill_Y(Y8, Yf);
+#pragma unroll
+  for (int k = 0; k < NS; ++k) in.X[k] = rho * Yf[k] * m.invM[k];
+#pragma unroll
+  for (int k = 0; k < NR; ++k) in.Xc[k] = in.X[k] < 1e-50 ? 1e-50 : in.X[k];
+  in.lT = log(T);
+  in.invT = 1.0 / T;
+  in.lT0T = in.lT + m.lnT0;
+  in.Tp = T / m.pref;
+  in.pT = m.pref * in.invT;
+}
+// get_gibbs (reaction_model.py:78-89) of species k: g = s/R - h/(R T)
+template <bool LO>
+__device__ __forceinline__ double chem_gibbs(const MP& m, int k, double T, const ChemIn& in) {
+  const double h = LO ? poly6(m.hc_lo[k], T) : poly6(m.hc_hi[k], T);
+  const double s = LO ? fma(m.lg_lo[k], in.lT0T, poly5(m.s_lo[k], T)) : fma(m.lg_hi[k], in.lT0T, poly5(m.s_hi[k], T));
+  return fma(-h, in.invT, s);
+}
+__device__ __forceinline__ void chem_equil(double gk, double& E, double& iE) {
+  E = exp(gk);
+  iE = rcp_nr(fmin(fmax(E, 1e-300), 1e300));  // finite where E over- or underflows
+}
+
 // Specialised chemistry (structure compiled in by gen_chem.py): one
 // exponential per reaction and one per species, the concentration and
 // equilibrium factors as products (their exponents are small integers),
@@ -1993,47 +2035,156 @@ constexpr int CHEM_SH = 3 * NREAC;  // per-cell shared doubles of the specialise
 __device__ __forceinline__ void chem_cell_gen(const MP& m, double rho, const double* Y8, double T,
                                               double dt, double* S, unsigned& st, double* sh,
                                               int stride) {
-  double Yf[NS], X[NS], Xc[NR], E[NR], iE[NR], rMX[NR], w[NR];
-  fill_Y(Y8, Yf);
+  double E[NR], iE[NR], rMX[NR], w[NR], gk[NR];
+  ChemIn in;
+  chem_in(m, rho, Y8, T, in);
 #pragma unroll
-  for (int k = 0; k < NS; ++k) X[k] = rho * Yf[k] * m.invM[k];
-#pragma unroll
-  for (int k = 0; k < NR; ++k) {
-    const double xc = X[k] < 1e-50 ? 1e-50 : X[k];
-    Xc[k] = xc;
-    rMX[k] = m.invM[k] * rcp_nr(xc);
-  }
-  const double lT = log(T), invT = 1.0 / T, lT0T = lT + m.lnT0;
-  // get_gibbs (reaction_model.py:78-89): g = s/R - h/(R T); E = exp(g).  One
-  // branch where all species switch ranges at the same temperature, so that
-  // one range's coefficients are read straight from the parameter bank.
-  double gk[NR];
+  for (int k = 0; k < NR; ++k) rMX[k] = m.invM[k] * rcp_nr(in.Xc[k]);
+  // one branch where all species switch NASA7 ranges at the same temperature,
+  // so that one range's coefficients are read straight from the parameter bank
   if (m.tcr_uniform) {
     if (T < m.Tcr[0]) {
 #pragma unroll
-      for (int k = 0; k < NR; ++k) gk[k] = poly5(m.s_lo[k], T) + m.lg_lo[k] * lT0T - poly6(m.hc_lo[k], T) * invT;
+      for (int k = 0; k < NR; ++k) gk[k] = chem_gibbs<true>(m, k, T, in);
     } else {
 #pragma unroll
-      for (int k = 0; k < NR; ++k) gk[k] = poly5(m.s_hi[k], T) + m.lg_hi[k] * lT0T - poly6(m.hc_hi[k], T) * invT;
+      for (int k = 0; k < NR; ++k) gk[k] = chem_gibbs<false>(m, k, T, in);
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const bool lo = T < m.Tcr[k];
-      const double h = lo ? poly6(m.hc_lo[k], T) : poly6(m.hc_hi[k], T);
-      const double s = lo ? poly5(m.s_lo[k], T) + m.lg_lo[k] * lT0T : poly5(m.s_hi[k], T) + m.lg_hi[k] * lT0T;
-      gk[k] = s - h * invT;
-    }
+    for (int k = 0; k < NR; ++k)
+      gk[k] = T < m.Tcr[k] ? chem_gibbs<true>(m, k, T, in) : chem_gibbs<false>(m, k, T, in);
   }
 #pragma unroll
-  for (int k = 0; k < NR; ++k) {
-    E[k] = exp(gk[k]);
-    iE[k] = rcp_nr(fmin(fmax(E[k], 1e-300), 1e300));  // finite where E over- or underflows
-  }
-  chem_rates_gen(m, lT, invT, T / m.pref, m.pref * invT, X, Xc, E, iE, sh, stride, w);
+  for (int k = 0; k < NR; ++k) chem_equil(gk[k], E[k], iE[k]);
+  chem_rates_gen<-1>(m, in.lT, in.invT, in.Tp, in.pT, in.X, in.Xc, E, iE, sh, stride, w);
   double J[NR][NR];
-  chem_jac_gen(m, rMX, sh, stride, J);
+  chem_jac_gen<-1>(m, rMX, sh, stride, J);
   chem_solve(m, J, w, rho, Y8, dt, S, st);
+}
+
+// The same for the 32 cells of a block of four warps: warp w takes two
+// species' equilibrium factors, every fourth reaction, and two columns of the
+// Jacobian of its lane's cell, warp 0 the solve (S and st are warp 0's).  A
+// cell's chemistry is one long chain of latencies in a single thread (17 us at
+// any grid that leaves the chip idle); here four threads share it.  Sums run
+// in the order of chem_cell_gen, so the two agree bitwise.  sh: the block's
+// [CHEM_SPLIT_ROWS][32] shared doubles; every thread of the block calls it,
+// and a block barrier separates it from the next use of sh.
+constexpr int CHEM_SPLIT_ROWS = JB_GEN_ROWS + 2 * NR + NR + NR * NR;
+template <int G>
+__device__ __forceinline__ void chem_split_part(const MP& m, const ChemIn& in, double* col) {
+  double E[NR], iE[NR], none[NR];
+  const double* e = col + JB_GEN_ROWS * 32;
+#pragma unroll
+  for (int k = 0; k < NR; ++k) {
+    E[k] = e[k * 32];
+    iE[k] = e[(NR + k) * 32];
+  }
+  chem_rates_gen<G>(m, in.lT, in.invT, in.Tp, in.pT, in.X, in.Xc, E, iE, col, 32, none);
+  __syncthreads();
+  double rMX[NR], J[NR][NR], w2[2];
+#pragma unroll
+  for (int k = 0; k < NR; ++k)
+    if (k / 2 == G) rMX[k] = m.invM[k] * rcp_nr(in.Xc[k]);
+  chem_jac_gen<G>(m, rMX, col, 32, J);
+  chem_w_gen<G>(col, 32, w2);
+  double* w = col + (JB_GEN_ROWS + 2 * NR) * 32;
+  double* j = w + NR * 32;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    w[(2 * G + i) * 32] = w2[i];
+#pragma unroll
+    for (int k = 0; k < NR; ++k) j[(k * NR + 2 * G + i) * 32] = J[k][2 * G + i];
+  }
+}
+__device__ __forceinline__ void chem_split(const MP& m, double rho, const double* Y8, double T, double dt, double* S,
+                                           unsigned& st, double* sh) {
+  double* col = sh + (threadIdx.x & 31);
+  const int wp = threadIdx.x >> 5;
+  ChemIn in;
+  chem_in(m, rho, Y8, T, in);
+  double* e = col + JB_GEN_ROWS * 32;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int k = 2 * wp + i;
+    double E, iE;
+    chem_equil(T < m.Tcr[k] ? chem_gibbs<true>(m, k, T, in) : chem_gibbs<false>(m, k, T, in), E, iE);
+    e[k * 32] = E;
+    e[(NR + k) * 32] = iE;
+  }
+  __syncthreads();
+  switch (wp) {  // each case holds one more block barrier
+    case 0: chem_split_part<0>(m, in, col); break;
+    case 1: chem_split_part<1>(m, in, col); break;
+    case 2: chem_split_part<2>(m, in, col); break;
+    default: chem_split_part<3>(m, in, col); break;
+  }
+  __syncthreads();
+  if (wp == 0) {
+    const double* w = col + (JB_GEN_ROWS + 2 * NR) * 32;
+    const double* j = w + NR * 32;
+    double J[NR][NR], wk[NR];
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      wk[k] = w[k * 32];
+#pragma unroll
+      for (int n = 0; n < NR; ++n) J[k][n] = j[(k * NR + n) * 32];
+    }
+    chem_solve(m, J, wk, rho, Y8, dt, S, st);
+  }
+}
+#endif
+
+// The end of a cell's chemistry: S itself (WRITE_S), or U + S and the
+// temperature solve; q holds the cell's fields.
+template <int DIM, bool WRITE_S, bool CELL>
+__device__ __forceinline__ void chem_store(const MP& m, const Grid& g, double* q, const double* S, double T,
+                                           double* out, const jb_fin& fin, long long c, unsigned& bits, double& amx,
+                                           double& amy, double& dtm, Slots* slots) {
+  constexpr int nY = DIM == 1 ? 3 : 4;
+  constexpr int nv = nY + NR;
+  const long long nc = g.ncell;
+  if (WRITE_S) {
+#pragma unroll
+    for (int f = 0; f < nY; ++f) out[f * nc + c] = 0.0;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) out[(nY + k) * nc + c] = S[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < NR; ++k) q[nY + k] = q[nY + k] + S[k];
+#pragma unroll
+    for (int f = 0; f < nv; ++f) out[f * nc + c] = q[f];
+    bits |= finish_state<DIM, CELL>(m, g, fin, q, T, c, amx, amy, dtm, slots);
+  }
+}
+
+#if JB_FAST
+// chem_cell_step of the block's 32 cells c (one per lane, the same in every
+// warp; cells past the end repeat one inside and have live = false).
+template <int DIM, bool WRITE_S, bool CELL>
+__device__ __forceinline__ void chem_split_step(const MP& m, const Grid& g, const double* U, double T, double* out,
+                                                const jb_fin& fin, long long c, bool live, double dt, double* sh,
+                                                unsigned& bits, unsigned& st, double& amx, double& amy, double& dtm,
+                                                Slots* slots) {
+  constexpr int nY = DIM == 1 ? 3 : 4;
+  constexpr int nv = nY + NR;
+  const long long nc = g.ncell;
+  double q[nv], Y8[NR], S[NR];
+  q[0] = U[c];
+#pragma unroll
+  for (int k = 0; k < NR; ++k) q[nY + k] = U[(nY + k) * nc + c];
+  const double ri = 1.0 / q[0];
+#pragma unroll
+  for (int k = 0; k < NR; ++k) Y8[k] = __dmul_rn(q[nY + k], ri);
+  unsigned s1 = 0;
+  chem_split(m, q[0], Y8, T, dt, S, s1, sh);
+  if (threadIdx.x < 32 && live) {
+    st |= s1;
+#pragma unroll
+    for (int f = 1; f < nY; ++f) q[f] = U[f * nc + c];
+    chem_store<DIM, WRITE_S, CELL>(m, g, q, S, T, out, fin, c, bits, amx, amy, dtm, slots);
+  }
 }
 #endif
 
@@ -2068,7 +2219,7 @@ __device__ __forceinline__ void chem_cell_step(const MP& m, const Grid& g, const
 #if JB_FAST
     const double ri = 1.0 / rho;
 #pragma unroll
-    for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] * ri;
+    for (int k = 0; k < NR; ++k) Y8[k] = __dmul_rn(q[nY + k], ri);
 #else
 #pragma unroll
     for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] / rho;
@@ -2082,18 +2233,7 @@ __device__ __forceinline__ void chem_cell_step(const MP& m, const Grid& g, const
     (void)sh;
     chem_cell(m, rho, Y8, T, dt, S, st);
 #endif
-    if (WRITE_S) {
-#pragma unroll
-      for (int f = 0; f < nY; ++f) out[f * nc + c] = 0.0;
-#pragma unroll
-      for (int k = 0; k < NR; ++k) out[(nY + k) * nc + c] = S[k];
-    } else {
-#pragma unroll
-      for (int k = 0; k < NR; ++k) q[nY + k] = q[nY + k] + S[k];
-#pragma unroll
-      for (int f = 0; f < nv; ++f) out[f * nc + c] = q[f];
-      bits |= finish_state<DIM, CELL>(m, g, fin, q, T, c, amx, amy, dtm, slots);
-    }
+    chem_store<DIM, WRITE_S, CELL>(m, g, q, S, T, out, fin, c, bits, amx, amy, dtm, slots);
   }
 }
 
@@ -2127,6 +2267,28 @@ __global__ void __launch_bounds__(JB_CHEM_NT, JB_CHEM_MINB) k_chem(MP m, Grid g,
   else
     finish_reduce(fin, amx, amy, dtm, bits | (st << 16), slots);
 }
+
+#if JB_FAST
+// k_chem with four threads a cell (chem_split), 32 cells a block.
+template <int DIM, bool WRITE_S, bool CELL>
+__global__ void __launch_bounds__(128, 3) k_chem_split(MP m, Grid g, const double* __restrict__ U,
+                                                     const double* __restrict__ aux, double* __restrict__ out,
+                                                     jb_fin fin, Slots* slots, double dt_arg) {
+  __shared__ double sh[CHEM_SPLIT_ROWS * 32];
+  const long long c0 = (long long)blockIdx.x * 32 + (threadIdx.x & 31);
+  const bool live = c0 < g.ncell;
+  const long long c = live ? c0 : g.ncell - 1;
+  const double dt = WRITE_S ? dt_arg : slots->dt;
+  unsigned bits = 0, st = 0;
+  double amx = 0.0, amy = 0.0, dtm = __longlong_as_double(0x7ff0000000000000LL);
+  const double T = aux ? aux[g.ncell + c] : fin.cand[(long long)halley_count(slots->mask[fin.midx - 1]) * g.ncell + c];
+  // the split's warps read T and U before warp 0 rewrites the iterates: its
+  // barriers lie between
+  chem_split_step<DIM, WRITE_S, CELL>(m, g, U, T, out, fin, c, live, dt, sh, bits, st, amx, amy, dtm, slots);
+  if (WRITE_S) block_reduce_store(0.0, 0.0, 0.0, st << 16, slots, 0, false, false, -1);
+  else finish_reduce(fin, amx, amy, dtm, bits | (st << 16), slots);
+}
+#endif
 
 // ---------------------------------------------------------------------------
 // U_to_prim (solver_{1D,2D}/aux_func.py:39-51): rho, u, [v,] Y, p, a

@@ -105,6 +105,10 @@ __global__ void __launch_bounds__(LR_NT, 3)
   const int tid = threadIdx.x, x0 = blockIdx.x * S, nin = min(S, g.nx - x0);
   const bool live = tid < nin;
   const long long c = x0 + tid, nc = g.ncell;
+  // S == 32: the cell of the thread's lane, for the split chemistry
+  const bool live32 = (tid & 31) < nin;
+  const long long cl = x0 + min(tid & 31, nin - 1);
+  (void)live32, (void)cl;
   const bool use_cfl = a.cfl > 0.0;
   const double inf = __longlong_as_double(0x7ff0000000000000LL);
   double* sh = reinterpret_cast<double*>(smraw) + tid;
@@ -153,9 +157,14 @@ __global__ void __launch_bounds__(LR_NT, 3)
       bits = line_tile<3, V, LR_NT, S>(m, g, a.W1, a.A1, U, a.W0, jb_fin_cell(a.A0, nullptr, -1, 0), a.strips + 2,
                                        bitsd(__ldcg(&cur->ax[2])), dt, x0, smraw, amx, dtm, cur);
       const jb_fin f4 = jb_fin_cell(a.aux_out, nullptr, 3, use_cfl);
-      if (live)
+      if constexpr (S == 32) {
+        // the other warps read what warp 0 wrote in stage 3 (line_tile ends in a block barrier)
+        chem_split_step<1, false, true>(m, g, a.W0, a.A0[nc + cl], a.U_out, f4, cl, live32, dt,
+                                        reinterpret_cast<double*>(smraw), bits, st, amx, amy, dtm, cur);
+      } else if (live) {
         chem_cell_step<1, false, true, true>(m, g, a.W0, a.A0[nc + c], a.U_out, f4, c, dt, sh, bits, st, amx, amy,
                                              dtm, cur);
+      }
       lr_strips(m, g, x0, nin, a.U_out, a.aux_out, a.strips, amx);
       finish_reduce(f4, amx, 0.0, dtm, bits | (st << 16), cur);
       go = lr_sync(a.bar, target);
@@ -191,10 +200,14 @@ __global__ void __launch_bounds__(LR_NT, 3)
       if (!(go = lr_sync(a.bar, target))) break;
       // chemistry at the selected stage-3 iterate
       bits = st = 0;
-      if (live)
-        chem_cell_step<1, false, true, false>(m, g, a.W0, a.cand[halley_count(__ldcg(&cur->mask[2])) * nc + c],
-                                              a.U_out, jb_fin_cand(a.cand, 3), c, dt, sh, bits, st, amx, amy, dtm,
-                                              nullptr);
+      const long long n3 = halley_count(__ldcg(&cur->mask[2])) * nc;
+      if constexpr (S == 32) {
+        chem_split_step<1, false, false>(m, g, a.W0, a.cand[n3 + cl], a.U_out, jb_fin_cand(a.cand, 3), cl, live32, dt,
+                                         reinterpret_cast<double*>(smraw), bits, st, amx, amy, dtm, nullptr);
+      } else if (live) {
+        chem_cell_step<1, false, true, false>(m, g, a.W0, a.cand[n3 + c], a.U_out, jb_fin_cand(a.cand, 3), c, dt, sh,
+                                              bits, st, amx, amy, dtm, nullptr);
+      }
       finish_reduce(jb_fin_cand(a.cand, 3), 0.0, 0.0, inf, bits | (st << 16), cur);
       if (!(go = lr_sync(a.bar, target))) break;
       amx = 0.0;
@@ -240,7 +253,7 @@ int lr_resident(size_t sm) {
 
 template <class V, int S>
 bool lr_try(const MP& m, const Grid& g, const LineRun& a, cudaStream_t st, cudaError_t& err) {
-  constexpr size_t chem = sizeof(double) * CHEM_SH * LR_NT, line = line_smem<V, S>(), sm = chem > line ? chem : line;
+  constexpr size_t chem = sizeof(double) * (S == 32 ? CHEM_SPLIT_ROWS * 32 : CHEM_SH * LR_NT), line = line_smem<V, S>(), sm = chem > line ? chem : line;
   const int nb = (g.nx + S - 1) / S;
   if (nb > lr_resident<V, S>(sm)) return false;
   void* args[] = {(void*)&m, (void*)&g, (void*)&a};
@@ -250,9 +263,9 @@ bool lr_try(const MP& m, const Grid& g, const LineRun& a, cudaStream_t st, cudaE
 
 }  // namespace
 
-// The run as one launch where one tile per resident CTA covers the line (26
-// cells a tile while that suffices: the fewest cells per thread; then 58, then
-// 122); false, and nothing launched, where it does not or the stream is being
+// The run as one launch where one tile per resident CTA covers the line (32
+// cells a tile while that suffices, one per lane with the chemistry split over
+// the four warps; then 58, then 122); false, and nothing launched, where it does not or the stream is being
 // captured (the separate launches are plain graph nodes).
 template <class V>
 static bool line_run_t(const MP& m, const Grid& g, const jb_line_io& io, cudaStream_t st, cudaError_t& err) {
@@ -263,7 +276,7 @@ static bool line_run_t(const MP& m, const Grid& g, const jb_line_io& io, cudaStr
   a.W0 = io.W0; a.W1 = io.W1; a.A0 = io.A0; a.A1 = io.A1; a.cand = io.cand; a.strips = io.strips;
   a.slots = io.slots; a.sets = io.slots + 1; a.bar = io.bar;
   a.dt_fixed = io.dt_fixed; a.cfl = io.cfl; a.nsteps = io.nsteps; a.dt_hist = io.dt_hist;
-  return lr_try<V, 26>(m, g, a, st, err) || lr_try<V, 58>(m, g, a, st, err) || lr_try<V, 122>(m, g, a, st, err);
+  return lr_try<V, 32>(m, g, a, st, err) || lr_try<V, 58>(m, g, a, st, err) || lr_try<V, 122>(m, g, a, st, err);
 }
 bool line_run(bool mixed, const MP& m, const Grid& g, const jb_line_io& io, cudaStream_t st, cudaError_t& err) {
   return mixed ? line_run_t<float>(m, g, io, st, err) : line_run_t<double>(m, g, io, st, err);

@@ -131,7 +131,9 @@ class _ProbeTrajectory(torch.autograd.Function):
         U0, aux0 = traj.s.state_from_PTY(P, Tc, Y)
         _, _, dts, pps, ckpts = traj.run(U0, aux0, nsteps)
         ctx.traj, ctx.nsteps, ctx.ckpts = traj, nsteps, ckpts
-        ctx.lnA = None if lnA is None else lnA.detach().clone()
+        # the offsets as the host holds them: the backward pass sets them
+        # again without waiting for the device
+        ctx.lnA = traj._lnA
         ctx.save_for_backward(Tc, P, Y)
         return dts, pps
 

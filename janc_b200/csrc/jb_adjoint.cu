@@ -36,6 +36,8 @@
 //   k_init_vjp      initial state from (P, T, Y): T adjoint
 #define JB_NS adj
 #define JB_FAST 1
+#include <atomic>
+
 #include "jb_kernels.cuh"
 
 #include "jb_adjoint.h"
@@ -505,10 +507,10 @@ __device__ __forceinline__ double weno_d(double v0, double v1, double v2, double
   const double b3 = 0.25 * d3 * d3 + 13.0 / 12.0 * e3 * e3;
   const double s1 = 1e-6 + b1, s2 = 1e-6 + b2, s3 = 1e-6 + b3;
   // one division for the three reciprocals (s_k lies in [1e-6, ~1e20])
-  const double s12 = s1 * s2, r = 1.0 / (s12 * s3);
+  const double s12 = s1 * s2, r = rcp_nr(s12 * s3);
   const double i1 = s2 * s3 * r, i2 = s1 * s3 * r, i3 = s12 * r;
   const double a1 = 0.1 * i1 * i1, a2 = 0.6 * i2 * i2, a3 = 0.3 * i3 * i3;
-  const double iS = 1.0 / (a1 + a2 + a3);
+  const double iS = rcp_nr(a1 + a2 + a3);
   const double w1 = a1 * iS, w2 = a2 * iS, w3 = a3 * iS;
   const double q1 = 1.0 / 3.0 * v0 - 7.0 / 6.0 * v1 + 11.0 / 6.0 * v2;
   const double q2 = -1.0 / 6.0 * v1 + 5.0 / 6.0 * v2 + 1.0 / 3.0 * v3;
@@ -932,7 +934,7 @@ __global__ void __launch_bounds__(128) k_outlet_ghosts(MP m, Grid g, const doubl
 // ---------------------------------------------------------------------------
 // flux VJP of one RK stage: line sweeps, then a per-cell merge
 // ---------------------------------------------------------------------------
-// The sweep thread of (direction D, line, segment, field f) owns SW_R
+// The sweep thread of (direction D, line, segment, field f) owns sw_r
 // consecutive padded cells of the line (ghosts included) and walks the
 // faces that touch them, keeping a six-cell window of H+, H- and the field
 // in registers: per face the two WENO5 reconstructions and their partials,
@@ -942,8 +944,7 @@ __global__ void __launch_bounds__(128) k_outlet_ghosts(MP m, Grid g, const doubl
 // Only faces 0..n carry a flux into the interior, so faces outside are
 // skipped.  No shared memory and no barriers: one thread's faces are
 // independent of the other threads'.
-constexpr int SW_R = 24;
-constexpr int SW_NT = 128;
+constexpr int SW_NT = 128, SW_MINB = 4;
 
 // H+ and H- of field f at padded cell a of a line, from the stage state and
 // its primitives (those of the source cell; ghosts flip the momentum), or
@@ -991,12 +992,12 @@ __device__ __forceinline__ void sweep_body(const Grid& g, const double* __restri
                                            const double* __restrict__ Pk, const double* __restrict__ og,
                                            const double* __restrict__ Uo_b,
                                            double coef, double alpha, double dt, int f, int line, int seg,
-                                           double* __restrict__ Fb, double* __restrict__ Ua, double& ab,
+                                           int sw_r, double* __restrict__ Fb, double* __restrict__ Ua, double& ab,
                                            double& dtb) {
   const int nA = D == 0 ? g.nx : g.ny;
   const long long nc = g.ncell;
   const double idA = 1.0 / (D == 0 ? g.dx : g.dy), dt_dA = dt * idA;
-  const int a0 = -3 + seg * SW_R, a1 = min(a0 + SW_R, nA + 3);  // owned padded cells [a0, a1)
+  const int a0 = -3 + seg * sw_r, a1 = min(a0 + sw_r, nA + 3);  // owned padded cells [a0, a1)
   const int flo = max(a0 - 2, 0), fhi = min(a1 + 2, nA);        // faces touching them
   const size_t npad = D == 0 ? (size_t)(g.nx + 6) * g.ny : (size_t)g.nx * (g.ny + 6);
   const double* ob = Uo_b + f * nc;
@@ -1071,13 +1072,13 @@ __device__ __forceinline__ void sweep_body(const Grid& g, const double* __restri
 // consecutive y per block), the rest y lines (SW_NT consecutive x); the
 // field runs fastest over blocks, then the line block, then the segment.
 template <int DIM>
-__global__ void __launch_bounds__(SW_NT, 4) k_flux_sweep(Grid g, const double* __restrict__ Uk,
+__global__ void __launch_bounds__(SW_NT, SW_MINB) k_flux_sweep(Grid g, const double* __restrict__ Uk,
                                                       const double* __restrict__ Pk,
                                                       const double* __restrict__ og,
                                                       const double* __restrict__ Uo_b, double coef,
                                                       const double* __restrict__ slots_rec, int stage, double* FbX,
                                                       double* UaX, double* FbY, double* UaY, double* red, int nbx,
-                                                      int nlx, int nly) {
+                                                      int nlx, int nly, int sw_r) {
   const jb_slots* rs = reinterpret_cast<const jb_slots*>(slots_rec);
   int b = blockIdx.x;
   const int D = b < nbx ? 0 : 1;
@@ -1091,11 +1092,11 @@ __global__ void __launch_bounds__(SW_NT, 4) k_flux_sweep(Grid g, const double* _
   const int seg = DIM == 1 ? b * SW_NT + threadIdx.x : b / nl;
   double ab = 0.0, dtb = 0.0;
   if (D == 0) {
-    if (line < g.ny && seg * SW_R < g.nx + 6)
-      sweep_body<0, DIM>(g, Uk, Pk, og, Uo_b, coef, bitsd(rs->ax[stage]), rs->dt, f, line, seg, FbX, UaX, ab, dtb);
+    if (line < g.ny && seg * sw_r < g.nx + 6)
+      sweep_body<0, DIM>(g, Uk, Pk, og, Uo_b, coef, bitsd(rs->ax[stage]), rs->dt, f, line, seg, sw_r, FbX, UaX, ab, dtb);
   } else if (DIM == 2) {
     if (line < g.nx)
-      sweep_body<1, DIM>(g, Uk, Pk, og, Uo_b, coef, bitsd(rs->ay[stage]), rs->dt, f, line, seg, FbY, UaY, ab, dtb);
+      sweep_body<1, DIM>(g, Uk, Pk, og, Uo_b, coef, bitsd(rs->ay[stage]), rs->dt, f, line, seg, sw_r, FbY, UaY, ab, dtb);
   }
   block_add(ab, red + red_ab(stage, D));
   block_add(dtb, red + RED_DTB);
@@ -1479,15 +1480,38 @@ static cudaError_t flux_stage_t(const jb_mech_params& m, const jb_grid& g, const
   constexpr int NVD = Lay<DIM>::NV;
   const size_t npx = NVD * (size_t)(g.nx + 6) * g.ny, npy = DIM == 2 ? NVD * (size_t)g.nx * (g.ny + 6) : 0;
   double *FbX = scratch, *UaX = FbX + npx, *FbY = UaX + npx, *UaY = FbY + npy;
-  const int nlx = (g.ny + SW_NT - 1) / SW_NT, nsx = (g.nx + 6 + SW_R - 1) / SW_R;
-  const int nly = (g.nx + SW_NT - 1) / SW_NT, nsy = (g.ny + 6 + SW_R - 1) / SW_R;
-  const int nbx = (DIM == 2 ? nlx * nsx : (nsx + SW_NT - 1) / SW_NT) * NVD, nby = DIM == 2 ? nly * nsy * NVD : 0;
+  // Segment length: a thread walks sw_r cells and about seven more faces; the
+  // length of 6 .. 48 that takes the fewest waves x (length + 7) over the
+  // resident blocks.  200 x 96 cells: 9 (one wave), where a fixed 24 left most
+  // of the chip idle (45 us a launch); large grids stay near 24.
+  static std::atomic<int> sm_count{0};
+  int nsm = sm_count.load(std::memory_order_relaxed);
+  if (!nsm) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    sm_count.store(nsm, std::memory_order_relaxed);
+  }
+  const int nlx = (g.ny + SW_NT - 1) / SW_NT, nly = (g.nx + SW_NT - 1) / SW_NT;
+  int sw_r = 24, nbx = 0, nby = 0;
+  long long best = -1;
+  for (int r = 6; r <= 48; ++r) {
+    const int nsx = (g.nx + 6 + r - 1) / r, nsy = (g.ny + 6 + r - 1) / r;
+    const int bx = (DIM == 2 ? nlx * nsx : (nsx + SW_NT - 1) / SW_NT) * NVD, by = DIM == 2 ? nly * nsy * NVD : 0;
+    const long long cost = ((long long)(bx + by) + SW_MINB * nsm - 1) / (SW_MINB * nsm) * (r + 7);
+    if (best < 0 || cost < best) {
+      best = cost;
+      sw_r = r;
+      nbx = bx;
+      nby = by;
+    }
+  }
   const bool outlet = has_outlet(DIM, g);
   double* og = og_of(DIM, g, scratch);
   double* ogb = og + (size_t)3 * 4 * OG_F * g.lstrip;
   k_flux_sweep<DIM><<<nbx + nby, SW_NT, 0, st>>>(g, Uk, Pk,
                                                  outlet ? og + (size_t)stage * 4 * OG_F * g.lstrip : nullptr, Uo_b,
-                                                 coef, slots_rec, stage, FbX, UaX, FbY, UaY, red, nbx, nlx, nly);
+                                                 coef, slots_rec, stage, FbX, UaX, FbY, UaY, red, nbx, nlx, nly, sw_r);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (outlet) {

@@ -69,12 +69,20 @@ __global__ void __launch_bounds__(256) k_visc_nodes(MP m, Grid g, const double* 
   }
   const double rho = q[0];
   double Y8[NR], Yf[NS];
+#if JB_FAST
+  const double ri = 1.0 / rho;
+#pragma unroll
+  for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] * ri;
+  nodes[np + i] = q[1] * ri;
+  if (DIM == 2) nodes[2 * np + i] = q[2] * ri;
+#else
 #pragma unroll
   for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] / rho;
-  fill_Y(Y8, Yf);
-  nodes[i] = rho;
   nodes[np + i] = q[1] / rho;
   if (DIM == 2) nodes[2 * np + i] = q[2] / rho;
+#endif
+  fill_Y(Y8, Yf);
+  nodes[i] = rho;
   nodes[(DIM + 1) * np + i] = T;
 #pragma unroll
   for (int k = 0; k < NS; ++k) nodes[(DIM + 2 + k) * np + i] = Yf[k];
@@ -181,6 +189,123 @@ __device__ __forceinline__ void node_transport(const MP& m, const jb_transport& 
     }
   }
 }
+
+#if JB_FAST
+// Sixth-order difference at an inner position c (stride st), the neighbours'
+// differences scaled by id60 = 1 / (60 d): six operations.
+__device__ __forceinline__ double d6(const double* c, int st, double id60) {
+  const double a = __ldg(c + st) - __ldg(c - st), b = __ldg(c + 2 * st) - __ldg(c - 2 * st);
+  return fma(45.0, a, fma(-9.0, b, __ldg(c + 3 * st) - __ldg(c - 3 * st))) * id60;
+}
+
+// One direction's node flux at a 2D node (XD: F_hat, else G_hat): each
+// species' derivative, cp and enthalpy are taken, used and stored before the
+// next, so that a thread holds a few sums instead of 9 diffusivities and
+// enthalpies.  IN: every stencil lies inside the padded array (all but its
+// outer three rows and columns).  The loop over the species stays a loop: with
+// every species and range unrolled the kernel waited for its instructions
+// (45 us at 512 x 256).  The node planes are read through the read-only path,
+// which may pass the stores.
+#ifndef JB_VF_UNROLL
+#define JB_VF_UNROLL 1
+#endif
+constexpr int VF_UNROLL = JB_VF_UNROLL;
+template <bool XD, bool IN>
+__device__ __forceinline__ void visc_node2d(const MP& m, const Grid& g, const jb_transport& tr,
+                                            const double* __restrict__ N, int px, int py, double T,
+                                            double* __restrict__ o, long long os) {
+  const int PX = g.nx + 6, PY = g.ny + 6;
+  const long long np = (long long)PX * PY;
+  const double* n0 = N + ((long long)px * PY + py);
+  const double idx60 = g.idx * (1.0 / 60.0), idy60 = g.idy * (1.0 / 60.0);
+  auto ddx = [&](int plane) {
+    return IN ? d6(n0 + plane * np, PY, idx60) : d_line(N + plane * np + py, PY, PX, px, g.dx);
+  };
+  auto ddy = [&](int plane) {
+    return IN ? d6(n0 + plane * np, 1, idy60) : d_line(N + plane * np + (long long)px * PY, 1, PY, py, g.dy);
+  };
+  auto ddn = [&](int plane) { return XD ? ddx(plane) : ddy(plane); };
+  const double rho = __ldg(n0), u = __ldg(n0 + np), v = __ldg(n0 + 2 * np);
+  const double du_dx = ddx(1), du_dy = ddy(1), dv_dx = ddx(2), dv_dy = ddy(2), dTn = ddn(3);
+  const double mu_t = tr.turbulence_model ? vreman_mu_t(rho, g.dx, g.dy, du_dx, du_dy, dv_dx, dv_dy) : 0.0;
+  double mu;
+  if (tr.viscosity_model == 0) {
+    const double x = T * rcp_nr(tr.T_ref);
+    mu = tr.mu_ref * (x * sqrt(x)) * (tr.T_ref + tr.S) * rcp_nr(T + tr.S);
+  } else {
+    mu = rho * tr.nu0;
+  }
+  if (tr.turbulence_model) mu = mu + mu_t;
+  // Prandtl and Lewis numbers without a turbulence model: rho D_k = mu / (Pr
+  // Le) for every species (cp_k cancels)
+  const bool simple = tr.conductivity_model == 0 && tr.diffusivity_model == 0 && !tr.turbulence_model;
+  const double iPr = rcp_nr(tr.Pr), rD0 = mu * iPr * rcp_nr(tr.Le);
+  double e = 0.0, cp = 0.0;
+  auto species = [&](int k, double cpk, double hk) {
+    const double dY = ddn(4 + k), Y = __ldg(n0 + (4 + k) * np);
+    cp = fma(cpk, Y, cp);
+    double rD = rD0;
+    if (!simple) {  // transport_model.py:133-157
+      if (tr.diffusivity_model == 0) {
+        const double k_i = tr.conductivity_model == 0 ? mu * cpk / tr.Pr : tr.k0;
+        rD = k_i / (tr.Le * cpk) + mu_t / tr.Pr_t / (tr.Le_t * cpk);
+      } else {
+        rD = rho * tr.D0 + mu_t / tr.Pr_t / tr.Le_t * cpk;
+      }
+    }
+    const double j = rD * dY;
+    e = fma(j, hk, e);
+    if (k < NR) o[(4 + k) * os] = j;
+  };
+  if (T < m.Tcr[0]) {
+#pragma unroll VF_UNROLL
+    for (int k = 0; k < NS; ++k) species(k, poly5(m.cp_lo[k], T), poly6(m.h_lo[k], T));
+  } else {
+#pragma unroll VF_UNROLL
+    for (int k = 0; k < NS; ++k) species(k, poly5(m.cp_hi[k], T), poly6(m.h_hi[k], T));
+  }
+  double kap = tr.conductivity_model == 0 ? mu * cp * iPr : tr.k0;
+  if (tr.turbulence_model) kap = kap + mu_t * cp / tr.Pr_t;
+  const double tau_nn = 2.0 * mu * (XD ? du_dx : dv_dy) - 2.0 / 3.0 * mu * (du_dx + dv_dy);
+  const double tau_xy = mu * (du_dy + dv_dx);
+  o[os] = XD ? tau_nn : tau_xy;
+  o[2 * os] = XD ? tau_xy : tau_nn;
+  o[3 * os] = (XD ? u * tau_nn + v * tau_xy : u * tau_xy + v * tau_nn) + kap * dTn + e;
+}
+
+template <bool XD>
+__device__ __forceinline__ void visc_node2d_any(const MP& m, const Grid& g, const jb_transport& tr,
+                                                const double* __restrict__ N, long long t, double* __restrict__ fh,
+                                                double* __restrict__ gh) {
+  const int PX = g.nx + 6, PY = g.ny + 6;
+  const long long sF = (long long)PX * g.ny, sG = (long long)g.nx * PY;
+  if (t >= (XD ? sF : sG)) return;
+  const int px = XD ? (int)(t / g.ny) : (int)(t / PY) + 3, py = XD ? (int)(t % g.ny) + 3 : (int)(t % PY);
+  const double T = __ldg(N + 3 * (long long)PX * PY + (long long)px * PY + py);
+  const bool in = px >= 3 && px < PX - 3 && py >= 3 && py < PY - 3;
+  double* o = (XD ? fh : gh) + t;
+  const long long os = XD ? sF : sG;
+  if (in) visc_node2d<XD, true>(m, g, tr, N, px, py, T, o, os);
+  else visc_node2d<XD, false>(m, g, tr, N, px, py, T, o, os);
+}
+
+// All node fluxes where every species switches NASA7 ranges at the same
+// temperature: blockIdx.y 0 takes the F_hat region, 1 the G_hat region, one
+// thread per node and direction (one thread for both left the chip at 28
+// warps an SM, waiting for its ~160 loads: 35 us at 512 x 256).  The density
+// carries no viscous flux: its planes stay unwritten and k_visc_div does not
+// read them.
+#ifndef JB_VF_MINB
+#define JB_VF_MINB 5
+#endif
+__global__ void __launch_bounds__(128, JB_VF_MINB) k_visc_flux2d(MP m, Grid g, jb_transport tr,
+                                                               const double* __restrict__ nodes,
+                                                               double* __restrict__ fh, double* __restrict__ gh) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.y == 0) visc_node2d_any<true>(m, g, tr, nodes, t, fh, gh);
+  else visc_node2d_any<false>(m, g, tr, nodes, t, fh, gh);
+}
+#endif
 
 // Node fluxes, one thread per node.  2D threads [0, nF) take the nodes of
 // the F_hat region (padded px in [0, nx+6), py in [3, ny+3) ->
@@ -308,6 +433,15 @@ __device__ __forceinline__ double central6(const double* f, long long st) {
          256.0;
 }
 
+// Difference of the interface values behind and before position 3 of seven
+// node fluxes (stride st): the two sixth-order sums share their centre, which
+// cancels.
+__device__ __forceinline__ double central6_diff(const double* f, long long st) {
+  return fma(175.0, f[4 * st] - f[2 * st], fma(-28.0, f[5 * st] - f[st], 3.0 * (f[6 * st] - f[0])));
+}
+
+// One thread per cell and field (blockIdx.y) in the fast variants, per cell in
+// the strict one.
 template <int DIM>
 __global__ void __launch_bounds__(128) k_visc_div(Grid g, const double* __restrict__ fh,
                                                   const double* __restrict__ gh, double* __restrict__ V) {
@@ -318,26 +452,30 @@ __global__ void __launch_bounds__(128) k_visc_div(Grid g, const double* __restri
   const int x = DIM == 2 ? (int)(c / g.ny) : (int)c, y = DIM == 2 ? (int)(c % g.ny) : 0;
   const int PX = g.nx + 6, PY = g.ny + 6;
   const long long sF = DIM == 2 ? (long long)PX * g.ny : PX, sG = (long long)g.nx * PY;
-#pragma unroll
-  for (int f = 0; f < nv; ++f) {
+#if JB_FAST
+  const int f = blockIdx.y;
+  double r = 0.0;  // the density has none
+  if (f > 0) {
     // faces x and x+1 of this cell: node fluxes at padded x .. x+6
     const double* a = fh + f * sF + (DIM == 2 ? (long long)x * g.ny + y : x);
-    const long long st = DIM == 2 ? g.ny : 1;
-#if JB_FAST
-    double r = (central6(a + st, st) - central6(a, st)) * g.idx;
-    if (DIM == 2) {
-      const double* b = gh + f * sG + (long long)x * PY + y;
-      r = r + (central6(b + 1, 1) - central6(b, 1)) * g.idy;
-    }
+    r = central6_diff(a, DIM == 2 ? g.ny : 1) * (g.idx * (1.0 / 256.0));
+    if (DIM == 2) r = r + central6_diff(gh + f * sG + (long long)x * PY + y, 1) * (g.idy * (1.0 / 256.0));
+  }
+  V[f * nc + c] = r;
+  (void)nv;
 #else
+#pragma unroll
+  for (int f = 0; f < nv; ++f) {
+    const double* a = fh + f * sF + (DIM == 2 ? (long long)x * g.ny + y : x);
+    const long long st = DIM == 2 ? g.ny : 1;
     double r = (central6(a + st, st) - central6(a, st)) / g.dx;
     if (DIM == 2) {
       const double* b = gh + f * sG + (long long)x * PY + y;
       r = r + (central6(b + 1, 1) - central6(b, 1)) / g.dy;
     }
-#endif
     V[f * nc + c] = r;
   }
+#endif
 }
 
 // The ghost-padded arrays themselves (boundary/boundary.py:120-132,

@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(AMR_UNT) k_amr_update_cells(MP m, long long nc
         const double res = (h - R[k] * T[k]) - e[k], d1 = cp[k] - R[k];
         if (fabs(res) > HALLEY_TOL) bits |= 1u;
         if (res != res) bits |= 2u;
-        Tn[k] = T[k] + ((-2.0 * res) * d1) * rcp_nr((2.0 * (d1 * d1)) - res * dcp);
+        Tn[k] = halley_next(T[k], res, d1, dcp);
       }
     }
     const int go = __syncthreads_or(bits & 1u), bad = __syncthreads_or(bits & 2u);

@@ -60,6 +60,40 @@ __device__ __forceinline__ double rcp_nr(double x) {
   const double e = fma(-x, r, 1.0);
   return fma(r, fma(e, e, e), r);
 }
+
+// exp(x) without branches: x = n ln 2 + r with the two-part ln 2 that fdlibm
+// publishes (Cody and Waite's reduction), |r| <= ln 2 / 2, the Taylor series
+// of e^r to r^13 (the remainder is below 4e-18) in its even and odd halves,
+// and 2^n as two factors, so that results down to the subnormals and up to
+// infinity come out of the products.  Within 2 ulp of exp; NaN stays NaN.
+// The library's exp branches on its range in every call, which keeps a
+// thread's exponentials from overlapping: the same throughput on a full chip,
+// a shorter chain on a short line.
+__device__ __forceinline__ double exp_nb(double x) {
+  const double xc = fmin(fmax(x, -1100.0), 1100.0);
+  const double big = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the nearest integer
+  const double t = fma(xc, 1.4426950408889634074, big), nd = t - big;
+  const int n = __double2loint(t);
+  const double r = fma(-nd, 1.90821492927058770002e-10, fma(-nd, 6.93147180369123816490e-01, xc));
+  const double r2 = r * r;
+  double pe = 1.0 / 479001600.0, po = 1.0 / 6227020800.0;
+  pe = fma(pe, r2, 1.0 / 3628800.0);
+  po = fma(po, r2, 1.0 / 39916800.0);
+  pe = fma(pe, r2, 1.0 / 40320.0);
+  po = fma(po, r2, 1.0 / 362880.0);
+  pe = fma(pe, r2, 1.0 / 720.0);
+  po = fma(po, r2, 1.0 / 5040.0);
+  pe = fma(pe, r2, 1.0 / 24.0);
+  po = fma(po, r2, 1.0 / 120.0);
+  pe = fma(pe, r2, 0.5);
+  po = fma(po, r2, 1.0 / 6.0);
+  pe = fma(pe, r2, 1.0);
+  po = fma(po, r2, 1.0);
+  const double p = fma(r, po, pe);
+  const int n1 = n >> 1, n2 = n - n1;
+  const double s1 = __hiloint2double((1023 + n1) << 20, 0), s2 = __hiloint2double((1023 + n2) << 20, 0);
+  return x != x ? x : __dmul_rn(__dmul_rn(p, s1), s2);
+}
 #endif
 
 // ---------------------------------------------------------------------------
@@ -232,6 +266,13 @@ __device__ __forceinline__ unsigned halley_iterates(const MP& m, double e, const
 }
 
 #if JB_FAST
+// One Halley step from the residual and its first two derivatives, its sums
+// fused in one way wherever it is inlined (instances of the ensemble match
+// the single-case solver bitwise).
+__device__ __forceinline__ double halley_next(double T, double res, double d1, double d2) {
+  return fma((-2.0 * res) * d1, rcp_nr(fma(-res, d2, 2.0 * (d1 * d1))), T);
+}
+
 // Fast-variant Halley iterates.  When every species switches NASA7 ranges at
 // the same temperature (m.tcr_uniform), the mixture's cp, dcp/dT and h are
 // polynomials in T whose coefficients are the Y-weighted sums of the
@@ -290,8 +331,7 @@ __device__ __forceinline__ unsigned halley_iterates_fast(const MP& m, double e, 
     const double d1 = cp - R;
     if (fabs(res) > HALLEY_TOL) bits |= 1u << i;
     if (res != res) bits |= 1u << (8 + i);
-    const double dT = ((-2.0 * res) * d1) * rcp_nr((2.0 * (d1 * d1)) - res * d2);
-    T = T + dT;
+    T = halley_next(T, res, d1, d2);
     cand[i + 1] = T;
   }
   return bits;
@@ -320,6 +360,45 @@ __device__ __forceinline__ int halley_count(unsigned word) {
 // ---------------------------------------------------------------------------
 // primitive recovery (solver_{1D,2D}/aux_func.py U_to_prim)
 // ---------------------------------------------------------------------------
+#if JB_FAST
+// The fast variants write their fused products out (fma, and __dmul_rn where
+// two products meet in a sum), so that a state's arithmetic rounds in one way
+// wherever it is inlined: the persistent 1D run, the ensemble and the single
+// launches give the same bits.
+//
+// prs = sum_k (rho Y_k) / M_k of a state's species fields rY = rho Y_k, with
+// rN = rho Y_N2 = rho - sum rho Y_k; the sums as trees, whose chains are a
+// third of the sequential ones.
+__device__ __forceinline__ double prim_sums(const MP& m, const double* rY, double rho, double& rN) {
+  rN = rho - (((rY[0] + rY[1]) + (rY[2] + rY[3])) + ((rY[4] + rY[5]) + (rY[6] + rY[7])));
+  const double p0 = fma(m.invM[1], rY[1], __dmul_rn(m.invM[0], rY[0]));
+  const double p1 = fma(m.invM[3], rY[3], __dmul_rn(m.invM[2], rY[2]));
+  const double p2 = fma(m.invM[5], rY[5], __dmul_rn(m.invM[4], rY[4]));
+  const double p3 = fma(m.invM[7], rY[7], __dmul_rn(m.invM[6], rY[6]));
+  return fma(m.invM[NR], rN, (p0 + p1) + (p2 + p3));
+}
+// prs, the mass fractions (the last one closing the balance) and R = prs / rho
+__device__ __forceinline__ void mix_sums(const MP& m, const double* rY, double rho, double ri, double* Yf,
+                                         double& prs, double& R) {
+  double rN;
+  prs = prim_sums(m, rY, rho, rN);
+  R = prs * ri;
+#pragma unroll
+  for (int k = 0; k < NR; ++k) Yf[k] = __dmul_rn(rY[k], ri);
+  Yf[NR] = __dmul_rn(rN, ri);
+}
+
+// The SSP-RK3 combination of stage STAGE (TVD_RK3.py:5-12): un of U^n, uk of
+// the stage input, L its flux divergence.
+template <int STAGE>
+__device__ __forceinline__ double rk_stage(double un, double uk, double dt, double L) {
+  const double s = fma(dt, L, uk);
+  if (STAGE == 1) return s;
+  if (STAGE == 2) return fma(1.0 / 4.0, s, __dmul_rn(3.0 / 4.0, un));
+  return fma(2.0 / 3.0, s, __dmul_rn(1.0 / 3.0, un));
+}
+#endif
+
 template <int DIM>
 struct Prim {
   double rho, u, v, p, a, R;
@@ -335,10 +414,8 @@ __device__ __forceinline__ Prim<DIM> u_to_prim(const MP& m, const double* q, dou
   const double ri = 1.0 / r.rho;
   r.u = q[1] * ri;
   r.v = DIM == 2 ? q[2] * ri : 0.0;
-  double sr = q[nY], pr = m.invM[0] * q[nY];
-#pragma unroll
-  for (int k = 1; k < NR; ++k) { sr += q[nY + k]; pr += m.invM[k] * q[nY + k]; }
-  pr += m.invM[NR] * (r.rho - sr);
+  double rN;
+  const double pr = prim_sums(m, q + nY, r.rho, rN);
   r.R = pr * ri;
   r.p = pr * T;
   r.a = sqrt(gamma * r.p * ri);
@@ -426,7 +503,7 @@ __device__ __forceinline__ double halley_cell(const MP& m, double e, const doubl
 #pragma unroll 1
     for (int i = 0; i < HALLEY_MAX && halley_go(res, polished); ++i) {
       const double d1 = cp - R;
-      T = T + ((-2.0 * res) * d1) * rcp_nr((2.0 * (d1 * d1)) - res * d2);
+      T = halley_next(T, res, d1, d2);
       const bool lo_i = T < Tcr;
       if (lo_i != lo) {  // the iterate crossed the range boundary (rare)
         lo = lo_i;
@@ -471,25 +548,13 @@ __device__ __forceinline__ unsigned finish_state(const MP& m, const Grid& g, con
   const double rho = q[0];
 #if JB_FAST
   if constexpr (CELL) {
-    // one reciprocal of rho; the primitives of the wave speeds as u_to_prim
-    // forms them (p = T sum_k (rho Y_k)/M_k, rho Y_N2 = rho - sum rho Y_k)
-    // are taken before the solve so that the state is no longer needed
+    // one reciprocal of rho; p = T sum_k (rho Y_k)/M_k with rho Y_N2 = rho -
+    // sum rho Y_k as u_to_prim forms it, R from the same sum
     const double ri = 1.0 / rho;
     const double u = q[1] * ri, v = DIM == 2 ? q[2] * ri : 0.0;
-    const double e = DIM == 2 ? q[3] * ri - 0.5 * (u * u + v * v) : q[2] * ri - 0.5 * (u * u);
-    double Y8[NR], Yf[NS];
-    double sr = q[nY], prs = m.invM[0] * q[nY];
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      Y8[k] = q[nY + k] * ri;
-      if (k > 0) {
-        sr += q[nY + k];
-        prs += m.invM[k] * q[nY + k];
-      }
-    }
-    prs += m.invM[NR] * (rho - sr);
-    fill_Y(Y8, Yf);
-    const double R = get_R(m, Yf);
+    const double e = fma(q[nY - 1], ri, -0.5 * (DIM == 2 ? fma(u, u, v * v) : u * u));
+    double Yf[NS], prs, R;
+    mix_sums(m, q + nY, rho, ri, Yf, prs, R);
     double cp;
     const double T = halley_cell(m, e, Yf, R, T0, cp);
     const double gamma = cp / (cp - R);
@@ -523,21 +588,22 @@ __device__ __forceinline__ unsigned finish_state(const MP& m, const Grid& g, con
 #endif
   {
     (void)amx; (void)amy; (void)dtm; (void)slots;
-    double Y8[NR], Yf[NS];
+    double Yf[NS];
 #if JB_FAST
     const double ri = 1.0 / rho;
     const double u = q[1] * ri, v = DIM == 2 ? q[2] * ri : 0.0;
-    const double e = q[nY - 1] * ri - 0.5 * (u * u + v * v);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] * ri;
+    const double e = fma(q[nY - 1], ri, -0.5 * (DIM == 2 ? fma(u, u, v * v) : u * u));
+    double prs, R;
+    mix_sums(m, q + nY, rho, ri, Yf, prs, R);
 #else
+    double Y8[NR];
     const double u = q[1] / rho, v = DIM == 2 ? q[2] / rho : 0.0;
     const double e = q[nY - 1] / rho - 0.5 * (u * u + v * v);
 #pragma unroll
     for (int k = 0; k < NR; ++k) Y8[k] = q[nY + k] / rho;
-#endif
     fill_Y(Y8, Yf);
     const double R = get_R(m, Yf);
+#endif
     double cnd[JB_NCAND];
     const unsigned bits = halley_any(m, e, Yf, R, T0, cnd);
 #pragma unroll
@@ -564,6 +630,30 @@ __device__ void pressure_outlet_state(const MP& m, const double* q, double gamma
                                       double normal_vel, double Pb, double* out) {
   constexpr int nY = DIM == 1 ? 3 : 4;
   constexpr int nv = nY + NR;
+#if JB_FAST
+  if (m.tcr_uniform) {
+    // one reciprocal of rho and the mixture's enthalpy polynomial: this is one
+    // thread's chain, and the whole launch waits for it
+    const double rho = q[0], ri = 1.0 / rho;
+    const double u = q[1] * ri, v = DIM == 2 ? q[2] * ri : 0.0;
+    double Yf[NS], prs, R, H[6], h, cp, dcp;
+    mix_sums(m, q + nY, rho, ri, Yf, prs, R);
+    const double p = prs * T, RT = R * T;
+    const bool sub = normal_vel < sqrt(gamma * RT);
+    const double rho_c = sub ? Pb / RT : rho, p_c = sub ? Pb : p, T_c = sub ? p_c / (rho_c * R) : T;
+    mix_h(m, Yf, T_c < m.Tcr[0], H);
+    poly6_d2(H, T_c, h, cp, dcp);
+    out[0] = rho_c;
+    out[1] = rho_c * u;
+    if (DIM == 2) out[2] = rho_c * v;
+    out[nY - 1] = fma(rho_c, fma(0.5, DIM == 2 ? fma(u, u, v * v) : u * u, h), -p_c);
+#pragma unroll
+    for (int k = 0; k < NR; ++k) out[nY + k] = rho_c * Yf[k];
+    out[nv] = cp / (cp - R);
+    out[nv + 1] = T_c;
+    return;
+  }
+#endif
   double rho = q[0];
   double u = q[1] / rho;
   double v = DIM == 2 ? q[2] / rho : 0.0;
@@ -747,7 +837,7 @@ __device__ __forceinline__ void weno_side(double dmm, double dm, double dp, doub
   const double t1 = fma(3.0, dm, -dmm), t2 = dm + dp, t3 = fma(3.0, dp, -dpp);
   const double e1 = fma(t1, t1, Da), e2 = fma(t2, t2, Db), e3 = fma(t3, t3, Dc);
   const double p1 = e2 * e3, p2 = e1 * e3, p3 = e1 * e2;
-  const double a1 = p1 * p1, a2 = 6.0 * (p2 * p2), a3 = 3.0 * (p3 * p3);
+  const double a1 = __dmul_rn(p1, p1), a2 = __dmul_rn(6.0, p2 * p2), a3 = __dmul_rn(3.0, p3 * p3);
   num = fma(a3, t3 + dp, fma(a2, t2 + dp, a1 * fma(2.0, t1, -dm)));
   den = (a1 + a2) + a3;
 }
@@ -1004,7 +1094,7 @@ __device__ __forceinline__ void weno_side(float dmm, float dm, float dp, float d
   const float t1 = fmaf(3.f, dm, -dmm), t2 = dm + dp, t3 = fmaf(3.f, dp, -dpp);
   const float e1 = fmaf(t1, t1, Da), e2 = fmaf(t2, t2, Db), e3 = fmaf(t3, t3, Dc);
   const float r1 = fminf(e2 * rcp_fast(e1), 6.5e4f), r3 = fminf(e2 * rcp_fast(e3), 6.5e4f);
-  const float a1 = r1 * r1, a3 = 3.f * (r3 * r3);
+  const float a1 = __fmul_rn(r1, r1), a3 = __fmul_rn(3.f, r3 * r3);
   num = fmaf(a3, t3 + dp, fmaf(a1, fmaf(2.f, t1, -dm), 6.f * (t2 + dp)));
   den = (a1 + 6.f) + a3;
 }
@@ -1105,13 +1195,13 @@ __device__ __forceinline__ void flux_prims(const MP& m, const float* q, float T,
   const float ri = __fdividef(1.f, rho);
   u = q[1] * ri;
   v = DIM == 2 ? q[2] * ri : 0.f;
-  float sr = q[nY], pr = (float)m.invM[0] * q[nY];
-#pragma unroll
-  for (int k = 1; k < NR; ++k) {
-    sr += q[nY + k];
-    pr += (float)m.invM[k] * q[nY + k];
-  }
-  pr += (float)m.invM[NR] * (rho - sr);
+  const float* r = q + nY;
+  const float rN = rho - (((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7])));
+  const float p0 = fmaf((float)m.invM[1], r[1], __fmul_rn((float)m.invM[0], r[0]));
+  const float p1 = fmaf((float)m.invM[3], r[3], __fmul_rn((float)m.invM[2], r[2]));
+  const float p2 = fmaf((float)m.invM[5], r[5], __fmul_rn((float)m.invM[4], r[4]));
+  const float p3 = fmaf((float)m.invM[7], r[7], __fmul_rn((float)m.invM[6], r[6]));
+  const float pr = fmaf((float)m.invM[NR], rN, (p0 + p1) + (p2 + p3));
   p = pr * T;
 }
 #endif
@@ -1856,45 +1946,8 @@ __device__ __forceinline__ void lu_solve(double (&J)[NR][NR], double (&b)[NR], d
   }
 }
 
-// (I/dt - M_k J) x = M_k w by LU with partial pivoting, then
-// detailed_reaction's clip and S = rho dY (construct_matrix_equation,
-// reaction_model.py:132-159 and :183-193; the reference solves with
-// jnp.linalg.solve, a partially pivoted LU).  The fast variants first test
-// the matrix for diagonal dominance by columns: partial pivoting then never
-// exchanges rows (each diagonal entry is the first maximum of its column, and
-// elimination keeps the dominance), so the elimination without the pivot
-// search and exchanges computes the same values; the other cells (the hot
-// reaction zone, where M_k J outweighs 1/dt) take the pivoted form.
-__device__ __forceinline__ void chem_solve(const MP& m, double (&J)[NR][NR], const double* w, double rho,
-                                           const double* Y8, double dt, double* S, unsigned& st) {
-  double b[NR];
-  const double idt = 1.0 / dt;
-#pragma unroll
-  for (int k = 0; k < NR; ++k) {
-    b[k] = m.M[k] * w[k];
-#pragma unroll
-    for (int n = 0; n < NR; ++n) {
-      double jk = m.M[k] * J[k][n];
-      J[k][n] = (k == n ? idt : 0.0) - jk;  // J now holds A
-    }
-  }
-  double x[NR];
-#if JB_FAST
-  bool cdd = true;
-#pragma unroll
-  for (int c = 0; c < NR; ++c) {
-    double off = 0.0;
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-      if (r != c) off += fabs(J[r][c]);
-    cdd = cdd && fabs(J[c][c]) > off;
-  }
-  if (cdd) lu_solve<false>(J, b, x, st);
-  else lu_solve<true>(J, b, x, st);
-#else
-  lu_solve<true>(J, b, x, st);
-#endif
-  // detailed_reaction (:183-193): dY = clip(drhoY/rho, -Y, 1-Y); S = rho dY
+// detailed_reaction (:183-193): dY = clip(drhoY/rho, -Y, 1-Y); S = rho dY
+__device__ __forceinline__ void chem_clip(const double* x, double rho, const double* Y8, double* S) {
 #if JB_FAST
   const double irho = 1.0 / rho;
 #endif
@@ -1916,6 +1969,50 @@ __device__ __forceinline__ void chem_solve(const MP& m, double (&J)[NR][NR], con
   }
 }
 
+// (I/dt - M_k J) x = M_k w by LU with partial pivoting, then
+// detailed_reaction's clip and S = rho dY (construct_matrix_equation,
+// reaction_model.py:132-159 and :183-193; the reference solves with
+// jnp.linalg.solve, a partially pivoted LU).  The fast variants first test
+// the matrix for diagonal dominance by columns: partial pivoting then never
+// exchanges rows (each diagonal entry is the first maximum of its column, and
+// elimination keeps the dominance), so the elimination without the pivot
+// search and exchanges computes the same values; the other cells (the hot
+// reaction zone, where M_k J outweighs 1/dt) take the pivoted form.
+__device__ __forceinline__ void chem_solve(const MP& m, double (&J)[NR][NR], const double* w, double rho,
+                                           const double* Y8, double dt, double* S, unsigned& st) {
+  double b[NR];
+  const double idt = 1.0 / dt;
+#pragma unroll
+  for (int k = 0; k < NR; ++k) {
+    b[k] = m.M[k] * w[k];
+#pragma unroll
+    for (int n = 0; n < NR; ++n) {
+#if JB_FAST
+      J[k][n] = fma(-m.M[k], J[k][n], k == n ? idt : 0.0);  // J now holds A
+#else
+      double jk = m.M[k] * J[k][n];
+      J[k][n] = (k == n ? idt : 0.0) - jk;  // J now holds A
+#endif
+    }
+  }
+  double x[NR];
+#if JB_FAST
+  bool cdd = true;
+#pragma unroll
+  for (int c = 0; c < NR; ++c) {
+    double off = 0.0;
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+      if (r != c) off += fabs(J[r][c]);
+    cdd = cdd && fabs(J[c][c]) > off;
+  }
+  if (cdd) lu_solve<false>(J, b, x, st);
+  else lu_solve<true>(J, b, x, st);
+#else
+  lu_solve<true>(J, b, x, st);
+#endif
+  chem_clip(x, rho, Y8, S);
+}
 
 // Rates, analytic Jacobian d(omega)/d(rho Y) and the solve of
 // (I/dt - J) x = omega for one cell.  Returns S_k = rho * clip(x_k/rho).
@@ -2023,7 +2120,7 @@ __device__ __forceinline__ double chem_gibbs(const MP& m, int k, double T, const
   return fma(-h, in.invT, s);
 }
 __device__ __forceinline__ void chem_equil(double gk, double& E, double& iE) {
-  E = exp(gk);
+  E = exp_nb(gk);
   iE = rcp_nr(fmin(fmax(E, 1e-300), 1e300));  // finite where E over- or underflows
 }
 
@@ -2065,21 +2162,26 @@ __device__ __forceinline__ void chem_cell_gen(const MP& m, double rho, const dou
 
 // The same for the 32 cells of a block of four warps: warp w takes two
 // species' equilibrium factors, every fourth reaction, and two columns of the
-// Jacobian of its lane's cell, warp 0 the solve (S and st are warp 0's).  A
-// cell's chemistry is one long chain of latencies in a single thread (17 us at
-// any grid that leaves the chip idle); here four threads share it.  Sums run
-// in the order of chem_cell_gen, so the two agree bitwise.  sh: the block's
-// [CHEM_SPLIT_ROWS][32] shared doubles; every thread of the block calls it,
-// and a block barrier separates it from the next use of sh.
-constexpr int CHEM_SPLIT_ROWS = JB_GEN_ROWS + 2 * NR + NR + NR * NR;
+// matrix of its lane's cell; then four neighbouring lanes share a cell's
+// solve, two rows each (chem_lu4).  A cell's chemistry is one long chain of
+// latencies in a single thread (17 us at any grid that leaves the chip idle).
+// Sums run in the order of chem_cell_gen and the pivots are its pivots, so
+// the two agree bitwise.  S is warp 0's, of its lane's cell.  sh: the block's
+// shared doubles (CHEM_SPLIT_SH); every thread of the block calls it, and a
+// block barrier separates it from the next use of sh.
+//
+// The matrix rows have a stride of 36 doubles: the four lanes of a cell read
+// rows 36 apart, which puts the 16 lanes of an access on 16 banks.
+constexpr int CS_LD = 36, CS_E = JB_GEN_ROWS * 32, CS_B = CS_E + 2 * NR * 32, CS_A = CS_B + NR * CS_LD;
+constexpr int CHEM_SPLIT_SH = CS_A + NR * NR * CS_LD;
 template <int G>
-__device__ __forceinline__ void chem_split_part(const MP& m, const ChemIn& in, double* col) {
+__device__ __forceinline__ void chem_split_part(const MP& m, const ChemIn& in, double idt, double* sh, int lane) {
+  double* col = sh + lane;
   double E[NR], iE[NR], none[NR];
-  const double* e = col + JB_GEN_ROWS * 32;
 #pragma unroll
   for (int k = 0; k < NR; ++k) {
-    E[k] = e[k * 32];
-    iE[k] = e[(NR + k) * 32];
+    E[k] = col[CS_E + k * 32];
+    iE[k] = col[CS_E + (NR + k) * 32];
   }
   chem_rates_gen<G>(m, in.lT, in.invT, in.Tp, in.pT, in.X, in.Xc, E, iE, col, 32, none);
   __syncthreads();
@@ -2089,49 +2191,137 @@ __device__ __forceinline__ void chem_split_part(const MP& m, const ChemIn& in, d
     if (k / 2 == G) rMX[k] = m.invM[k] * rcp_nr(in.Xc[k]);
   chem_jac_gen<G>(m, rMX, col, 32, J);
   chem_w_gen<G>(col, 32, w2);
-  double* w = col + (JB_GEN_ROWS + 2 * NR) * 32;
-  double* j = w + NR * 32;
+  // the matrix I/dt - M_k J and the right-hand side M_k w as chem_solve forms them
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    w[(2 * G + i) * 32] = w2[i];
+    col[CS_B + (2 * G + i) * CS_LD] = m.M[2 * G + i] * w2[i];
 #pragma unroll
-    for (int k = 0; k < NR; ++k) j[(k * NR + 2 * G + i) * 32] = J[k][2 * G + i];
+    for (int k = 0; k < NR; ++k) {
+      col[CS_A + ((2 * G + i) * NR + k) * CS_LD] = fma(-m.M[k], J[k][2 * G + i], k == 2 * G + i ? idt : 0.0);
+    }
   }
 }
+
+// Solve of cell threadIdx.x / 4's system by its four lanes, lane part holding
+// rows part and part + 4: Gaussian elimination with partial pivoting as
+// lu_solve<true> (first maximal |pivot| in the order its row exchanges would
+// give: pos is a row's place in that order), the rows staying where they are.
+// Every lane ends with the whole solution.
+__device__ __forceinline__ void chem_lu4(const double* sh, double (&x)[NR], unsigned& st) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, part = lane & 3, base = lane & ~3;
+  const double* c0 = sh + (threadIdx.x >> 2);
+  double a[2][NR], b[2], ipv[NR];
+  int pos[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int k = part + 4 * h;
+    pos[h] = k;
+    b[h] = c0[CS_B + k * CS_LD];
+#pragma unroll
+    for (int n = 0; n < NR; ++n) a[h][n] = c0[CS_A + (n * NR + k) * CS_LD];
+  }
+#pragma unroll
+  for (int c = 0; c < NR; ++c) {
+    // (key, pos, row) of the best candidate; the row now at place c wins
+    // against NaN, and a NaN elsewhere never wins, as its comparisons give
+    double key = -1.0;
+    int id = 0x7fffffff;  // pos * 8 + row
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      double v = fabs(a[h][c]);
+      if (v != v) v = pos[h] == c ? __longlong_as_double(0x7ff0000000000000LL) : -1.0;
+      if (pos[h] < c) v = -2.0;
+      const int i = pos[h] * 8 + part + 4 * h;
+      if (v > key || (v == key && i < id)) {
+        key = v;
+        id = i;
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      const double k2 = __shfl_xor_sync(full, key, o);
+      const int i2 = __shfl_xor_sync(full, id, o);
+      if (k2 > key || (k2 == key && i2 < id)) {
+        key = k2;
+        id = i2;
+      }
+    }
+    const int prow = id & 7, ppos = id >> 3, src = base | (prow & 3);
+    const bool hi = prow >= 4;
+    double pr[NR];
+#pragma unroll
+    for (int j = 0; j < NR; ++j)
+      if (j >= c) pr[j] = __shfl_sync(full, hi ? a[1][j] : a[0][j], src);
+    const double pb = __shfl_sync(full, hi ? b[1] : b[0], src);
+    if (pr[c] == 0.0) st |= JB_ERR_SINGULAR;
+    ipv[c] = rcp_nr(pr[c]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const bool is_pivot = part + 4 * h == prow;
+      if (is_pivot) pos[h] = c;
+      else if (pos[h] == c) pos[h] = ppos;
+      if (pos[h] > c) {
+        const double l = a[h][c] * ipv[c];
+#pragma unroll
+        for (int j = 0; j < NR; ++j)
+          if (j > c) a[h][j] = a[h][j] - l * pr[j];
+        b[h] = b[h] - l * pb;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NR; ++i) {
+    const int r = NR - 1 - i;
+    const bool h1 = pos[1] == r;
+    double s = h1 ? b[1] : b[0];
+#pragma unroll
+    for (int j = 0; j < NR; ++j)
+      if (j > r) s = s - (h1 ? a[1][j] : a[0][j]) * x[j];
+    s = s * ipv[r];
+    // the one lane of the four that holds the row at place r
+    const unsigned own = __ballot_sync(full, h1 || pos[0] == r) >> base & 15u;
+    x[r] = __shfl_sync(full, s, base | (__ffs(own) - 1));
+  }
+}
+
 __device__ __forceinline__ void chem_split(const MP& m, double rho, const double* Y8, double T, double dt, double* S,
                                            unsigned& st, double* sh) {
-  double* col = sh + (threadIdx.x & 31);
-  const int wp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   ChemIn in;
   chem_in(m, rho, Y8, T, in);
-  double* e = col + JB_GEN_ROWS * 32;
+  const double idt = 1.0 / dt;
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int k = 2 * wp + i;
     double E, iE;
     chem_equil(T < m.Tcr[k] ? chem_gibbs<true>(m, k, T, in) : chem_gibbs<false>(m, k, T, in), E, iE);
-    e[k * 32] = E;
-    e[(NR + k) * 32] = iE;
+    sh[CS_E + k * 32 + lane] = E;
+    sh[CS_E + (NR + k) * 32 + lane] = iE;
   }
   __syncthreads();
   switch (wp) {  // each case holds one more block barrier
-    case 0: chem_split_part<0>(m, in, col); break;
-    case 1: chem_split_part<1>(m, in, col); break;
-    case 2: chem_split_part<2>(m, in, col); break;
-    default: chem_split_part<3>(m, in, col); break;
+    case 0: chem_split_part<0>(m, in, idt, sh, lane); break;
+    case 1: chem_split_part<1>(m, in, idt, sh, lane); break;
+    case 2: chem_split_part<2>(m, in, idt, sh, lane); break;
+    default: chem_split_part<3>(m, in, idt, sh, lane); break;
   }
   __syncthreads();
+  double x[NR];
+  unsigned s1 = 0;
+  chem_lu4(sh, x, s1);
+  // each cell's solution over its right-hand side, which only its own four
+  // lanes (of one warp) read
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < NR; ++k)
+    if (k % 4 == (lane & 3)) sh[CS_B + k * CS_LD + (threadIdx.x >> 2)] = x[k];
+  st |= s1;
+  __syncthreads();
   if (wp == 0) {
-    const double* w = col + (JB_GEN_ROWS + 2 * NR) * 32;
-    const double* j = w + NR * 32;
-    double J[NR][NR], wk[NR];
 #pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      wk[k] = w[k * 32];
-#pragma unroll
-      for (int n = 0; n < NR; ++n) J[k][n] = j[(k * NR + n) * 32];
-    }
-    chem_solve(m, J, wk, rho, Y8, dt, S, st);
+    for (int k = 0; k < NR; ++k) x[k] = sh[CS_B + k * CS_LD + lane];
+    chem_clip(x, rho, Y8, S);
   }
 }
 #endif
@@ -2177,10 +2367,9 @@ __device__ __forceinline__ void chem_split_step(const MP& m, const Grid& g, cons
   const double ri = 1.0 / q[0];
 #pragma unroll
   for (int k = 0; k < NR; ++k) Y8[k] = __dmul_rn(q[nY + k], ri);
-  unsigned s1 = 0;
-  chem_split(m, q[0], Y8, T, dt, S, s1, sh);
+  // (a singular system may be reported by any warp; padding lanes repeat a live cell)
+  chem_split(m, q[0], Y8, T, dt, S, st, sh);
   if (threadIdx.x < 32 && live) {
-    st |= s1;
 #pragma unroll
     for (int f = 1; f < nY; ++f) q[f] = U[f * nc + c];
     chem_store<DIM, WRITE_S, CELL>(m, g, q, S, T, out, fin, c, bits, amx, amy, dtm, slots);
@@ -2271,10 +2460,13 @@ __global__ void __launch_bounds__(JB_CHEM_NT, JB_CHEM_MINB) k_chem(MP m, Grid g,
 #if JB_FAST
 // k_chem with four threads a cell (chem_split), 32 cells a block.
 template <int DIM, bool WRITE_S, bool CELL>
-__global__ void __launch_bounds__(128, 3) k_chem_split(MP m, Grid g, const double* __restrict__ U,
+#ifndef JB_CHEM_SPLIT_MINB
+#define JB_CHEM_SPLIT_MINB 4
+#endif
+__global__ void __launch_bounds__(128, JB_CHEM_SPLIT_MINB) k_chem_split(MP m, Grid g, const double* __restrict__ U,
                                                      const double* __restrict__ aux, double* __restrict__ out,
                                                      jb_fin fin, Slots* slots, double dt_arg) {
-  __shared__ double sh[CHEM_SPLIT_ROWS * 32];
+  __shared__ double sh[CHEM_SPLIT_SH];
   const long long c0 = (long long)blockIdx.x * 32 + (threadIdx.x & 31);
   const bool live = c0 < g.ncell;
   const long long c = live ? c0 : g.ncell - 1;

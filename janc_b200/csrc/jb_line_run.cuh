@@ -253,7 +253,7 @@ int lr_resident(size_t sm) {
 
 template <class V, int S>
 bool lr_try(const MP& m, const Grid& g, const LineRun& a, cudaStream_t st, cudaError_t& err) {
-  constexpr size_t chem = sizeof(double) * (S == 32 ? CHEM_SPLIT_ROWS * 32 : CHEM_SH * LR_NT), line = line_smem<V, S>(), sm = chem > line ? chem : line;
+  constexpr size_t chem = sizeof(double) * (S == 32 ? CHEM_SPLIT_SH : CHEM_SH * LR_NT), line = line_smem<V, S>(), sm = chem > line ? chem : line;
   const int nb = (g.nx + S - 1) / S;
   if (nb > lr_resident<V, S>(sm)) return false;
   void* args[] = {(void*)&m, (void*)&g, (void*)&a};

@@ -44,6 +44,7 @@ __device__ __forceinline__ double vsub(double a, double b) { return a - b; }
 __device__ __forceinline__ float vsub(float a, float b) { return a - b; }
 __device__ __forceinline__ double vmul(double a, double b) { return a * b; }
 __device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ f2 vadd(f2 a, f2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ f2 vsub(f2 a, f2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ f2 vmul(f2 a, f2 b) { return __fmul2_rn(a, b); }
@@ -138,8 +139,8 @@ __device__ __forceinline__ void win_push(Win<V>& w, V fn, V& base, V& num, V& de
 __device__ __forceinline__ void split_pack(int j, int dir, double q, double vel, double p, double al, double& hp,
                                            double& hm) {
   double F = vel * q;
-  if (j == 1 + dir) F += p;
-  if (j == 3) F += vel * p;
+  if (j == 1 + dir) F = fma(vel, q, p);
+  if (j == 3) F = fma(vel, p, F);
   hp = fma(al, q, F);
   hm = fma(-al, q, F);
 }
@@ -400,15 +401,11 @@ __global__ void __launch_bounds__(YR_S, VT<V>::W == 2 ? JB_YR_MINB : JB_YRD_MINB
 #pragma unroll
       for (int h = 0; h < W; ++h) {
         const int f = W * i + h;
-        const double rhs =
-            dt * visc_add<VISC>(g, f, cell, -((double)vget(dF, h) * hx + (double)vget(dG, h) * hy));
-        double r = rhs;
-        if (STAGE > 0) {
-          const double uk = Uk[f * nc + cell];  // read again (L1): no registers held across the WENO
-          if (STAGE == 1) r = uk + rhs;
-          else if (STAGE == 2) r = 3.0 / 4.0 * Un[f * nc + cell] + 1.0 / 4.0 * (uk + rhs);
-          else r = 1.0 / 3.0 * Un[f * nc + cell] + 2.0 / 3.0 * (uk + rhs);
-        }
+        const double L =
+            visc_add<VISC>(g, f, cell, -fma((double)vget(dF, h), hx, __dmul_rn((double)vget(dG, h), hy)));
+        // Uk is read again (L1): no registers held across the WENO
+        const double r = STAGE == 0 ? dt * L
+                                    : rk_stage<STAGE>(STAGE == 1 ? 0.0 : Un[f * nc + cell], Uk[f * nc + cell], dt, L);
         out[f * nc + cell] = r;
         q[f] = r;
       }
@@ -478,10 +475,10 @@ __device__ __forceinline__ unsigned line_tile(const MP& m, const Grid& g, const 
 #pragma unroll
     for (int f = 0; f < L1_NF; ++f) {
       V Fl = u * q[f];
-      if (f == 1) Fl += p;
-      if (f == 2) Fl += u * p;
-      sHp[f * C + at] = Fl + al * q[f];
-      sHm[f * C + at] = Fl - al * q[f];
+      if (f == 1) Fl = vfma(u, q[f], p);
+      if (f == 2) Fl = vfma(u, p, Fl);
+      sHp[f * C + at] = vfma(al, q[f], Fl);
+      sHm[f * C + at] = vfma(-al, q[f], Fl);
     }
   }
   __syncthreads();
@@ -498,15 +495,9 @@ __device__ __forceinline__ unsigned line_tile(const MP& m, const Grid& g, const 
 #pragma unroll
     for (int f = 0; f < L1_NF; ++f) {
       const double dF = (double)(sF[f * F + yr_at(tid + 1)] - sF[f * F + yr_at(tid)]);
-      const double rhs = dt * visc_add<VISC>(g, f, cell, -(dF * hx));
-      double r = rhs;
-      if (STAGE > 0) {
-        const double uk = Uk[f * nc + cell];
-        if (STAGE == 1) r = uk + rhs;
-        else if (STAGE == 2) r = 3.0 / 4.0 * Un[f * nc + cell] + 1.0 / 4.0 * (uk + rhs);
-        else r = 1.0 / 3.0 * Un[f * nc + cell] + 2.0 / 3.0 * (uk + rhs);
-      }
-      q[f] = r;
+      const double L = visc_add<VISC>(g, f, cell, __dmul_rn(-dF, hx));
+      q[f] = STAGE == 0 ? dt * L
+                        : rk_stage<STAGE>(STAGE == 1 ? 0.0 : Un[f * nc + cell], Uk[f * nc + cell], dt, L);
     }
 #pragma unroll
     for (int f = 0; f < L1_NF; ++f) out[f * nc + cell] = q[f];

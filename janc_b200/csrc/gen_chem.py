@@ -98,7 +98,7 @@ def generate(path=None):
             return [f"{arr}[{k}]" for k, c in terms for _ in range(c)]
 
         w(f"  if constexpr (G < 0 || G == {i % 4}) {{  // reaction {i}")
-        w(f"    const double k0 = exp_nb(fma(-m.EaR[{i}], invT, fma(m.B[{i}], lT, m.lnA[{i}])));")
+        w(f"    const double k0 = exp(fma(-m.EaR[{i}], invT, fma(m.B[{i}], lT, m.lnA[{i}])));")
         if is_tb[i]:
             js = [j for j in range(ns) if tb[i, j] != 0]
             expr = f"m.tb[{i}][{js[0]}] * X[{js[0]}]"

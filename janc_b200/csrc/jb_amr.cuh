@@ -18,7 +18,7 @@
 // One CTA per block, so each block's reductions stay inside its CTA:
 //   k_amr_stage   alpha of the padded block; the interior in tiles of
 //                 tx x ty cells, a shape the host picks per block size so
-//                 that few, well-filled tiles cover the block (LF + WENO5-JS
+//                 that few tiles cover the block (20 x 20 blocks: one) (LF + WENO5-JS
 //                 / MUSCL faces in shared memory, the RK combination); every
 //                 ghost entry takes the combination with a zero right-hand
 //                 side (the reference pads the rhs with zeros); update_aux
@@ -35,9 +35,27 @@
 namespace {  // internal linkage
 
 constexpr int AMR_NT = 256;
-constexpr int AMR_AQ_MAX = 640;  // padded cells of a tile, (tx + 6)(ty + 6)
-constexpr int AMR_H_MAX = 420;   // (tx + 6) ty and tx (ty + 6) when (tx + 1) ty, tx (ty + 1) <= 256
-constexpr size_t AMR_STAGE_SMEM = sizeof(double) * (4 * AMR_AQ_MAX + 4 * AMR_H_MAX + 2 * AMR_NT);
+// Shared doubles of a tx x ty tile: rho, u, v, p of its padded cells, and of
+// two fields at a time the split fluxes along both axes and the face values.
+__host__ __device__ constexpr int amr_tile_doubles(int tx, int ty) {
+  return 4 * (tx + 6) * (ty + 6) + 4 * ((tx + 6) * ty + tx * (ty + 6)) + 2 * ((tx + 1) * ty + tx * (ty + 1));
+}
+constexpr int AMR_SMEM_DOUBLES = 72 * 1024 / 8;  // three blocks an SM
+
+// Items i = tid, tid + AMR_NT, ... of an array with rows of w entries as (row,
+// column), stepped without a division.
+struct AmrIt {
+  int r, c, dr, dc, w;
+  __device__ __forceinline__ AmrIt(int tid, int w_) : r(tid / w_), c(tid % w_), dr(AMR_NT / w_), dc(AMR_NT % w_), w(w_) {}
+  __device__ __forceinline__ void next() {
+    r += dr;
+    c += dc;
+    if (c >= w) {
+      c -= w;
+      ++r;
+    }
+  }
+};
 
 struct AmrBlocks {
   int nb, bx, by, tx, ty;  // blocks, block cells, interior tile of k_amr_stage
@@ -149,7 +167,7 @@ typedef jb_amr_io AmrIO;  // the stage call's block arrays (jb_ops.h)
 // filled; U0: the step's first stage input.
 template <int STAGE>
 #ifndef JB_AMR_MINB
-#define JB_AMR_MINB 4  // 64 registers (8 B of spills)
+#define JB_AMR_MINB 3
 #endif
 __global__ void __launch_bounds__(AMR_NT, JB_AMR_MINB) k_amr_stage(MP m, Grid g, AmrBlocks B, AmrIO io, Slots* slots,
                                                     double dt) {
@@ -157,13 +175,12 @@ __global__ void __launch_bounds__(AMR_NT, JB_AMR_MINB) k_amr_stage(MP m, Grid g,
   constexpr int nv = 12;
   const int TX = B.tx, TY = B.ty, APX = TX + 6, APY = TY + 6, AQ = APX * APY;
   const int HX = APX * TY, HY = TX * APY;
+  const int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
   double* sP = reinterpret_cast<double*>(smraw);  // [4][APX][APY]: rho, u, v, p
-  double* sHxp = sP + 4 * AQ;                      // [APX][TY]
-  double* sHxm = sHxp + HX;
-  double* sHyp = sHxm + HX;                        // [TX][APY]
-  double* sHym = sHyp + HY;
-  double* sFx = sHym + HY;                         // [TX+1][TY]
-  double* sFy = sFx + (TX + 1) * TY;               // [TX][TY+1]
+  double* sHx = sP + 4 * AQ;                       // [2 fields][H+, H-][APX][TY]
+  double* sHy = sHx + 4 * HX;                      // [2][2][TX][APY]
+  double* sFx = sHy + 4 * HY;                      // [2][TX+1][TY]
+  double* sFy = sFx + 2 * NFX;                     // [2][TX][TY+1]
   const int tid = threadIdx.x;
   const int PX = B.bx + 6, PY = B.by + 6;
   const long long nc = (long long)PX * PY;
@@ -188,8 +205,6 @@ __global__ void __launch_bounds__(AMR_NT, JB_AMR_MINB) k_amr_stage(MP m, Grid g,
   amr_block_max2(ax, ay);
 
   // ---- the interior, tile by tile
-  const bool owner = tid < TX * TY;
-  const int ix = owner ? tid / TY : 0, iy = owner ? tid % TY : 0;
   const int ntx = (B.bx + TX - 1) / TX, nty = (B.by + TY - 1) / TY;
   for (int t = 0; t < ntx * nty; ++t) {
     const int x0 = (t / nty) * TX, y0 = (t % nty) * TY;  // interior coordinates of the tile
@@ -212,75 +227,86 @@ __global__ void __launch_bounds__(AMR_NT, JB_AMR_MINB) k_amr_stage(MP m, Grid g,
       sP[3 * AQ + i] = p;
     }
     __syncthreads();
-    const int gx = x0 + ix, gy = y0 + iy;
-    const bool live = owner && gx < B.bx && gy < B.by;
-    const long long cell = (long long)(gx + 3) * PY + (gy + 3);
-    for (int f = 0; f < nv; ++f) {
-      // split fluxes H+- = 0.5 (F +- alpha U) (flux_splitting/LF.py:4-16)
-      for (int i = tid; i < HX + HY; i += AMR_NT) {
-        int px, py, dir;
-        if (i < HX) { px = i / TY; py = i % TY + 3; dir = 0; }
-        else { const int j = i - HX; px = j / APY + 3; py = j % APY; dir = 1; }
+    // two fields at a time, two barriers a pair
+    for (int f0 = 0; f0 < nv; f0 += 2) {
+      // split fluxes H+- = 0.5 (F +- alpha U) (flux_splitting/LF.py:4-16) of
+      // tile cell (px, py) along dir into h[field][sign][n] at position k
+      auto split = [&](int dir, int px, int py, double al, double* h, int n, int k) {
         const int c = px * APY + py;
-        const int bxp = x0 + px, byp = y0 + py;
-        const long long gc = (long long)bxp * PY + byp;
-        const bool in = bxp < PX && byp < PY;
-        const double qf = in ? gU[f * nc + gc] : 1.0;
-        const double al = dir == 0 ? ax : ay;
-#if JB_FAST
-        // F = vel q + pressure terms: the reference's LF flux regrouped
-        const double vel = sP[(1 + dir) * AQ + c];
-        double F = vel * qf;
-        if (f == 1 + dir) F += sP[3 * AQ + c];
-        if (f == 3) F += vel * sP[3 * AQ + c];
-#else
+        const bool in = x0 + px < PX && y0 + py < PY;
+        const long long gc = (long long)(x0 + px) * PY + (y0 + py);
+#if !JB_FAST
         const double E = in ? gU[3 * nc + gc] : 1.0;
-        const double F = lf_flux<2>(f, dir, qf, sP[c], sP[AQ + c], sP[2 * AQ + c], sP[3 * AQ + c], E);
 #endif
-        const double hp = 0.5 * (F + al * qf), hm = 0.5 * (F - al * qf);
-        if (dir == 0) { sHxp[px * TY + (py - 3)] = hp; sHxm[px * TY + (py - 3)] = hm; }
-        else { sHyp[(px - 3) * APY + py] = hp; sHym[(px - 3) * APY + py] = hm; }
-      }
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+          const int f = f0 + d;
+          const double qf = in ? gU[f * nc + gc] : 1.0;
+#if JB_FAST
+          // F = vel q + pressure terms: the reference's LF flux regrouped
+          const double vel = sP[(1 + dir) * AQ + c];
+          double F = vel * qf;
+          if (f == 1 + dir) F += sP[3 * AQ + c];
+          if (f == 3) F += vel * sP[3 * AQ + c];
+#else
+          const double F = lf_flux<2>(f, dir, qf, sP[c], sP[AQ + c], sP[2 * AQ + c], sP[3 * AQ + c], E);
+#endif
+          h[(2 * d) * n + k] = 0.5 * (F + al * qf);
+          h[(2 * d + 1) * n + k] = 0.5 * (F - al * qf);
+        }
+      };
+      int k = tid;
+      for (AmrIt i(tid, TY); i.r < APX; i.next(), k += AMR_NT) split(0, i.r, i.c + 3, ax, sHx, HX, k);
+      k = tid;
+      for (AmrIt i(tid, APY); i.r < TX; i.next(), k += AMR_NT) split(1, i.r + 3, i.c, ay, sHy, HY, k);
       __syncthreads();
       // face values F = L(H+) + R(H-) (flux.py:56-68, WENO5_JS.py / MUSCL.py)
-      if (tid < (TX + 1) * TY) {
-        const int mxf = tid / TY, jy = tid % TY;
-        const double* hp = sHxp + jy;
-        const double* hm = sHxm + jy;
-        const double L = recon_L(g, hp[mxf * TY], hp[(mxf + 1) * TY], hp[(mxf + 2) * TY], hp[(mxf + 3) * TY],
-                                 hp[(mxf + 4) * TY]);
-        const double Rr = recon_R(g, hm[(mxf + 1) * TY], hm[(mxf + 2) * TY], hm[(mxf + 3) * TY],
-                                  hm[(mxf + 4) * TY], hm[(mxf + 5) * TY]);
-        sFx[mxf * TY + jy] = L + Rr;
-      }
-      if (tid < TX * (TY + 1)) {
-        const int jx = tid / (TY + 1), myf = tid % (TY + 1);
-        const double* gp = sHyp + jx * APY + myf;
-        const double* gm = sHym + jx * APY + myf;
-        const double Lg = recon_L(g, gp[0], gp[1], gp[2], gp[3], gp[4]);
-        const double Rg = recon_R(g, gm[1], gm[2], gm[3], gm[4], gm[5]);
-        sFy[jx * (TY + 1) + myf] = Lg + Rg;
+      auto face = [&](const double* hp, const double* hm, int s) {
+        return recon_L(g, hp[0], hp[s], hp[2 * s], hp[3 * s], hp[4 * s]) +
+               recon_R(g, hm[s], hm[2 * s], hm[3 * s], hm[4 * s], hm[5 * s]);
+      };
+#pragma unroll 1
+      for (int d = 0; d < 2; ++d) {
+        const double* hp = sHx + 2 * d * HX;
+#pragma unroll 1
+        for (k = tid; k < NFX; k += AMR_NT) sFx[d * NFX + k] = face(hp + k, hp + HX + k, TY);
+        const double* gp = sHy + 2 * d * HY;
+        k = tid;
+#pragma unroll 1
+        for (AmrIt i(tid, TY + 1); i.r < TX; i.next(), k += AMR_NT) {
+          const double* p = gp + i.r * APY + i.c;
+          sFy[d * NFY + k] = face(p, p + HY, 1);
+        }
       }
       __syncthreads();
-      // divergence and the RK combination (TVD_RK3.py:17, 24, 31)
-      if (live) {
-        const double dF = sFx[(ix + 1) * TY + iy] - sFx[ix * TY + iy];
-        const double dG = sFy[ix * (TY + 1) + iy + 1] - sFy[ix * (TY + 1) + iy];
+      // divergence and the RK combination (TVD_RK3.py:17, 24, 31); the next
+      // pair's split fluxes do not touch the face values
+      for (AmrIt i(tid, TY); i.r < TX; i.next()) {
+        const int gx = x0 + i.r, gy = y0 + i.c;
+        if (gx >= B.bx || gy >= B.by) continue;
+        const long long cell = (long long)(gx + 3) * PY + (gy + 3);
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+          const int f = f0 + d;
+          const double* Fx = sFx + d * NFX + i.r * TY + i.c;
+          const double* Fy = sFy + d * NFY + i.r * (TY + 1) + i.c;
+          const double dF = Fx[TY] - Fx[0], dG = Fy[1] - Fy[0];
 #if JB_FAST
-        const double rhs = dt * (-(dF * B.idx + dG * B.idy));
+          const double rhs = dt * (-(dF * B.idx + dG * B.idy));
 #else
-        const double rhs = dt * (-(dF / B.dx + dG / B.dy));
+          const double rhs = dt * (-(dF / B.dx + dG / B.dy));
 #endif
-        const double uk = gU[f * nc + cell];
-        double r;
-        if (STAGE == 0) r = rhs;
-        else if (STAGE == 1) r = uk + rhs;
-        else if (STAGE == 2) r = 3.0 / 4.0 * u0[f * nc + cell] + 1.0 / 4.0 * (uk + rhs);
-        else r = 1.0 / 3.0 * u0[f * nc + cell] + 2.0 / 3.0 * (uk + rhs);
-        oU[f * nc + cell] = r;
+          const double uk = gU[f * nc + cell];
+          double r;
+          if (STAGE == 0) r = rhs;
+          else if (STAGE == 1) r = uk + rhs;
+          else if (STAGE == 2) r = 3.0 / 4.0 * u0[f * nc + cell] + 1.0 / 4.0 * (uk + rhs);
+          else r = 1.0 / 3.0 * u0[f * nc + cell] + 2.0 / 3.0 * (uk + rhs);
+          oU[f * nc + cell] = r;
+        }
       }
-      __syncthreads();
     }
+    __syncthreads();  // the next tile's primitives replace this one's
   }
   // ---- ghost entries: the combination with the zero-padded rhs
   for (long long c = tid; c < nc; c += AMR_NT) {

@@ -41,7 +41,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     wk[7] = 0.0;
   }
   if constexpr (G < 0 || G == 0) {  // reaction 0
-    const double k0 = exp_nb(fma(-m.EaR[0], invT, fma(m.B[0], lT, m.lnA[0])));
+    const double k0 = exp(fma(-m.EaR[0], invT, fma(m.B[0], lT, m.lnA[0])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[0], Xc[1]);
     const double kb = __dmul_rn(k0 * E[0] * E[1] * iE[4] * iE[6] * Xc[4], Xc[6]);
@@ -58,7 +58,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(0 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 1) {  // reaction 1
-    const double k0 = exp_nb(fma(-m.EaR[1], invT, fma(m.B[1], lT, m.lnA[1])));
+    const double k0 = exp(fma(-m.EaR[1], invT, fma(m.B[1], lT, m.lnA[1])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[1], Xc[4]);
     const double kb = __dmul_rn(k0 * E[1] * E[4] * iE[2] * iE[3] * Xc[2], Xc[3]);
@@ -75,7 +75,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(3 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 2) {  // reaction 2
-    const double k0 = exp_nb(fma(-m.EaR[2], invT, fma(m.B[2], lT, m.lnA[2])));
+    const double k0 = exp(fma(-m.EaR[2], invT, fma(m.B[2], lT, m.lnA[2])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[0], Xc[3]);
     const double kb = __dmul_rn(k0 * E[0] * E[3] * iE[2] * iE[4] * Xc[2], Xc[4]);
@@ -92,7 +92,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(6 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 3) {  // reaction 3
-    const double k0 = exp_nb(fma(-m.EaR[3], invT, fma(m.B[3], lT, m.lnA[3])));
+    const double k0 = exp(fma(-m.EaR[3], invT, fma(m.B[3], lT, m.lnA[3])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[0], Xc[2]);
     const double kb = __dmul_rn(k0 * E[0] * E[2] * iE[4] * iE[5] * Xc[4], Xc[5]);
@@ -109,7 +109,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(9 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 0) {  // reaction 4
-    const double k0 = exp_nb(fma(-m.EaR[4], invT, fma(m.B[4], lT, m.lnA[4])));
+    const double k0 = exp(fma(-m.EaR[4], invT, fma(m.B[4], lT, m.lnA[4])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[2], Xc[2]);
     const double kb = __dmul_rn(k0 * E[2] * E[2] * iE[3] * iE[5] * Xc[3], Xc[5]);
@@ -125,7 +125,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(12 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 1) {  // reaction 5
-    const double k0 = exp_nb(fma(-m.EaR[5], invT, fma(m.B[5], lT, m.lnA[5])));
+    const double k0 = exp(fma(-m.EaR[5], invT, fma(m.B[5], lT, m.lnA[5])));
     const double Mi = fma(m.tb[5][8], X[8], fma(m.tb[5][7], X[7], fma(m.tb[5][6], X[6], fma(m.tb[5][5], X[5], fma(m.tb[5][4], X[4], fma(m.tb[5][3], X[3], fma(m.tb[5][2], X[2], fma(m.tb[5][1], X[1], m.tb[5][0] * X[0]))))))));
     const double kf = __dmul_rn(k0 * Xc[2], Xc[4]);
     const double kb = __dmul_rn(k0 * E[2] * E[4] * iE[5] * pT, Xc[5]);
@@ -143,7 +143,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(15 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 2) {  // reaction 6
-    const double k0 = exp_nb(fma(-m.EaR[6], invT, fma(m.B[6], lT, m.lnA[6])));
+    const double k0 = exp(fma(-m.EaR[6], invT, fma(m.B[6], lT, m.lnA[6])));
     const double Mi = fma(m.tb[6][8], X[8], fma(m.tb[6][7], X[7], fma(m.tb[6][6], X[6], fma(m.tb[6][5], X[5], fma(m.tb[6][4], X[4], fma(m.tb[6][3], X[3], fma(m.tb[6][2], X[2], fma(m.tb[6][1], X[1], m.tb[6][0] * X[0]))))))));
     const double kf = __dmul_rn(k0 * Xc[4], Xc[4]);
     const double kb = __dmul_rn(k0 * E[4] * E[4] * iE[0] * pT, Xc[0]);
@@ -160,7 +160,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(18 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 3) {  // reaction 7
-    const double k0 = exp_nb(fma(-m.EaR[7], invT, fma(m.B[7], lT, m.lnA[7])));
+    const double k0 = exp(fma(-m.EaR[7], invT, fma(m.B[7], lT, m.lnA[7])));
     const double Mi = fma(m.tb[7][8], X[8], fma(m.tb[7][7], X[7], fma(m.tb[7][6], X[6], fma(m.tb[7][5], X[5], fma(m.tb[7][4], X[4], fma(m.tb[7][3], X[3], fma(m.tb[7][2], X[2], fma(m.tb[7][1], X[1], m.tb[7][0] * X[0]))))))));
     const double kf = __dmul_rn(k0 * Xc[3], Xc[4]);
     const double kb = __dmul_rn(k0 * E[3] * E[4] * iE[2] * pT, Xc[2]);
@@ -178,7 +178,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(21 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 0) {  // reaction 8
-    const double k0 = exp_nb(fma(-m.EaR[8], invT, fma(m.B[8], lT, m.lnA[8])));
+    const double k0 = exp(fma(-m.EaR[8], invT, fma(m.B[8], lT, m.lnA[8])));
     const double Mi = fma(m.tb[8][8], X[8], fma(m.tb[8][7], X[7], fma(m.tb[8][6], X[6], fma(m.tb[8][5], X[5], fma(m.tb[8][4], X[4], fma(m.tb[8][3], X[3], fma(m.tb[8][2], X[2], fma(m.tb[8][1], X[1], m.tb[8][0] * X[0]))))))));
     const double kf = __dmul_rn(k0 * Xc[1], Xc[4]);
     const double kb = __dmul_rn(k0 * E[1] * E[4] * iE[6] * pT, Xc[6]);
@@ -196,7 +196,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(24 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 1) {  // reaction 9
-    const double k0 = exp_nb(fma(-m.EaR[9], invT, fma(m.B[9], lT, m.lnA[9])));
+    const double k0 = exp(fma(-m.EaR[9], invT, fma(m.B[9], lT, m.lnA[9])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[4], Xc[6]);
     const double kb = __dmul_rn(k0 * E[4] * E[6] * iE[2] * iE[2] * Xc[2], Xc[2]);
@@ -212,7 +212,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(27 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 2) {  // reaction 10
-    const double k0 = exp_nb(fma(-m.EaR[10], invT, fma(m.B[10], lT, m.lnA[10])));
+    const double k0 = exp(fma(-m.EaR[10], invT, fma(m.B[10], lT, m.lnA[10])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[4], Xc[6]);
     const double kb = __dmul_rn(k0 * E[4] * E[6] * iE[3] * iE[5] * Xc[3], Xc[5]);
@@ -229,7 +229,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(30 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 3) {  // reaction 11
-    const double k0 = exp_nb(fma(-m.EaR[11], invT, fma(m.B[11], lT, m.lnA[11])));
+    const double k0 = exp(fma(-m.EaR[11], invT, fma(m.B[11], lT, m.lnA[11])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[3], Xc[6]);
     const double kb = __dmul_rn(k0 * E[3] * E[6] * iE[1] * iE[2] * Xc[1], Xc[2]);
@@ -246,7 +246,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(33 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 0) {  // reaction 12
-    const double k0 = exp_nb(fma(-m.EaR[12], invT, fma(m.B[12], lT, m.lnA[12])));
+    const double k0 = exp(fma(-m.EaR[12], invT, fma(m.B[12], lT, m.lnA[12])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[2], Xc[6]);
     const double kb = __dmul_rn(k0 * E[2] * E[6] * iE[1] * iE[5] * Xc[1], Xc[5]);
@@ -263,7 +263,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(36 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 1) {  // reaction 13
-    const double k0 = exp_nb(fma(-m.EaR[13], invT, fma(m.B[13], lT, m.lnA[13])));
+    const double k0 = exp(fma(-m.EaR[13], invT, fma(m.B[13], lT, m.lnA[13])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[6], Xc[6]);
     const double kb = __dmul_rn(k0 * E[6] * E[6] * iE[1] * iE[7] * Xc[1], Xc[7]);
@@ -279,7 +279,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(39 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 2) {  // reaction 14
-    const double k0 = exp_nb(fma(-m.EaR[14], invT, fma(m.B[14], lT, m.lnA[14])));
+    const double k0 = exp(fma(-m.EaR[14], invT, fma(m.B[14], lT, m.lnA[14])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[4], Xc[7]);
     const double kb = __dmul_rn(k0 * E[4] * E[7] * iE[0] * iE[6] * Xc[0], Xc[6]);
@@ -296,7 +296,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(42 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 3) {  // reaction 15
-    const double k0 = exp_nb(fma(-m.EaR[15], invT, fma(m.B[15], lT, m.lnA[15])));
+    const double k0 = exp(fma(-m.EaR[15], invT, fma(m.B[15], lT, m.lnA[15])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[3], Xc[7]);
     const double kb = __dmul_rn(k0 * E[3] * E[7] * iE[2] * iE[6] * Xc[2], Xc[6]);
@@ -313,7 +313,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(45 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 0) {  // reaction 16
-    const double k0 = exp_nb(fma(-m.EaR[16], invT, fma(m.B[16], lT, m.lnA[16])));
+    const double k0 = exp(fma(-m.EaR[16], invT, fma(m.B[16], lT, m.lnA[16])));
     const double Mi = 1.0;
     const double kf = __dmul_rn(k0 * Xc[2], Xc[7]);
     const double kb = __dmul_rn(k0 * E[2] * E[7] * iE[5] * iE[6] * Xc[5], Xc[6]);
@@ -330,7 +330,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(48 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 1) {  // reaction 17
-    const double k0 = exp_nb(fma(-m.EaR[17], invT, fma(m.B[17], lT, m.lnA[17])));
+    const double k0 = exp(fma(-m.EaR[17], invT, fma(m.B[17], lT, m.lnA[17])));
     const double Mi = fma(m.tb[17][8], X[8], fma(m.tb[17][7], X[7], fma(m.tb[17][6], X[6], fma(m.tb[17][5], X[5], fma(m.tb[17][4], X[4], fma(m.tb[17][3], X[3], fma(m.tb[17][2], X[2], fma(m.tb[17][1], X[1], m.tb[17][0] * X[0]))))))));
     const double kf = __dmul_rn(k0, Xc[7]);
     const double kb = __dmul_rn(k0 * E[7] * iE[2] * iE[2] * Tp * Xc[2], Xc[2]);
@@ -347,7 +347,7 @@ __device__ __forceinline__ void chem_rates_gen(const MP& m, double lT, double in
     sh[(51 + 2) * stride] = Mi * kb;
   }
   if constexpr (G < 0 || G == 2) {  // reaction 18
-    const double k0 = exp_nb(fma(-m.EaR[18], invT, fma(m.B[18], lT, m.lnA[18])));
+    const double k0 = exp(fma(-m.EaR[18], invT, fma(m.B[18], lT, m.lnA[18])));
     const double Mi = fma(m.tb[18][8], X[8], fma(m.tb[18][7], X[7], fma(m.tb[18][6], X[6], fma(m.tb[18][5], X[5], fma(m.tb[18][4], X[4], fma(m.tb[18][3], X[3], fma(m.tb[18][2], X[2], fma(m.tb[18][1], X[1], m.tb[18][0] * X[0]))))))));
     const double kf = __dmul_rn(k0 * Xc[3], Xc[3]);
     const double kb = __dmul_rn(k0 * E[3] * E[3] * iE[1] * pT, Xc[1]);

@@ -60,40 +60,6 @@ __device__ __forceinline__ double rcp_nr(double x) {
   const double e = fma(-x, r, 1.0);
   return fma(r, fma(e, e, e), r);
 }
-
-// exp(x) without branches: x = n ln 2 + r with the two-part ln 2 that fdlibm
-// publishes (Cody and Waite's reduction), |r| <= ln 2 / 2, the Taylor series
-// of e^r to r^13 (the remainder is below 4e-18) in its even and odd halves,
-// and 2^n as two factors, so that results down to the subnormals and up to
-// infinity come out of the products.  Within 2 ulp of exp; NaN stays NaN.
-// The library's exp branches on its range in every call, which keeps a
-// thread's exponentials from overlapping: the same throughput on a full chip,
-// a shorter chain on a short line.
-__device__ __forceinline__ double exp_nb(double x) {
-  const double xc = fmin(fmax(x, -1100.0), 1100.0);
-  const double big = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the nearest integer
-  const double t = fma(xc, 1.4426950408889634074, big), nd = t - big;
-  const int n = __double2loint(t);
-  const double r = fma(-nd, 1.90821492927058770002e-10, fma(-nd, 6.93147180369123816490e-01, xc));
-  const double r2 = r * r;
-  double pe = 1.0 / 479001600.0, po = 1.0 / 6227020800.0;
-  pe = fma(pe, r2, 1.0 / 3628800.0);
-  po = fma(po, r2, 1.0 / 39916800.0);
-  pe = fma(pe, r2, 1.0 / 40320.0);
-  po = fma(po, r2, 1.0 / 362880.0);
-  pe = fma(pe, r2, 1.0 / 720.0);
-  po = fma(po, r2, 1.0 / 5040.0);
-  pe = fma(pe, r2, 1.0 / 24.0);
-  po = fma(po, r2, 1.0 / 120.0);
-  pe = fma(pe, r2, 0.5);
-  po = fma(po, r2, 1.0 / 6.0);
-  pe = fma(pe, r2, 1.0);
-  po = fma(po, r2, 1.0);
-  const double p = fma(r, po, pe);
-  const int n1 = n >> 1, n2 = n - n1;
-  const double s1 = __hiloint2double((1023 + n1) << 20, 0), s2 = __hiloint2double((1023 + n2) << 20, 0);
-  return x != x ? x : __dmul_rn(__dmul_rn(p, s1), s2);
-}
 #endif
 
 // ---------------------------------------------------------------------------
@@ -231,6 +197,18 @@ __device__ __forceinline__ Th thermo_mix(const MP& m, double T, const double* Yf
 
 __device__ __forceinline__ double cp_mix(const MP& m, double T, const double* Yf) {
   double cp = 0.0;
+#if JB_FAST
+  if (m.tcr_uniform) {  // one range for every species
+    if (T < m.Tcr[0]) {
+#pragma unroll
+      for (int k = 0; k < NS; ++k) cp = fma(poly5(m.cp_lo[k], T), Yf[k], cp);
+    } else {
+#pragma unroll
+      for (int k = 0; k < NS; ++k) cp = fma(poly5(m.cp_hi[k], T), Yf[k], cp);
+    }
+    return cp;
+  }
+#endif
 #pragma unroll
   for (int k = 0; k < NS; ++k) {
     const bool lo = T < m.Tcr[k];
@@ -1946,6 +1924,20 @@ __device__ __forceinline__ void lu_solve(double (&J)[NR][NR], double (&b)[NR], d
   }
 }
 
+// strict diagonal dominance by columns
+__device__ __forceinline__ bool col_dominant(const double (&J)[NR][NR]) {
+  bool cdd = true;
+#pragma unroll
+  for (int c = 0; c < NR; ++c) {
+    double off = 0.0;
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+      if (r != c) off += fabs(J[r][c]);
+    cdd = cdd && fabs(J[c][c]) > off;
+  }
+  return cdd;
+}
+
 // detailed_reaction (:183-193): dY = clip(drhoY/rho, -Y, 1-Y); S = rho dY
 __device__ __forceinline__ void chem_clip(const double* x, double rho, const double* Y8, double* S) {
 #if JB_FAST
@@ -1997,16 +1989,7 @@ __device__ __forceinline__ void chem_solve(const MP& m, double (&J)[NR][NR], con
   }
   double x[NR];
 #if JB_FAST
-  bool cdd = true;
-#pragma unroll
-  for (int c = 0; c < NR; ++c) {
-    double off = 0.0;
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-      if (r != c) off += fabs(J[r][c]);
-    cdd = cdd && fabs(J[c][c]) > off;
-  }
-  if (cdd) lu_solve<false>(J, b, x, st);
+  if (col_dominant(J)) lu_solve<false>(J, b, x, st);
   else lu_solve<true>(J, b, x, st);
 #else
   lu_solve<true>(J, b, x, st);
@@ -2120,7 +2103,7 @@ __device__ __forceinline__ double chem_gibbs(const MP& m, int k, double T, const
   return fma(-h, in.invT, s);
 }
 __device__ __forceinline__ void chem_equil(double gk, double& E, double& iE) {
-  E = exp_nb(gk);
+  E = exp(gk);
   iE = rcp_nr(fmin(fmax(E, 1e-300), 1e300));  // finite where E over- or underflows
 }
 
@@ -2162,17 +2145,13 @@ __device__ __forceinline__ void chem_cell_gen(const MP& m, double rho, const dou
 
 // The same for the 32 cells of a block of four warps: warp w takes two
 // species' equilibrium factors, every fourth reaction, and two columns of the
-// matrix of its lane's cell; then four neighbouring lanes share a cell's
-// solve, two rows each (chem_lu4).  A cell's chemistry is one long chain of
-// latencies in a single thread (17 us at any grid that leaves the chip idle).
-// Sums run in the order of chem_cell_gen and the pivots are its pivots, so
-// the two agree bitwise.  S is warp 0's, of its lane's cell.  sh: the block's
-// shared doubles (CHEM_SPLIT_SH); every thread of the block calls it, and a
-// block barrier separates it from the next use of sh.
-//
-// The matrix rows have a stride of 36 doubles: the four lanes of a cell read
-// rows 36 apart, which puts the 16 lanes of an access on 16 banks.
-constexpr int CS_LD = 36, CS_E = JB_GEN_ROWS * 32, CS_B = CS_E + 2 * NR * 32, CS_A = CS_B + NR * CS_LD;
+// matrix of its lane's cell, warp 0 the solve (S and st are warp 0's).  A
+// cell's chemistry is one long chain of latencies in a single thread (17 us at
+// any grid that leaves the chip idle).  Sums run in the order of
+// chem_cell_gen and the solve is chem_solve's, so the two agree bitwise.  sh:
+// the block's shared doubles (CHEM_SPLIT_SH); every thread of the block calls
+// it, and a block barrier separates it from the next use of sh.
+constexpr int CS_LD = 32, CS_E = JB_GEN_ROWS * 32, CS_B = CS_E + 2 * NR * 32, CS_A = CS_B + NR * CS_LD;
 constexpr int CHEM_SPLIT_SH = CS_A + NR * NR * CS_LD;
 template <int G>
 __device__ __forceinline__ void chem_split_part(const MP& m, const ChemIn& in, double idt, double* sh, int lane) {
@@ -2202,89 +2181,6 @@ __device__ __forceinline__ void chem_split_part(const MP& m, const ChemIn& in, d
   }
 }
 
-// Solve of cell threadIdx.x / 4's system by its four lanes, lane part holding
-// rows part and part + 4: Gaussian elimination with partial pivoting as
-// lu_solve<true> (first maximal |pivot| in the order its row exchanges would
-// give: pos is a row's place in that order), the rows staying where they are.
-// Every lane ends with the whole solution.
-__device__ __forceinline__ void chem_lu4(const double* sh, double (&x)[NR], unsigned& st) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, part = lane & 3, base = lane & ~3;
-  const double* c0 = sh + (threadIdx.x >> 2);
-  double a[2][NR], b[2], ipv[NR];
-  int pos[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int k = part + 4 * h;
-    pos[h] = k;
-    b[h] = c0[CS_B + k * CS_LD];
-#pragma unroll
-    for (int n = 0; n < NR; ++n) a[h][n] = c0[CS_A + (n * NR + k) * CS_LD];
-  }
-#pragma unroll
-  for (int c = 0; c < NR; ++c) {
-    // (key, pos, row) of the best candidate; the row now at place c wins
-    // against NaN, and a NaN elsewhere never wins, as its comparisons give
-    double key = -1.0;
-    int id = 0x7fffffff;  // pos * 8 + row
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      double v = fabs(a[h][c]);
-      if (v != v) v = pos[h] == c ? __longlong_as_double(0x7ff0000000000000LL) : -1.0;
-      if (pos[h] < c) v = -2.0;
-      const int i = pos[h] * 8 + part + 4 * h;
-      if (v > key || (v == key && i < id)) {
-        key = v;
-        id = i;
-      }
-    }
-#pragma unroll
-    for (int o = 1; o < 4; o <<= 1) {
-      const double k2 = __shfl_xor_sync(full, key, o);
-      const int i2 = __shfl_xor_sync(full, id, o);
-      if (k2 > key || (k2 == key && i2 < id)) {
-        key = k2;
-        id = i2;
-      }
-    }
-    const int prow = id & 7, ppos = id >> 3, src = base | (prow & 3);
-    const bool hi = prow >= 4;
-    double pr[NR];
-#pragma unroll
-    for (int j = 0; j < NR; ++j)
-      if (j >= c) pr[j] = __shfl_sync(full, hi ? a[1][j] : a[0][j], src);
-    const double pb = __shfl_sync(full, hi ? b[1] : b[0], src);
-    if (pr[c] == 0.0) st |= JB_ERR_SINGULAR;
-    ipv[c] = rcp_nr(pr[c]);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const bool is_pivot = part + 4 * h == prow;
-      if (is_pivot) pos[h] = c;
-      else if (pos[h] == c) pos[h] = ppos;
-      if (pos[h] > c) {
-        const double l = a[h][c] * ipv[c];
-#pragma unroll
-        for (int j = 0; j < NR; ++j)
-          if (j > c) a[h][j] = a[h][j] - l * pr[j];
-        b[h] = b[h] - l * pb;
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < NR; ++i) {
-    const int r = NR - 1 - i;
-    const bool h1 = pos[1] == r;
-    double s = h1 ? b[1] : b[0];
-#pragma unroll
-    for (int j = 0; j < NR; ++j)
-      if (j > r) s = s - (h1 ? a[1][j] : a[0][j]) * x[j];
-    s = s * ipv[r];
-    // the one lane of the four that holds the row at place r
-    const unsigned own = __ballot_sync(full, h1 || pos[0] == r) >> base & 15u;
-    x[r] = __shfl_sync(full, s, base | (__ffs(own) - 1));
-  }
-}
-
 __device__ __forceinline__ void chem_split(const MP& m, double rho, const double* Y8, double T, double dt, double* S,
                                            unsigned& st, double* sh) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -2307,20 +2203,16 @@ __device__ __forceinline__ void chem_split(const MP& m, double rho, const double
     default: chem_split_part<3>(m, in, idt, sh, lane); break;
   }
   __syncthreads();
-  double x[NR];
-  unsigned s1 = 0;
-  chem_lu4(sh, x, s1);
-  // each cell's solution over its right-hand side, which only its own four
-  // lanes (of one warp) read
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < NR; ++k)
-    if (k % 4 == (lane & 3)) sh[CS_B + k * CS_LD + (threadIdx.x >> 2)] = x[k];
-  st |= s1;
-  __syncthreads();
   if (wp == 0) {
+    double A[NR][NR], b[NR], x[NR];
 #pragma unroll
-    for (int k = 0; k < NR; ++k) x[k] = sh[CS_B + k * CS_LD + lane];
+    for (int k = 0; k < NR; ++k) {
+      b[k] = sh[CS_B + k * CS_LD + lane];
+#pragma unroll
+      for (int n = 0; n < NR; ++n) A[k][n] = sh[CS_A + (n * NR + k) * CS_LD + lane];
+    }
+    if (col_dominant(A)) lu_solve<false>(A, b, x, st);
+    else lu_solve<true>(A, b, x, st);
     chem_clip(x, rho, Y8, S);
   }
 }
@@ -2367,8 +2259,7 @@ __device__ __forceinline__ void chem_split_step(const MP& m, const Grid& g, cons
   const double ri = 1.0 / q[0];
 #pragma unroll
   for (int k = 0; k < NR; ++k) Y8[k] = __dmul_rn(q[nY + k], ri);
-  // (a singular system may be reported by any warp; padding lanes repeat a live cell)
-  chem_split(m, q[0], Y8, T, dt, S, st, sh);
+  chem_split(m, q[0], Y8, T, dt, S, st, sh);  // padding lanes repeat a live cell
   if (threadIdx.x < 32 && live) {
 #pragma unroll
     for (int f = 1; f < nY; ++f) q[f] = U[f * nc + c];
@@ -2461,7 +2352,7 @@ __global__ void __launch_bounds__(JB_CHEM_NT, JB_CHEM_MINB) k_chem(MP m, Grid g,
 // k_chem with four threads a cell (chem_split), 32 cells a block.
 template <int DIM, bool WRITE_S, bool CELL>
 #ifndef JB_CHEM_SPLIT_MINB
-#define JB_CHEM_SPLIT_MINB 4
+#define JB_CHEM_SPLIT_MINB 3
 #endif
 __global__ void __launch_bounds__(128, JB_CHEM_SPLIT_MINB) k_chem_split(MP m, Grid g, const double* __restrict__ U,
                                                      const double* __restrict__ aux, double* __restrict__ out,

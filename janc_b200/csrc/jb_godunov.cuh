@@ -18,6 +18,17 @@ __device__ __forceinline__ void face_thermo(const MP& m, double rho, double p, c
   fill_Y(Y8, Yf);
   const double R = get_R(m, Yf);
   const double T = p / (R * rho);
+#if JB_FAST
+  if (m.tcr_uniform) {
+    // the mixture's enthalpy polynomial in the range T lies in: 70 operations
+    // for the species sums' 200 (both ranges)
+    double H[6], cp, dcp;
+    mix_h(m, Yf, T < m.Tcr[0], H);
+    poly6_d2(H, T, h, cp, dcp);
+    gamma = cp / (cp - R);
+    return;
+  }
+#endif
   const Th t = thermo_mix(m, T, Yf);
   h = t.h;
   gamma = t.cp / (t.cp - R);
@@ -33,8 +44,13 @@ __device__ __forceinline__ void hllc_flux(const MP& m, const double* wL, const d
   double gL, hL, gR, hR;
   face_thermo(m, rL, pL, wL + IY, gL, hL);
   face_thermo(m, rR, pR, wR + IY, gR, hR);
+#if JB_FAST
+  const double iL = 1.0 / rL, iR = 1.0 / rR;
+  const double aL = sqrt(gL * pL * iL), aR = sqrt(gR * pR * iR);
+#else
   const double aL = sqrt(gL * pL / rL);
   const double aR = sqrt(gR * pR / rR);
+#endif
   const double unL = wL[N], unR = wR[N];
   const double kL = DIM == 2 ? wL[1] * wL[1] + wL[2] * wL[2] : wL[1] * wL[1];
   const double kR = DIM == 2 ? wR[1] * wR[1] + wR[2] * wR[2] : wR[1] * wR[1];
@@ -46,8 +62,13 @@ __device__ __forceinline__ void hllc_flux(const MP& m, const double* wL, const d
   const bool c1 = sL >= 0.0, c2 = sL <= 0.0 && sM >= 0.0, c3 = sM <= 0.0 && sR >= 0.0;
   // the star-state factor and energy of each side
   const double fL = rL * (sL - unL) / (sL - sM), fR = rR * (sR - unR) / (sR - sM);
+#if JB_FAST
+  const double eL = EL * iL + (sM - unL) * (sM + pL / (rL * (sL - unL)));
+  const double eR = ER * iR + (sM - unR) * (sM + pR / (rR * (sR - unR)));
+#else
   const double eL = EL / rL + (sM - unL) * (sM + pL / (rL * (sL - unL)));
   const double eR = ER / rR + (sM - unR) * (sM + pR / (rR * (sR - unR)));
+#endif
   // component c: conserved U, star U_M, physical flux of each side
   auto pick = [&](double UL, double UML, double FL_, double UR, double UMR, double FR_) {
     const double FLM = FL_ + sL * (UML - UL);
@@ -146,6 +167,16 @@ __device__ __forceinline__ void cons_to_w(const MP& m, const double* q, double T
   constexpr int nY = DIM == 1 ? 3 : 4;
   const double rho = q[0];
   w[0] = rho;
+#if JB_FAST
+  const double ri = 1.0 / rho;  // one reciprocal for the eleven quotients
+  double rN;
+  w[1] = q[1] * ri;
+  if (DIM == 2) w[2] = q[2] * ri;
+  w[DIM + 1] = prim_sums(m, q + nY, rho, rN) * T;
+#pragma unroll
+  for (int k = 0; k < NR; ++k) w[DIM + 2 + k] = q[nY + k] * ri;
+  return;
+#endif
   w[1] = q[1] / rho;
   if (DIM == 2) w[2] = q[2] / rho;
   double Y8[NR], Yf[NS];

@@ -206,6 +206,8 @@ __device__ __forceinline__ void pack_load(const MP& m, const Grid& g, const doub
 }
 
 constexpr int SX_NT = 128;
+// blocks per SM: 72 registers for float32 pairs, 96 for float64 (80 at 6: the
+// channel 715 against 710 us for two steps)
 #ifndef JB_SX_MINB
 #define JB_SX_MINB 7
 #endif
@@ -323,8 +325,11 @@ __device__ __forceinline__ void yr_run(const V* hp, const V* hm, V* f, int k0) {
   }
 }
 
+// float32 pairs at 7 blocks per SM (72 registers, no spills): annulus 1600 x
+// 1000 1236 us a step, 1292 at 8 (64 registers), 1258 at 6; channel 1024 x 256
+// 455, 461, 461 us for two.  float64 at 4 (128 registers): 710 us, 717 at 5.
 #ifndef JB_YR_MINB
-#define JB_YR_MINB 8
+#define JB_YR_MINB 7
 #endif
 #ifndef JB_YRD_MINB
 #define JB_YRD_MINB 4

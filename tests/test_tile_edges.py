@@ -140,3 +140,38 @@ def test_line_run_is_the_separate_launches(nx, bc, prec):
         for x, y in zip(a, r):
             assert torch.equal(x, y) and bool(torch.isfinite(x).all())
     assert one.status() == sep.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny", [(4, 4), (4, 8), (5, 7), (11, 3 * 32), (111, 128), (111, 129)])
+def test_chemistry_forms_match_the_strict_build(nx, ny):
+    """reaction_source_terms with four threads a cell (up to 14208 cells:
+    whole and ragged 32-cell blocks, the largest of its range) and with one (the
+    first size above), against the strict build's table-driven kernel; hot
+    and cold cells, so both eliminations.  Two float64 evaluations of the rates,
+    whose differences of near-equal rates amplify 1e-16 by up to 1e4."""
+    s0, s1 = _pair(2, nx, ny, "walls", "fp64", False, 1e-4)
+    U, aux = _state(s0, (nx, ny))
+    a, b = s0.reaction_source_terms(U, aux, 3e-9), s1.reaction_source_terms(U, aux, 3e-9)
+    for f in range(4, 12):
+        assert float((a[f] - b[f]).abs().sum()) <= 1e-12 * float(a[f].abs().sum()), f
+    assert s0.status() == s1.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bx,by", [(1, 1), (1, 9), (5, 33), (20, 20), (21, 20), (24, 24), (40, 17)])
+def test_block_stage_matches_the_strict_build(bx, by):
+    """Stages of blocks whose interiors are one tile and several, one cell wide
+    and ragged.  Each stage combines the state with dt L(U), both builds'
+    fluxes within 1e-13 of the size of their terms: 1e-12 of each field."""
+    from janc_b200.solver import Solver
+    d, X, Y = 1e-4, bx + 6, by + 6
+    s0 = Solver(2, 32, 32, d, d, precision="fp64_strict")
+    s1 = Solver(2, 32, 32, d, d, precision="fp64")
+    U, aux = _state(s0, (2 * X, Y))
+    G = torch.cat([U, aux]).reshape(14, 2, X, Y).transpose(0, 1).contiguous()
+    for stage in (1, 2, 3):
+        a, b = (s.amr_stage(G, G if stage > 1 else None, stage, d, d, 1e-9) for s in (s0, s1))
+        for f in range(14):
+            assert float((a[:, f] - b[:, f]).abs().max()) <= 1e-12 * float(a[:, f].abs().max()), (stage, f)
+    assert s0.status() == s1.status() == 0

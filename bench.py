@@ -80,11 +80,11 @@ BYTES_STEP_PER_CELL = 864 + 224  # fused-step minimum + separate chemistry pass 
 BYTES_FLUX_STAGE_PER_CELL = 288  # one RK stage of the fused minimum: (224 + 320 + 320) / 3
 # DRAM bytes per cell measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum,
 # each launch cold) on the 1024x256 channel, mixed precision, with this tree's
-# kernels: one RK stage 2/3 (k_sweep_x 27.35 + 0.00 MB, k_flux_y_rk 67.43 +
-# 5.98 MB) and one chemistry launch (27.38 + 3.46 MB); the capture and its
+# kernels: one RK stage 2/3 (k_sweep_x 27.35 + 0.00 MB, k_flux_y 67.19 +
+# 0.77 MB) and one chemistry launch (27.37 + 0.73 MB); the capture and its
 # command are in profiles/launches_channel1024x256_mixed.md.  Per cell-step of
 # the persistent ensemble kernel: profiles/k_ensemble_64tubes.md.
-TRAFFIC_PER_CELL = {"flux": 384.3, "chem": 117.6}
+TRAFFIC_PER_CELL = {"flux": 363.6, "chem": 107.2}
 TRAFFIC_SOURCE = "profiles/launches_channel1024x256_mixed.md"
 TRAFFIC_ENS_PER_CELL_STEP = 764.0
 
@@ -611,8 +611,9 @@ def run_ours(args):
                          "chem": "k_chem (point-implicit chemistry + final Halley)",
                          "flux": ("k_god2d (reconstruction on primitives + Riemann solver + RK stage + Halley)"
                                   if args.flux not in ("LF", "SW") else
-                                  "flux stage: k_sweep_x + k_flux_y_rk (LF + WENO5 + RK stage + Halley)"
-                                  if args.precision == "mixed" and args.flux == "LF" and args.recon == "WENO5_JS"
+                                  "flux stage: k_sweep_x + k_flux_y (LF + WENO5 + RK stage + Halley)"
+                                  if args.precision in ("mixed", "fp64") and args.flux == "LF" and
+                                  args.recon == "WENO5_JS"
                                   else f"k_flux2d ({args.flux} splitting + reconstruction + RK stage + Halley)")}[dom],
                      "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                      "traffic": (TRAFFIC_PER_CELL[dom] * ncell if args.workload == "channel" and

@@ -40,7 +40,7 @@ struct jb_handle {
   // adjoint support
   double base_A[JB_NREAC_MAX];  // pre-exponential factors as created (jb_set_log_A_offset)
   int probe[4];                 // x0, y0, wx, wy of the pressure probe (wx*wy = 0: none)
-  void* fwork;                  // 2D flux scratch (primitives, x flux differences: sweep_work)
+  void* fwork;                  // 2D sweeps' primitives (sweep_work)
   jb_transport tr;              // laminar transport model (viscous fluxes when grid.visc is set)
   double* vbuf;                 // viscous node planes and node fluxes
   double* vcell;                // viscous rhs of the current stage state (nv x ncell)
@@ -176,25 +176,23 @@ int jb_create(const jb_mech_params* mech, int dim, int nx, int ny, double dx, do
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&h->W[i], bytes_W);
   for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&h->auxw[i], bytes_aux);
-  if (e == cudaSuccess) e = cudaMalloc(&h->cand, bytes_cand);
+  // 2D sweeps (jb_sweep.cuh): the primitives of the stage state, float64 in
+  // fp64; in mixed float32, and those of the state being written (two buffers
+  // used in turn); behind the iterates in their allocation
+  const size_t bytes_fwork = dim != 2 || precision == JB_PREC_STRICT ? 0 : 24 * nc;
+  if (e == cudaSuccess) e = cudaMalloc(&h->cand, bytes_cand + bytes_fwork);
+  if (bytes_fwork) h->fwork = h->cand + JB_NCAND * nc;
   if (e == cudaSuccess) e = cudaMalloc(&h->strips, bytes_strip);
   const size_t bytes_slots = 3 * sizeof(jb_slots) + 16 * sizeof(unsigned);
   if (e == cudaSuccess) e = cudaMalloc(&h->slots, bytes_slots);
   if (e == cudaSuccess) e = cudaMemset(h->strips, 0, bytes_strip);
   if (e == cudaSuccess) e = cudaMemset(h->slots, 0, bytes_slots);
-  for (int i = 1; i < 3 && e == cudaSuccess; ++i) {  // as a run's last block leaves them
+  for (int i = 1; i < 3 && dim == 1 && e == cudaSuccess; ++i) {  // as a run's last block leaves them
     jb_slots clear;
     std::memset(&clear, 0, sizeof(clear));
     clear.dtmin_next = 0x7ff0000000000000ull;
     e = cudaMemcpy(h->slots + i, &clear, sizeof(clear), cudaMemcpyHostToDevice);
   }
-  // 2D sweeps (jb_sweep.cuh): the primitives of the stage state (mixed: and
-  // of the state being written, two buffers used in turn), then the x flux
-  // differences; float32 in mixed, float64 in fp64
-  const size_t bytes_fwork = dim != 2 || precision == JB_PREC_STRICT ? 0
-                             : precision == JB_PREC_MIXED            ? sizeof(float) * 18 * nc
-                                                                     : sizeof(double) * 15 * nc;
-  if (e == cudaSuccess && bytes_fwork) e = cudaMalloc(&h->fwork, bytes_fwork);
   if (e != cudaSuccess) {
     jb_destroy(h);
     return JB_ERR_CUDA;
@@ -215,7 +213,6 @@ int jb_destroy(jb_handle* h) {
   if (h->cand) cudaFree(h->cand);
   if (h->strips) cudaFree(h->strips);
   if (h->slots) cudaFree(h->slots);
-  if (h->fwork) cudaFree(h->fwork);
   if (h->vbuf) cudaFree(h->vbuf);
   if (h->adj_ws) cudaFree(h->adj_ws);
   if (h->adj_mult) cudaFree(h->adj_mult);
@@ -301,21 +298,20 @@ int jb_set_ghost_cells(jb_handle* h, double* sendx, double* halox, double* sendy
   return JB_OK;
 }
 
-// Parts of the handle's 2D sweep scratch: the stage state's primitives, the
-// buffer of the next state's (mixed) and the x flux differences; null where
-// the handle's flux options take the tile kernels.
+// Parts of the handle's 2D sweep scratch: the stage state's primitives and
+// the buffer of the next state's (mixed); null where the handle's flux
+// options take the tile kernels.
 struct sweep_work {
-  void *prims, *prims_next, *dfx;
+  void *prims, *prims_next;
 };
 static sweep_work sweep_parts(const jb_handle* h) {
   const jb_grid& g = h->grid;
-  if (!h->fwork || g.scheme != JB_FLUX_LF || g.recon != JB_RECON_WENO5) return {nullptr, nullptr, nullptr};
+  if (!h->fwork || g.scheme != JB_FLUX_LF || g.recon != JB_RECON_WENO5) return {nullptr, nullptr};
   if (h->precision == JB_PREC_MIXED) {
     float* b = static_cast<float*>(h->fwork);
-    return {b, b + 3 * g.ncell, b + 6 * g.ncell};
+    return {b, b + 3 * g.ncell};
   }
-  double* b = static_cast<double*>(h->fwork);
-  return {b, b, b + 3 * g.ncell};
+  return {h->fwork, h->fwork};
 }
 
 int jb_flux_func(jb_handle* h, const double* U, const double* aux, double dt, double* rhs,
@@ -333,7 +329,7 @@ int jb_flux_func(jb_handle* h, const double* U, const double* aux, double dt, do
   if (h->grid.visc)
     JB_TRY(o.visc(h->dim, h->mech, h->grid, h->tr, U, aux, h->strips, h->vbuf, h->vcell, st), "viscous");
   JB_TRY(o.flux(h->dim, 0, h->mech, h->grid, U, aux, nullptr, rhs, h->strips, h->slots, 3, jb_fin_cand(nullptr, -1),
-                sw.prims, sw.dfx, dt, st),
+                sw.prims, dt, st),
          "flux");
   return JB_OK;
 }
@@ -432,7 +428,6 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
   const sweep_work sw = sweep_parts(h);
   void* pin = sw.prims;
   float* pout = static_cast<float*>(pc ? sw.prims_next : nullptr);
-  void* dfx = sw.dfx;
   auto swap_prims = [&]() {
     float* t = static_cast<float*>(pin);
     pin = pout;
@@ -467,12 +462,12 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
       JB_TIMED(JB_KCAT_FLUX, o.visc(d, m, g, h->tr, Un, an, h->strips, h->vbuf, h->vcell, st), "viscous");
     if (pc) {
       JB_TIMED(JB_KCAT_FLUX, o.flux(d, 1, m, g, Un, an, Un, W1, h->strips, h->slots, 0,
-                                    jb_fin_cell(A1, pout, 1, 0), pin, dfx, 0.0, st), "stage1");
+                                    jb_fin_cell(A1, pout, 1, 0), pin, 0.0, st), "stage1");
       swap_prims();
       JB_TIMED(JB_KCAT_SELECT, o.strips(d, m, g, W1, A1, h->strips, h->slots, 1, st), "strips1");
     } else {
       JB_TIMED(JB_KCAT_FLUX, o.flux(d, 1, m, g, Un, an, Un, W1, h->strips, h->slots, 0, jb_fin_cand(h->cand, 0),
-                                    pin, dfx, 0.0, st), "stage1");
+                                    pin, 0.0, st), "stage1");
       JB_TIMED(JB_KCAT_SELECT, o.select(d, true, true, false, m, g, W1, nullptr, h->cand, A1, h->strips,
                       h->slots, 0, 1, pin, st),
              "select1");
@@ -483,12 +478,12 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
       JB_TIMED(JB_KCAT_FLUX, o.visc(d, m, g, h->tr, W1, A1, h->strips, h->vbuf, h->vcell, st), "viscous");
     if (pc) {
       JB_TIMED(JB_KCAT_FLUX, o.flux(d, 2, m, g, W1, A1, Un, W2, h->strips, h->slots, 1,
-                                    jb_fin_cell(A2, pout, 2, 0), pin, dfx, 0.0, st), "stage2");
+                                    jb_fin_cell(A2, pout, 2, 0), pin, 0.0, st), "stage2");
       swap_prims();
       JB_TIMED(JB_KCAT_SELECT, o.strips(d, m, g, W2, A2, h->strips, h->slots, 2, st), "strips2");
     } else {
       JB_TIMED(JB_KCAT_FLUX, o.flux(d, 2, m, g, W1, A1, Un, W2, h->strips, h->slots, 1, jb_fin_cand(h->cand, 1),
-                                    pin, dfx, 0.0, st), "stage2");
+                                    pin, 0.0, st), "stage2");
       JB_TIMED(JB_KCAT_SELECT, o.select(d, true, true, false, m, g, W2, nullptr, h->cand, A2, h->strips,
                       h->slots, 1, 2, pin, st),
              "select2");
@@ -501,7 +496,7 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
       // without the chemistry this is the step's result: its alpha, CFL
       // minimum and primitives serve the next step
       const jb_fin f3 = chemistry ? jb_fin_cell(A3, nullptr, -1, 0) : jb_fin_cell(A3, pout, 3, use_cfl);
-      JB_TIMED(JB_KCAT_FLUX, o.flux(d, 3, m, g, W2, A2, Un, W3, h->strips, h->slots, 2, f3, pin, dfx, 0.0, st),
+      JB_TIMED(JB_KCAT_FLUX, o.flux(d, 3, m, g, W2, A2, Un, W3, h->strips, h->slots, 2, f3, pin, 0.0, st),
                "stage3");
       if (!chemistry) {
         swap_prims();
@@ -510,7 +505,7 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
       }
     } else {
       JB_TIMED(JB_KCAT_FLUX, o.flux(d, 3, m, g, W2, A2, Un, W3, h->strips, h->slots, 2, jb_fin_cand(h->cand, 2),
-                                    pin, dfx, 0.0, st), "stage3");
+                                    pin, 0.0, st), "stage3");
       if (!chemistry) {
         JB_TIMED(JB_KCAT_SELECT, o.select(d, true, true, use_cfl, m, g, W3, nullptr, h->cand, A3,
                                           h->strips, h->slots, 2, 3, pin, st),

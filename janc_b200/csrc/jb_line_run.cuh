@@ -2,8 +2,9 @@
 // cooperative launch (included by jb_variant.inc in the LINE part of the fast
 // variants).  A short line's step is a chain of short latencies; as separate
 // launches (8 a step in mixed, 9 in fp64, plus the outlet strips) the host's
-// 4-6 us per launch and the launch gaps outweigh it: 500 cells took 67 us a
-// step, 12000 cells with an outlet 68 us, against 29 us and 26 us here.
+// 4-6 us per launch and the launch gaps outweigh it: 500 cells in fp64 took
+// 69 us a step, 12000 cells in mixed with an outlet 68 us, against 52 us and
+// 36 us here.
 //
 // Each CTA owns one tile of S cells through every phase, so the passes that
 // only touch a cell's own state follow each other without a barrier; the

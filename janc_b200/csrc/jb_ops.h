@@ -45,13 +45,12 @@ struct Ops {
   bool per_cell;
   // STAGE 0 writes dt * flux; STAGE 1..3 writes the RK stage and finishes
   // its temperature solve as fin says (jb_fin.h).  aidx: the alpha slot the
-  // stage reads.  prims: u, v, p of the stage state [3][ncell] and work:
-  // scratch of the x flux differences [12][ncell] (2D LF / WENO5-JS; float64
-  // in fp64, float32 in mixed), or null.
+  // stage reads.  prims: u, v, p of the stage state [3][ncell] (2D LF /
+  // WENO5-JS; float64 in fp64, float32 in mixed), or null.
   cudaError_t (*flux)(int dim, int stage, const jb_mech_params& m, const jb_grid& g,
                       const double* Uk, const double* auxk, const double* Un, double* out,
                       const double* strips, jb_slots* slots, int aidx, const jb_fin& fin,
-                      const void* prims, void* work, double dt, cudaStream_t st);
+                      const void* prims, double dt, cudaStream_t st);
   // work: where the pass writes the u, v, p of its state when it computes
   // alpha (as prims of flux), or null
   cudaError_t (*select)(int dim, bool select, bool alpha, bool cfl, const jb_mech_params& m,

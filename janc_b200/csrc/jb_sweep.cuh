@@ -14,8 +14,10 @@
 // paired float32 instructions FFMA2 / FADD2 / FMUL2, 6 packs).  The RK
 // combination and the temperature solve are float64 in both.  The stage
 // state's u, v, p come from the kernel that finished that state
-// (prims[3][ncell], in the pack's scalar type); the x differences go through
-// dfx[packs][ncell].
+// (prims[3][ncell], in the pack's scalar type).  The x differences wait in the
+// stage's own output: pack j of a cell in the 8 bytes that field W j of that
+// cell takes, which only the thread that combines the cell reads, before it
+// writes them (k_flux_y reads them through out, which is neither Uk nor Un).
 typedef float2 f2;
 template <class V> struct VT;
 template <> struct VT<double> {
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(SX_NT, VT<V>::W == 2 ? JB_SX_MINB : JB_SXD_MIN
     }
   };
   fetch(a0 + 2);
-  V* out = dfx + (long long)j * nc + y;
+  V* out = dfx + (long long)W * j * nc + y;
   V Fprev = vset<V>((R)0);
 #pragma unroll 4  // the windows shift by renaming inside the unrolled bodies
   for (int fa = a0; fa <= a1; ++fa) {
@@ -340,8 +342,8 @@ template <int STAGE, class V, bool VISC>
 __global__ void __launch_bounds__(YR_S, VT<V>::W == 2 ? JB_YR_MINB : JB_YRD_MINB)
     k_flux_y(MP m, Grid g, const double* __restrict__ Uk, const double* __restrict__ auxk,
              const double* __restrict__ Un, const typename VT<V>::S* __restrict__ prims,
-             const double* __restrict__ strips, const V* __restrict__ dfx, double* __restrict__ out, Slots* slots,
-             int aidx, jb_fin fin, double dt_arg, int nsy) {
+             const double* __restrict__ strips, double* __restrict__ out, Slots* slots, int aidx, jb_fin fin,
+             double dt_arg, int nsy) {
   typedef typename VT<V>::S R;
   constexpr int W = VT<V>::W, NP = VT<V>::NP;
   extern __shared__ __align__(128) unsigned char smraw[];
@@ -401,7 +403,7 @@ __global__ void __launch_bounds__(YR_S, VT<V>::W == 2 ? JB_YR_MINB : JB_YRD_MINB
     double q[12];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
-      const V dF = dfx[i * nc + cell];
+      const V dF = reinterpret_cast<const V*>(out)[(long long)W * i * nc + cell];  // own planes, stored below
       const V dG = vsub(sF[i * YR_F + yr_at(t + 1)], sF[i * YR_F + yr_at(t)]);
 #pragma unroll
       for (int h = 0; h < W; ++h) {

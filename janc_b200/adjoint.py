@@ -61,7 +61,8 @@ class Trajectory:
             _native.check(L.jb_set_log_A_offset(self.s._h, None), self.s._h, "jb_set_log_A_offset")
             self._lnA = None
             return
-        off = [float(v) for v in torch.as_tensor(offset).detach().cpu().reshape(-1)]
+        # float64 also for a list, of which torch makes float32 by itself
+        off = torch.as_tensor(offset, dtype=torch.float64).detach().cpu().reshape(-1).tolist()
         arr = (ctypes.c_double * len(off))(*off)
         _native.check(L.jb_set_log_A_offset(self.s._h, arr), self.s._h, "jb_set_log_A_offset")
         self._lnA = off

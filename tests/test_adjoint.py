@@ -151,6 +151,35 @@ def test_twin_gradient_matches_finite_differences(omech, bc):
         assert abs(fd - ad) <= 1e-5 * abs(fd)
 
 
+def test_rate_offsets_reach_the_library_unrounded():
+    """The forward and the backward pass hand the library the same ln A
+    offsets, bit for bit, and so does a plain list of floats."""
+    import types
+    from janc_b200.adjoint import Trajectory, probe_trajectory
+    seen = []
+
+    class Lib:
+        def jb_set_log_A_offset(self, h, arr):
+            seen.append(None if arr is None else list(arr))
+            return 0
+
+    off = np.random.default_rng(3).uniform(-0.7, 0.7, 19)
+    assert not np.any(off == off.astype(np.float32))
+    one = torch.ones(1, dtype=torch.float64)
+    traj = Trajectory.__new__(Trajectory)
+    traj._lnA = None
+    traj.s = types.SimpleNamespace(_lib=Lib(), _h=None, state_from_PTY=lambda P, T, Y: (T, T))
+    traj.run = lambda U, aux, n: (U, aux, one.clone(), one.clone(), [(U, aux)])
+    traj.backward = lambda *a: (one, one, torch.zeros(19, dtype=torch.float64))
+    traj.state_vjp = lambda P, T, Y, Ub, Ab: torch.zeros_like(T)
+    T = torch.full((1, 4), 300.0, dtype=torch.float64, requires_grad=True)
+    dts, pps = probe_trajectory(traj, T.detach(), T, T.detach(), torch.tensor(off, requires_grad=True), 1)
+    (dts * pps).sum().backward()
+    traj.set_log_A_offset(off.tolist())
+    traj.set_log_A_offset(off)
+    assert seen == [off.tolist()] * 4
+
+
 # --------------------------------------------------------------------- GPU
 def _native(om, nx, ny, bc, P, T, Y, nsteps, cfl, probe, K, lnA=None):
     from janc_b200.adjoint import Trajectory, probe_trajectory
@@ -168,10 +197,10 @@ def _native(om, nx, ny, bc, P, T, Y, nsteps, cfl, probe, K, lnA=None):
     return float(loss), Tg.grad.cpu().numpy(), lg.grad.cpu().numpy(), traj
 
 
-def _twin(om, nx, ny, bc, P, T, Y, nsteps, cfl, probe):
+def _twin(om, nx, ny, bc, P, T, Y, nsteps, cfl, probe, lnA=None):
     tw = tt.Twin(om, 1.953125e-4, 1.953125e-4, bc, cfl, Pb=PB)
     Tt = torch.tensor(T, requires_grad=True)
-    lnA = torch.zeros(19, dtype=torch.float64, requires_grad=True)
+    lnA = torch.tensor(np.zeros(19) if lnA is None else lnA, requires_grad=True)
     L, _, _ = tt.trajectory_loss(tw, torch.tensor(P), Tt, torch.tensor(Y), nsteps, probe, lnA)
     L.backward()
     return float(L), Tt.grad.numpy(), lnA.grad.numpy()
@@ -196,6 +225,28 @@ def test_adjoint_matches_autograd_twin(omech, bc, noisy):
     assert abs(L - Lr) <= 1e-12 * abs(Lr)
     assert _rel(gT, gTr) < 1e-8
     assert _rel(gA, gAr) < 1e-8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nsteps,K", [(1, 1), (2, 1), (4, 3)])
+def test_adjoint_with_rate_offsets_matches_twin(omech, nsteps, K):
+    """Offsets that float32 does not hold, on a field with 1 % of noise
+    everywhere: one ulp of P, T or Y changes the twin's own gradients there by
+    at most 2e-13, a step's some hundred roundings by far less than 1e-10.
+    (Offsets rounded to float32 change the ln A gradient by 1e-8.)"""
+    nx, ny = 24, 16
+    rng = np.random.default_rng(0)
+    P, T, Y = _fields(omech, nx, ny, 3, noisy=False)
+    P *= 1 + 0.01 * rng.uniform(-1, 1, P.shape)
+    T *= 1 + 0.01 * rng.uniform(-1, 1, T.shape)
+    off = np.random.default_rng(3).uniform(-0.7, 0.7, 19)
+    lnA = torch.tensor(off, device="cuda", requires_grad=True)
+    probe = (12, 6, 4, 4)
+    L, gT, gA, _ = _native(omech, nx, ny, BC_SLIP, P, T, Y, nsteps, 0.1, probe, K, lnA)
+    Lr, gTr, gAr = _twin(omech, nx, ny, BC_SLIP, P, T, Y, nsteps, 0.1, probe, off)
+    assert abs(L - Lr) <= 1e-12 * abs(Lr)
+    assert _rel(gT, gTr) < 1e-10
+    assert _rel(gA, gAr) < 1e-10
 
 
 @pytest.mark.gpu

@@ -73,9 +73,19 @@ int jb_reaction_source_terms(jb_handle* h, const double* U, const double* aux, d
  * TVD_RK3.py:5-12, chemistry, temperature solve).  cfl > 0: each step's dt is
  * cfl * min(...) as Simulator.advance_func (set_simulator.py:420-447);
  * otherwise dt_fixed.  dt_hist (device, nsteps doubles, may be NULL) receives
- * each step's dt.  U/aux are not modified; U_out/aux_out receive the result. */
+ * each step's dt.  U/aux are not modified; U_out/aux_out receive the result.
+ * Short 1D LF / WENO5-JS lines (fp64, mixed) run all steps in one launch whose
+ * blocks wait for one another, each wait at most 2 s (a GPU shared by
+ * time slices may take longer); such a run is abandoned with U_out, aux_out
+ * and dt_hist filled with NaN and JB_ERR_TIMEOUT in jb_status. */
 int jb_advance(jb_handle* h, const double* U, const double* aux, double* U_out, double* aux_out,
                double dt_fixed, double cfl, int nsteps, double* dt_hist, void* stream);
+
+/* Test hook for that path: the handle's next 1D run waits at most
+ * wait_limit_ms (at most 1000) and for `missing` blocks more than are
+ * launched, so that with missing > 0 its first wait runs out and every block
+ * returns. */
+int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing);
 
 /* One SSP-RK3 step of the flux alone, followed by update_aux after each
  * stage: time_step_dict['TVD_RK3'](U, aux, dx, dy, dt, theta, flux_func,
@@ -101,7 +111,8 @@ int jb_get_thermo(jb_handle* h, long long n, const double* T, const double* Y, d
                   double* gamma, double* hh, double* R, double* dcp, void* stream);
 
 /* Synchronise `stream` and return the device status bits accumulated since
- * the last call (non-finite state, singular chemistry matrix), then clear. */
+ * the last call (non-finite state, singular chemistry matrix, a device wait
+ * that gave up), then clear. */
 int jb_status(jb_handle* h, unsigned* status, void* stream);
 
 /* Bytes of device workspace the handle holds. */

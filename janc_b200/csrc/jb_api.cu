@@ -29,6 +29,8 @@ struct jb_handle {
   double* cand;        // Halley iterates [6][ncell]
   double* strips;      // ghost strips [4][nv+2][lstrip]
   jb_slots* slots;     // the step's slots, then two more sets and 16 barrier words (1D runs)
+  double lr_wait_ms;   // of the next 1D run (jb_selftest_line_run)
+  unsigned lr_missing;
   long long ws_bytes;
   // optional per-kernel timing of jb_advance (jb_set_kernel_timing)
   int timing;
@@ -417,7 +419,9 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
     const jb::jb_line_io io = {U,          aux,      U_out,   aux_out,  h->W[0],
                                h->W[1],    h->auxw[0], h->auxw[1], h->cand, h->strips,
                                h->slots,   reinterpret_cast<unsigned*>(h->slots + 3), dt_fixed, use_cfl ? cfl : 0.0,
-                               nsteps,     dt_hist};
+                               nsteps,     dt_hist,  h->lr_wait_ms, h->lr_missing};
+    h->lr_wait_ms = 0.0;
+    h->lr_missing = 0;
     cudaError_t e = cudaSuccess;
     if (o.line_run(m, g, io, st, e)) return check_cuda(h, e, "line run");
   }
@@ -552,6 +556,15 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
 int jb_advance(jb_handle* h, const double* U, const double* aux, double* U_out, double* aux_out,
                double dt_fixed, double cfl, int nsteps, double* dt_hist, void* stream) {
   return advance_impl(h, U, aux, U_out, aux_out, dt_fixed, cfl, nsteps, dt_hist, stream, true);
+}
+
+int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing) {
+  if (!h) return JB_ERR_ARG;
+  if (!(wait_limit_ms > 0.0) || wait_limit_ms > 1000.0) return set_err(h, JB_ERR_ARG, "wait limit must be in (0, 1000] ms");
+  if (missing < 0) return set_err(h, JB_ERR_ARG, "missing must be >= 0");
+  h->lr_wait_ms = wait_limit_ms;
+  h->lr_missing = (unsigned)missing;
+  return JB_OK;
 }
 
 int jb_rk3(jb_handle* h, const double* U, const double* aux, double* U_out, double* aux_out,

@@ -20,8 +20,9 @@
 // still reading another.  The slot sets alternate between even and odd steps.
 //
 // Every wait is bounded (2 s and 2^26 polls), after which the run is
-// abandoned with JB_ERR_TIMEOUT; the last CTA to leave clears the barrier
-// words and slot sets for the next launch.
+// abandoned: the last CTA to leave fills the outputs and the time steps with
+// NaN and sets JB_ERR_TIMEOUT.  It clears the barrier words and slot sets for
+// the next launch in any case.
 struct LineRun {
   const double *U, *aux;
   double *U_out, *aux_out, *W0, *W1, *A0, *A1, *cand, *strips;
@@ -30,6 +31,8 @@ struct LineRun {
   double dt_fixed, cfl;
   int nsteps;
   double* dt_hist;
+  unsigned arrivals;             // CTAs that a barrier waits for
+  unsigned long long limit_ns;   // and how long
 };
 
 namespace {
@@ -45,13 +48,14 @@ __device__ __forceinline__ unsigned lr_acquire(const unsigned* p) {
 }
 
 // Barrier of all CTAs (every thread calls it); false when the run is abandoned.
-__device__ __forceinline__ bool lr_sync(unsigned* bar, unsigned& target) {
+__device__ __forceinline__ bool lr_sync(const LineRun& a, unsigned& target) {
   __shared__ int s_go;
   __syncthreads();
-  if (gridDim.x == 1) return true;
+  if (a.arrivals == 1) return true;
+  unsigned* bar = a.bar;
   if (threadIdx.x == 0) {
     int go = 1;
-    target += gridDim.x;
+    target += a.arrivals;
     __threadfence();
     atomicAdd(&bar[0], 1u);
     unsigned long long t0 = 0;
@@ -61,7 +65,7 @@ __device__ __forceinline__ bool lr_sync(unsigned* bar, unsigned& target) {
         unsigned long long now;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
         if (it == 0) t0 = now;
-        if (it >= LR_SPIN_MAX || now - t0 > LR_LIMIT_NS) {
+        if (it >= LR_SPIN_MAX || now - t0 > a.limit_ns) {
           atomicExch(&bar[2], 1u);
           go = 0;
           break;
@@ -122,7 +126,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
       select_cell<1, false, true, true>(m, g, a.U, a.aux, nullptr, nullptr, a.strips, &a.sets[1], 0u, c, amx, amy,
                                         dtm, st);
     block_reduce_store(amx, amy, dtm, st << 16, &a.sets[1], 3, true, use_cfl, -1);
-    go = lr_sync(a.bar, target);
+    go = lr_sync(a, target);
   }
 #pragma unroll 1
   for (int step = 0; go && step < a.nsteps; ++step) {
@@ -143,7 +147,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
                                        amx, dtm, cur);
       lr_strips(m, g, x0, nin, a.W0, a.A0, a.strips + 1, amx);
       finish_reduce(f1, amx, 0.0, dtm, bits, cur);
-      if (!(go = lr_sync(a.bar, target))) break;
+      if (!(go = lr_sync(a, target))) break;
       if (blockIdx.x == 0 && tid == 0) lr_clear(prv);  // every CTA has read it
       // stage 2: U2 = 3/4 U + 1/4 (U1 + L(U1))
       amx = 0.0;
@@ -152,7 +156,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
                                        smraw, amx, dtm, cur);
       lr_strips(m, g, x0, nin, a.W1, a.A1, a.strips + 2, amx);
       finish_reduce(f2, amx, 0.0, dtm, bits, cur);
-      if (!(go = lr_sync(a.bar, target))) break;
+      if (!(go = lr_sync(a, target))) break;
       // stage 3: U3 = 1/3 U + 2/3 (U2 + L(U2)); then the chemistry of the own cells
       amx = 0.0;
       bits = line_tile<3, V, LR_NT, S>(m, g, a.W1, a.A1, U, a.W0, jb_fin_cell(a.A0, nullptr, -1, 0), a.strips + 2,
@@ -168,7 +172,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
       }
       lr_strips(m, g, x0, nin, a.U_out, a.aux_out, a.strips, amx);
       finish_reduce(f4, amx, 0.0, dtm, bits | (st << 16), cur);
-      go = lr_sync(a.bar, target);
+      go = lr_sync(a, target);
     } else {
       unsigned bits = 0, st = 0;
       double amx = 0.0, amy = 0.0, dtm = inf;
@@ -179,26 +183,26 @@ __global__ void __launch_bounds__(LR_NT, 3)
           select_cell<1, true, true, false>(m, g, Us, nullptr, a.cand, As, a.strips, cur, __ldcg(&cur->mask[midx]), c,
                                             amx, amy, dtm, st);
         block_reduce_store(amx, 0.0, inf, st << 16, cur, aidx, true, false, -1);
-        return lr_sync(a.bar, target);
+        return lr_sync(a, target);
       };
       // stage 1: U1 = U + L(U)
       bits = line_tile<1, V, LR_NT, S>(m, g, U, aux, U, a.W0, jb_fin_cand(a.cand, 0), a.strips,
                                        bitsd(__ldcg(&prv->ax[3])), dt, x0, smraw, amx, dtm, cur);
       finish_reduce(jb_fin_cand(a.cand, 0), 0.0, 0.0, inf, bits, cur);
-      if (!(go = lr_sync(a.bar, target))) break;
+      if (!(go = lr_sync(a, target))) break;
       if (blockIdx.x == 0 && tid == 0) lr_clear(prv);  // every CTA has read it
       if (!(go = select(a.W0, a.A0, 0, 1))) break;
       // stage 2: U2 = 3/4 U + 1/4 (U1 + L(U1))
       bits = line_tile<2, V, LR_NT, S>(m, g, a.W0, a.A0, U, a.W1, jb_fin_cand(a.cand, 1), a.strips,
                                        bitsd(__ldcg(&cur->ax[1])), dt, x0, smraw, amx, dtm, cur);
       finish_reduce(jb_fin_cand(a.cand, 1), 0.0, 0.0, inf, bits, cur);
-      if (!(go = lr_sync(a.bar, target))) break;
+      if (!(go = lr_sync(a, target))) break;
       if (!(go = select(a.W1, a.A1, 1, 2))) break;
       // stage 3: U3 = 1/3 U + 2/3 (U2 + L(U2))
       bits = line_tile<3, V, LR_NT, S>(m, g, a.W1, a.A1, U, a.W0, jb_fin_cand(a.cand, 2), a.strips,
                                        bitsd(__ldcg(&cur->ax[2])), dt, x0, smraw, amx, dtm, cur);
       finish_reduce(jb_fin_cand(a.cand, 2), 0.0, 0.0, inf, bits, cur);
-      if (!(go = lr_sync(a.bar, target))) break;
+      if (!(go = lr_sync(a, target))) break;
       // chemistry at the selected stage-3 iterate
       bits = st = 0;
       const long long n3 = halley_count(__ldcg(&cur->mask[2])) * nc;
@@ -210,7 +214,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
                                               bits, st, amx, amy, dtm, nullptr);
       }
       finish_reduce(jb_fin_cand(a.cand, 3), 0.0, 0.0, inf, bits | (st << 16), cur);
-      if (!(go = lr_sync(a.bar, target))) break;
+      if (!(go = lr_sync(a, target))) break;
       amx = 0.0;
       dtm = inf;
       st = 0;
@@ -218,21 +222,35 @@ __global__ void __launch_bounds__(LR_NT, 3)
         select_cell<1, true, true, true>(m, g, a.U_out, nullptr, a.cand, a.aux_out, a.strips, cur,
                                          __ldcg(&cur->mask[3]), c, amx, amy, dtm, st);
       block_reduce_store(amx, 0.0, dtm, st << 16, cur, 3, true, use_cfl, -1);
-      go = lr_sync(a.bar, target);
+      go = lr_sync(a, target);
     }
   }
+  __shared__ int s_gone;
   __syncthreads();
   if (tid == 0) {
+    s_gone = 0;
     __threadfence();
     if (atomicAdd(&a.bar[1], 1u) == gridDim.x - 1) {  // the last to leave: no CTA waits any more
+      __threadfence();
       unsigned st = atomicExch(&a.sets[0].status, 0u) | atomicExch(&a.sets[1].status, 0u);
-      if (atomicExch(&a.bar[2], 0u)) st |= JB_ERR_TIMEOUT;
+      if (atomicExch(&a.bar[2], 0u)) {
+        st |= JB_ERR_TIMEOUT;
+        s_gone = 1;
+      }
       if (st) atomicOr(&a.slots->status, st);
       lr_clear(&a.sets[0]);
       lr_clear(&a.sets[1]);
       a.bar[0] = 0u;
       a.bar[1] = 0u;
     }
+  }
+  __syncthreads();
+  if (s_gone) {  // half a run is no result
+    const double nan = __longlong_as_double(0x7ff8000000000000LL);
+    for (long long i = tid; i < L1_NF * nc; i += LR_NT) a.U_out[i] = nan;
+    for (long long i = tid; i < 2 * nc; i += LR_NT) a.aux_out[i] = nan;
+    if (a.dt_hist)
+      for (int i = tid; i < a.nsteps; i += LR_NT) a.dt_hist[i] = nan;
   }
 }
 
@@ -253,10 +271,11 @@ int lr_resident(size_t sm) {
 }
 
 template <class V, int S>
-bool lr_try(const MP& m, const Grid& g, const LineRun& a, cudaStream_t st, cudaError_t& err) {
+bool lr_try(const MP& m, const Grid& g, LineRun& a, unsigned missing, cudaStream_t st, cudaError_t& err) {
   constexpr size_t chem = sizeof(double) * (S == 32 ? CHEM_SPLIT_SH : CHEM_SH * LR_NT), line = line_smem<V, S>(), sm = chem > line ? chem : line;
   const int nb = (g.nx + S - 1) / S;
   if (nb > lr_resident<V, S>(sm)) return false;
+  a.arrivals = (unsigned)nb + missing;
   void* args[] = {(void*)&m, (void*)&g, (void*)&a};
   err = cudaLaunchCooperativeKernel((void*)k_line_run<V, S>, dim3(nb), dim3(LR_NT), args, sm, st);
   return true;
@@ -277,7 +296,9 @@ static bool line_run_t(const MP& m, const Grid& g, const jb_line_io& io, cudaStr
   a.W0 = io.W0; a.W1 = io.W1; a.A0 = io.A0; a.A1 = io.A1; a.cand = io.cand; a.strips = io.strips;
   a.slots = io.slots; a.sets = io.slots + 1; a.bar = io.bar;
   a.dt_fixed = io.dt_fixed; a.cfl = io.cfl; a.nsteps = io.nsteps; a.dt_hist = io.dt_hist;
-  return lr_try<V, 32>(m, g, a, st, err) || lr_try<V, 58>(m, g, a, st, err) || lr_try<V, 122>(m, g, a, st, err);
+  a.limit_ns = io.wait_ms > 0.0 ? (unsigned long long)(io.wait_ms * 1e6) : LR_LIMIT_NS;
+  return lr_try<V, 32>(m, g, a, io.missing, st, err) || lr_try<V, 58>(m, g, a, io.missing, st, err) ||
+         lr_try<V, 122>(m, g, a, io.missing, st, err);
 }
 bool line_run(bool mixed, const MP& m, const Grid& g, const jb_line_io& io, cudaStream_t st, cudaError_t& err) {
   return mixed ? line_run_t<float>(m, g, io, st, err) : line_run_t<double>(m, g, io, st, err);

@@ -34,6 +34,8 @@ struct jb_line_io {
   double dt_fixed, cfl;
   int nsteps;
   double* dt_hist;
+  double wait_ms;    // limit of a barrier wait, 0: the kernel's own
+  unsigned missing;  // arrivals expected beyond the CTAs launched (jb_selftest_line_run)
 };
 
 struct Ops {

@@ -143,6 +143,32 @@ def test_line_run_is_the_separate_launches(nx, bc, prec):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx", [20, 500, 15000])
+def test_abandoned_line_run_shows_in_its_results(nx, prec):
+    """A run whose first wait runs out (it expects a block that is never
+    launched; one block, several, and the longest tiles) returns with NaN in
+    place of the state and the time steps and with the status bit, and the
+    same handle's next run is as if nothing had been."""
+    from janc_b200 import _native
+    from janc_b200 import mechanism as jm
+    from janc_b200.solver import Solver
+    b = dict(zip(KEYS[:2], BCS["walls"]))
+    one, sep = [Solver(1, nx, dx=5e-5, boundary_config=b, mechanism=jm.load(), precision=prec) for _ in range(2)]
+    sep.set_kernel_timing(True)
+    U, aux = _state(one, (nx,))
+    keep = U.clone(), aux.clone()
+    _native.check(one._lib.jb_selftest_line_run(one._h, 20.0, 1), one._h, "jb_selftest_line_run")
+    for t in one.advance(U, aux, 3, cfl=0.05):
+        assert bool(torch.isnan(t).all())
+    assert one.status() == 16 and _native.status_text(16) == "device wait timed out"
+    assert torch.equal(U, keep[0]) and torch.equal(aux, keep[1])
+    for x, y in zip(one.advance(U, aux, 3, cfl=0.05), sep.advance(U, aux, 3, cfl=0.05)):
+        assert torch.equal(x, y) and bool(torch.isfinite(x).all())
+    assert one.status() == sep.status() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("nx,ny", [(4, 4), (4, 8), (5, 7), (11, 3 * 32), (111, 128), (111, 129)])
 def test_chemistry_forms_match_the_strict_build(nx, ny):
     """reaction_source_terms with four threads a cell (up to 14208 cells:

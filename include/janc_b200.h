@@ -84,8 +84,9 @@ int jb_advance(jb_handle* h, const double* U, const double* aux, double* U_out, 
 /* Test hook for that path: the handle's next 1D run waits at most
  * wait_limit_ms (at most 1000) and for `missing` blocks more than are
  * launched, so that with missing > 0 its first wait runs out and every block
- * returns. */
-int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing);
+ * returns; its barriers count on from count0 (as late in a long run).
+ * Synchronises the stream. */
+int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing, unsigned count0, void* stream);
 
 /* One SSP-RK3 step of the flux alone, followed by update_aux after each
  * stage: time_step_dict['TVD_RK3'](U, aux, dx, dy, dt, theta, flux_func,

@@ -30,7 +30,7 @@ struct jb_handle {
   double* strips;      // ghost strips [4][nv+2][lstrip]
   jb_slots* slots;     // the step's slots, then two more sets and 16 barrier words (1D runs)
   double lr_wait_ms;   // of the next 1D run (jb_selftest_line_run)
-  unsigned lr_missing;
+  unsigned lr_missing, lr_count0;
   long long ws_bytes;
   // optional per-kernel timing of jb_advance (jb_set_kernel_timing)
   int timing;
@@ -419,9 +419,9 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
     const jb::jb_line_io io = {U,          aux,      U_out,   aux_out,  h->W[0],
                                h->W[1],    h->auxw[0], h->auxw[1], h->cand, h->strips,
                                h->slots,   reinterpret_cast<unsigned*>(h->slots + 3), dt_fixed, use_cfl ? cfl : 0.0,
-                               nsteps,     dt_hist,  h->lr_wait_ms, h->lr_missing};
+                               nsteps,     dt_hist,  h->lr_wait_ms, h->lr_missing, h->lr_count0};
     h->lr_wait_ms = 0.0;
-    h->lr_missing = 0;
+    h->lr_missing = h->lr_count0 = 0;
     cudaError_t e = cudaSuccess;
     if (o.line_run(m, g, io, st, e)) return check_cuda(h, e, "line run");
   }
@@ -558,12 +558,17 @@ int jb_advance(jb_handle* h, const double* U, const double* aux, double* U_out, 
   return advance_impl(h, U, aux, U_out, aux_out, dt_fixed, cfl, nsteps, dt_hist, stream, true);
 }
 
-int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing) {
+int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing, unsigned count0, void* stream) {
   if (!h) return JB_ERR_ARG;
   if (!(wait_limit_ms > 0.0) || wait_limit_ms > 1000.0) return set_err(h, JB_ERR_ARG, "wait limit must be in (0, 1000] ms");
   if (missing < 0) return set_err(h, JB_ERR_ARG, "missing must be >= 0");
+  // the arrival count, the first of the barrier words behind the slot sets
+  JB_TRY(cudaMemcpyAsync(h->slots + 3, &count0, sizeof(count0), cudaMemcpyHostToDevice, (cudaStream_t)stream),
+         "arrival count");
+  JB_TRY(cudaStreamSynchronize((cudaStream_t)stream), "arrival count");
   h->lr_wait_ms = wait_limit_ms;
   h->lr_missing = (unsigned)missing;
+  h->lr_count0 = count0;
   return JB_OK;
 }
 

@@ -86,7 +86,7 @@ __device__ __forceinline__ bool group_sync(const jb_ens_inst& I, unsigned& targe
       atomicAdd(I.bar, 1u);
       const unsigned long long t0 = global_ns();
       for (long long it = 0;; ++it) {
-        if (ld_acquire_u32(I.bar) >= target) break;
+        if (jb_arrived(ld_acquire_u32(I.bar), target)) break;
         if (*(volatile unsigned*)&ctl->abort) { go = 0; break; }
         if (it >= SPIN_MAX || global_ns() - t0 > limit_ns) {
           if (atomicExch(&ctl->timeout, 1u) == 0u) {

@@ -32,6 +32,7 @@ struct LineRun {
   int nsteps;
   double* dt_hist;
   unsigned arrivals;             // CTAs that a barrier waits for
+  unsigned count0;               // the arrival count before the first
   unsigned long long limit_ns;   // and how long
 };
 
@@ -59,7 +60,7 @@ __device__ __forceinline__ bool lr_sync(const LineRun& a, unsigned& target) {
     __threadfence();
     atomicAdd(&bar[0], 1u);
     unsigned long long t0 = 0;
-    for (long long it = 0; lr_acquire(&bar[0]) < target; ++it) {
+    for (long long it = 0; !jb_arrived(lr_acquire(&bar[0]), target); ++it) {
       if (*(volatile unsigned*)&bar[2]) { go = 0; break; }
       if ((it & 63) == 0) {
         unsigned long long now;
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
   const bool use_cfl = a.cfl > 0.0;
   const double inf = __longlong_as_double(0x7ff0000000000000LL);
   double* sh = reinterpret_cast<double*>(smraw) + tid;
-  unsigned target = 0;
+  unsigned target = a.count0;
   bool go = true;
   {  // alpha and CFL minimum of the initial state (set 1 plays the previous step)
     double amx = 0.0, amy = 0.0, dtm = inf;
@@ -296,6 +297,7 @@ static bool line_run_t(const MP& m, const Grid& g, const jb_line_io& io, cudaStr
   a.W0 = io.W0; a.W1 = io.W1; a.A0 = io.A0; a.A1 = io.A1; a.cand = io.cand; a.strips = io.strips;
   a.slots = io.slots; a.sets = io.slots + 1; a.bar = io.bar;
   a.dt_fixed = io.dt_fixed; a.cfl = io.cfl; a.nsteps = io.nsteps; a.dt_hist = io.dt_hist;
+  a.count0 = io.count0;
   a.limit_ns = io.wait_ms > 0.0 ? (unsigned long long)(io.wait_ms * 1e6) : LR_LIMIT_NS;
   return lr_try<V, 32>(m, g, a, io.missing, st, err) || lr_try<V, 58>(m, g, a, io.missing, st, err) ||
          lr_try<V, 122>(m, g, a, io.missing, st, err);

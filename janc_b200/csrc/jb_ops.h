@@ -36,6 +36,7 @@ struct jb_line_io {
   double* dt_hist;
   double wait_ms;    // limit of a barrier wait, 0: the kernel's own
   unsigned missing;  // arrivals expected beyond the CTAs launched (jb_selftest_line_run)
+  unsigned count0;   // the barrier words' arrival count at the launch
 };
 
 struct Ops {

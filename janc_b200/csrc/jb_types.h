@@ -135,4 +135,13 @@ typedef struct jb_slots {
   double dt;                        // time step of the current step
 } jb_slots;
 
+// Whether a barrier's arrival count has reached target.  Both are counted
+// modulo 2^32 over a whole run (444 blocks and 7 barriers a step pass 2^32
+// after 1.4 million steps), and the count is never 2^31 ahead or behind, so
+// their difference decides.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+static inline int jb_arrived(unsigned int count, unsigned int target) { return (int)(count - target) >= 0; }
+
 #endif  // JB_TYPES_H

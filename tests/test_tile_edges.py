@@ -7,6 +7,10 @@ and 122-cell line tiles, and the 512-cell register slots of a block.
 The flux bound is relative to dt/dx max(|F| + alpha |U|) of each field, the
 size of the terms whose difference is taken: about 100 roundings of float64
 (1e-13) and of float32 (2e-5) per face value, weights included."""
+import ctypes
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -158,7 +162,8 @@ def test_abandoned_line_run_shows_in_its_results(nx, prec):
     sep.set_kernel_timing(True)
     U, aux = _state(one, (nx,))
     keep = U.clone(), aux.clone()
-    _native.check(one._lib.jb_selftest_line_run(one._h, 20.0, 1), one._h, "jb_selftest_line_run")
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _native.check(one._lib.jb_selftest_line_run(one._h, 20.0, 1, 0, st), one._h, "jb_selftest_line_run")
     for t in one.advance(U, aux, 3, cfl=0.05):
         assert bool(torch.isnan(t).all())
     assert one.status() == 16 and _native.status_text(16) == "device wait timed out"
@@ -166,6 +171,44 @@ def test_abandoned_line_run_shows_in_its_results(nx, prec):
     for x, y in zip(one.advance(U, aux, 3, cfl=0.05), sep.advance(U, aux, 3, cfl=0.05)):
         assert torch.equal(x, y) and bool(torch.isfinite(x).all())
     assert one.status() == sep.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("before", [1, 17, 40, 100])
+def test_line_run_barriers_count_past_32_bits(before, prec):
+    """A run whose arrival count passes 2^32 (`before` arrivals into it: within
+    a barrier, at one and between two of its 16 blocks' barriers) is the run
+    that starts from zero, bit for bit."""
+    from janc_b200 import _native
+    from janc_b200 import mechanism as jm
+    from janc_b200.solver import Solver
+    s = Solver(1, 500, dx=5e-5, boundary_config=dict(zip(KEYS[:2], BCS["walls"])), mechanism=jm.load(), precision=prec)
+    U, aux = _state(s, (500,))
+    ref = s.advance(U, aux, 3, cfl=0.05)
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _native.check(s._lib.jb_selftest_line_run(s._h, 1000.0, 0, 2 ** 32 - before, st), s._h, "jb_selftest_line_run")
+    for x, y in zip(s.advance(U, aux, 3, cfl=0.05), ref):
+        assert torch.equal(x, y) and bool(torch.isfinite(x).all())
+    assert s.status() == 0
+
+
+def test_arrival_counts_compare_modulo_2_to_32(tmp_path):
+    """jb_arrived as the barriers use it, compiled for the host: a block whose
+    target has wrapped waits for the arrivals before the wrap, and one whose
+    target has not passes on a count that has."""
+    src = tmp_path / "a.c"
+    src.write_text('#include "jb_types.h"\nint arrived(unsigned c, unsigned t) { return jb_arrived(c, t); }\n')
+    so = tmp_path / "a.so"
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run(["gcc", "-shared", "-fPIC", "-I", os.path.join(root, "janc_b200", "csrc"), str(src), "-o", str(so)],
+                   check=True)
+    arrived = ctypes.CDLL(str(so)).arrived
+    arrived.argtypes = [ctypes.c_uint, ctypes.c_uint]
+    for base in (0, 444 * 7, 2 ** 31 - 100, 2 ** 32 - 500, 2 ** 32 - 1):
+        target = (base + 444) % 2 ** 32
+        for k in (0, 1, 443, 444, 445, 887):
+            assert bool(arrived((base + k) % 2 ** 32, target)) == (k >= 444), (base, k)
 
 
 @pytest.mark.gpu

@@ -77,7 +77,8 @@ int jb_reaction_source_terms(jb_handle* h, const double* U, const double* aux, d
  * Short 1D LF / WENO5-JS lines (fp64, mixed) run all steps in one launch whose
  * blocks wait for one another, each wait at most 2 s (a GPU shared by
  * time slices may take longer); such a run is abandoned with U_out, aux_out
- * and dt_hist filled with NaN and JB_ERR_TIMEOUT in jb_status. */
+ * and dt_hist filled with NaN and JB_ERR_TIMEOUT in jb_status.  Where such a
+ * launch is refused the steps are separate launches. */
 int jb_advance(jb_handle* h, const double* U, const double* aux, double* U_out, double* aux_out,
                double dt_fixed, double cfl, int nsteps, double* dt_hist, void* stream);
 
@@ -85,8 +86,11 @@ int jb_advance(jb_handle* h, const double* U, const double* aux, double* U_out, 
  * wait_limit_ms (at most 1000) and for `missing` blocks more than are
  * launched, so that with missing > 0 its first wait runs out and every block
  * returns; its barriers count on from count0 (as late in a long run).
- * Synchronises the stream. */
-int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing, unsigned count0, void* stream);
+ * oversize: the launch is tried also for lines whose blocks cannot all be
+ * resident, which the driver refuses, as it does on a part of a device, so
+ * that the steps go through separate launches.  Synchronises the stream. */
+int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing, unsigned count0, int oversize,
+                         void* stream);
 
 /* One SSP-RK3 step of the flux alone, followed by update_aux after each
  * stage: time_step_dict['TVD_RK3'](U, aux, dx, dy, dt, theta, flux_func,

@@ -121,7 +121,7 @@ def lib(path=None):
     L.jb_amr_flux.argtypes = [vp, i, i, i, d, d, dp, dp, d, dp, vp]
     L.jb_amr_update_aux.argtypes = [vp, i, i, i, dp, dp, dp, vp]
     L.jb_ens_selftest_timeout.argtypes = [vp, d, ctypes.POINTER(ctypes.c_uint), vp]
-    L.jb_selftest_line_run.argtypes = [vp, d, i, ctypes.c_uint, vp]
+    L.jb_selftest_line_run.argtypes = [vp, d, i, ctypes.c_uint, i, vp]
     L.jb_ens_last_error.argtypes = [vp]
     L.jb_ens_last_error.restype = ctypes.c_char_p
     for name in EXPORTS:

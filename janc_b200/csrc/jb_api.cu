@@ -31,6 +31,7 @@ struct jb_handle {
   jb_slots* slots;     // the step's slots, then two more sets and 16 barrier words (1D runs)
   double lr_wait_ms;   // of the next 1D run (jb_selftest_line_run)
   unsigned lr_missing, lr_count0;
+  bool lr_oversize;
   long long ws_bytes;
   // optional per-kernel timing of jb_advance (jb_set_kernel_timing)
   int timing;
@@ -419,9 +420,11 @@ static int advance_impl(jb_handle* h, const double* U, const double* aux, double
     const jb::jb_line_io io = {U,          aux,      U_out,   aux_out,  h->W[0],
                                h->W[1],    h->auxw[0], h->auxw[1], h->cand, h->strips,
                                h->slots,   reinterpret_cast<unsigned*>(h->slots + 3), dt_fixed, use_cfl ? cfl : 0.0,
-                               nsteps,     dt_hist,  h->lr_wait_ms, h->lr_missing, h->lr_count0};
+                               nsteps,     dt_hist,  h->lr_wait_ms, h->lr_missing, h->lr_count0,
+                               h->lr_oversize};
     h->lr_wait_ms = 0.0;
     h->lr_missing = h->lr_count0 = 0;
+    h->lr_oversize = false;
     cudaError_t e = cudaSuccess;
     if (o.line_run(m, g, io, st, e)) return check_cuda(h, e, "line run");
   }
@@ -558,7 +561,8 @@ int jb_advance(jb_handle* h, const double* U, const double* aux, double* U_out, 
   return advance_impl(h, U, aux, U_out, aux_out, dt_fixed, cfl, nsteps, dt_hist, stream, true);
 }
 
-int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing, unsigned count0, void* stream) {
+int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing, unsigned count0, int oversize,
+                         void* stream) {
   if (!h) return JB_ERR_ARG;
   if (!(wait_limit_ms > 0.0) || wait_limit_ms > 1000.0) return set_err(h, JB_ERR_ARG, "wait limit must be in (0, 1000] ms");
   if (missing < 0) return set_err(h, JB_ERR_ARG, "missing must be >= 0");
@@ -569,6 +573,7 @@ int jb_selftest_line_run(jb_handle* h, double wait_limit_ms, int missing, unsign
   h->lr_wait_ms = wait_limit_ms;
   h->lr_missing = (unsigned)missing;
   h->lr_count0 = count0;
+  h->lr_oversize = oversize != 0;
   return JB_OK;
 }
 

@@ -271,23 +271,31 @@ int lr_resident(size_t sm) {
   return n * nsm;
 }
 
+// Launch with tiles of S cells; false, and nothing launched, where their CTAs
+// do not fit the device, or not the part of it that this process may use (an
+// MPS share, a green context), which only the launch itself can tell.
 template <class V, int S>
-bool lr_try(const MP& m, const Grid& g, LineRun& a, unsigned missing, cudaStream_t st, cudaError_t& err) {
+bool lr_try(const MP& m, const Grid& g, LineRun& a, const jb_line_io& io, cudaStream_t st, cudaError_t& err) {
   constexpr size_t chem = sizeof(double) * (S == 32 ? CHEM_SPLIT_SH : CHEM_SH * LR_NT), line = line_smem<V, S>(), sm = chem > line ? chem : line;
   const int nb = (g.nx + S - 1) / S;
-  if (nb > lr_resident<V, S>(sm)) return false;
-  a.arrivals = (unsigned)nb + missing;
+  const int fit = lr_resident<V, S>(sm);
+  if (!fit || (nb > fit && !io.oversize)) return false;
+  a.arrivals = (unsigned)nb + io.missing;
   void* args[] = {(void*)&m, (void*)&g, (void*)&a};
   err = cudaLaunchCooperativeKernel((void*)k_line_run<V, S>, dim3(nb), dim3(LR_NT), args, sm, st);
-  return true;
+  if (err != cudaErrorCooperativeLaunchTooLarge) return true;
+  (void)cudaGetLastError();  // refused, not failed: the next launch check must not find it
+  err = cudaSuccess;
+  return false;
 }
 
 }  // namespace
 
 // The run as one launch where one tile per resident CTA covers the line (32
 // cells a tile while that suffices, one per lane with the chemistry split over
-// the four warps; then 58, then 122); false, and nothing launched, where it does not or the stream is being
-// captured (the separate launches are plain graph nodes).
+// the four warps; then 58, then 122); false, and nothing launched, where it does not,
+// the driver refuses the launch, or the stream is being captured (the separate
+// launches are plain graph nodes).
 template <class V>
 static bool line_run_t(const MP& m, const Grid& g, const jb_line_io& io, cudaStream_t st, cudaError_t& err) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -299,8 +307,8 @@ static bool line_run_t(const MP& m, const Grid& g, const jb_line_io& io, cudaStr
   a.dt_fixed = io.dt_fixed; a.cfl = io.cfl; a.nsteps = io.nsteps; a.dt_hist = io.dt_hist;
   a.count0 = io.count0;
   a.limit_ns = io.wait_ms > 0.0 ? (unsigned long long)(io.wait_ms * 1e6) : LR_LIMIT_NS;
-  return lr_try<V, 32>(m, g, a, io.missing, st, err) || lr_try<V, 58>(m, g, a, io.missing, st, err) ||
-         lr_try<V, 122>(m, g, a, io.missing, st, err);
+  return lr_try<V, 32>(m, g, a, io, st, err) || lr_try<V, 58>(m, g, a, io, st, err) ||
+         lr_try<V, 122>(m, g, a, io, st, err);
 }
 bool line_run(bool mixed, const MP& m, const Grid& g, const jb_line_io& io, cudaStream_t st, cudaError_t& err) {
   return mixed ? line_run_t<float>(m, g, io, st, err) : line_run_t<double>(m, g, io, st, err);

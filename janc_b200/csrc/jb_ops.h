@@ -37,6 +37,7 @@ struct jb_line_io {
   double wait_ms;    // limit of a barrier wait, 0: the kernel's own
   unsigned missing;  // arrivals expected beyond the CTAs launched (jb_selftest_line_run)
   unsigned count0;   // the barrier words' arrival count at the launch
+  bool oversize;     // launch also where the CTAs cannot all be resident (refused)
 };
 
 struct Ops {

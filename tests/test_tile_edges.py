@@ -163,7 +163,7 @@ def test_abandoned_line_run_shows_in_its_results(nx, prec):
     U, aux = _state(one, (nx,))
     keep = U.clone(), aux.clone()
     st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-    _native.check(one._lib.jb_selftest_line_run(one._h, 20.0, 1, 0, st), one._h, "jb_selftest_line_run")
+    _native.check(one._lib.jb_selftest_line_run(one._h, 20.0, 1, 0, 0, st), one._h, "jb_selftest_line_run")
     for t in one.advance(U, aux, 3, cfl=0.05):
         assert bool(torch.isnan(t).all())
     assert one.status() == 16 and _native.status_text(16) == "device wait timed out"
@@ -187,10 +187,30 @@ def test_line_run_barriers_count_past_32_bits(before, prec):
     U, aux = _state(s, (500,))
     ref = s.advance(U, aux, 3, cfl=0.05)
     st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-    _native.check(s._lib.jb_selftest_line_run(s._h, 1000.0, 0, 2 ** 32 - before, st), s._h, "jb_selftest_line_run")
+    _native.check(s._lib.jb_selftest_line_run(s._h, 1000.0, 0, 2 ** 32 - before, 0, st), s._h, "jb_selftest_line_run")
     for x, y in zip(s.advance(U, aux, 3, cfl=0.05), ref):
         assert torch.equal(x, y) and bool(torch.isfinite(x).all())
     assert s.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_refused_line_run_takes_the_separate_launches(prec):
+    """A cooperative launch that the driver refuses (70000 cells are 574 blocks
+    of the longest tiles, more than the device holds at three an SM) leaves the
+    steps to the separate launches, and no error behind."""
+    from janc_b200 import _native
+    from janc_b200 import mechanism as jm
+    from janc_b200.solver import Solver
+    nx = 70000
+    one, sep = [Solver(1, nx, dx=5e-5, boundary_config=dict(zip(KEYS[:2], BCS["walls"])), mechanism=jm.load(),
+                       precision=prec) for _ in range(2)]
+    U, aux = _state(one, (nx,))
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _native.check(one._lib.jb_selftest_line_run(one._h, 1000.0, 0, 0, 1, st), one._h, "jb_selftest_line_run")
+    for x, y in zip(one.advance(U, aux, 2, cfl=0.05), sep.advance(U, aux, 2, cfl=0.05)):
+        assert torch.equal(x, y) and bool(torch.isfinite(x).all())
+    assert one.status() == sep.status() == 0
 
 
 def test_arrival_counts_compare_modulo_2_to_32(tmp_path):

@@ -250,6 +250,30 @@ def test_adjoint_with_rate_offsets_matches_twin(omech, nsteps, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64_strict", "fp64"])
+def test_adjoint_of_gas_at_rest_matches_twin(omech, prec):
+    """Two steps of a jump into exactly uniform gas at rest, as smoke() takes
+    them, to its 1e-8.  The gradient there hangs on the state's last bits (one
+    ulp of P, T or Y changes the twin's own by its whole size), so this holds as
+    far as the build rounds as the reference's formulas do."""
+    from janc_b200.adjoint import Trajectory, probe_trajectory
+    from janc_b200.solver import Solver
+    nx, ny, dx, probe = 24, 16, 1.953125e-4, (12, 6, 4, 4)
+    P = np.full((1, nx, ny), 101325.0)
+    T = np.full((1, nx, ny), 300.0)
+    P[:, :3] = 30 * 101325.0
+    T[:, :3] = 3000.0
+    Y = np.tile(jo.stoich_Y(omech, 1.0)[:, None, None], (1, nx, ny))
+    traj = Trajectory(Solver(2, nx, ny, dx, dx, BC_SLIP, precision=prec), 0.1, probe, checkpoint=1)
+    cu = lambda a: torch.as_tensor(a, dtype=torch.float64, device="cuda")  # noqa: E731
+    Tg = cu(T).requires_grad_()
+    dts, pps = probe_trajectory(traj, cu(P), Tg, cu(Y), None, 2)
+    (dts * pps).sum().backward()
+    _, gTr, _ = _twin(omech, nx, ny, BC_SLIP, P, T, Y, 2, 0.1, probe)
+    assert _rel(Tg.grad.cpu().numpy(), gTr) <= 1e-8
+
+
+@pytest.mark.gpu
 def test_adjoint_matches_finite_differences(omech):
     from janc_b200.adjoint import Trajectory
     from janc_b200.solver import Solver

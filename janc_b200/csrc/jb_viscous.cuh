@@ -239,7 +239,9 @@ __device__ __forceinline__ void visc_node2d(const MP& m, const Grid& g, const jb
   // Prandtl and Lewis numbers without a turbulence model: rho D_k = mu / (Pr
   // Le) for every species (cp_k cancels)
   const bool simple = tr.conductivity_model == 0 && tr.diffusivity_model == 0 && !tr.turbulence_model;
-  const double iPr = rcp_nr(tr.Pr), rD0 = mu * iPr * rcp_nr(tr.Le);
+  // (divisions: an infinite number, which switches its transport off, has the
+  // reciprocal 0, and rcp_nr's would be NaN)
+  const double iPr = 1.0 / tr.Pr, rD0 = mu * iPr * (1.0 / tr.Le);
   double e = 0.0, cp = 0.0;
   auto species = [&](int k, double cpk, double hk) {
     const double dY = ddn(4 + k), Y = __ldg(n0 + (4 + k) * np);

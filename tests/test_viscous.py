@@ -182,6 +182,26 @@ def test_viscous_flux_2d_vs_oracle(omech, prec, tkey, combo):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64_strict", "fp64"])
+@pytest.mark.parametrize("off", [{"Le": np.inf}, {"Pr": np.inf}, {"Pr": np.inf, "Le": np.inf}])
+def test_infinite_transport_numbers_switch_transport_off(omech, prec, off):
+    """An infinite Lewis or Prandtl number is no species diffusion and no heat
+    conduction: the oracle's fluxes, to the bounds of the other models."""
+    from janc_b200.solver import Solver
+    bc = dict(zip(["left_boundary", "right_boundary", "bottom_boundary", "top_boundary"], COMBOS[1]))
+    nx, ny, dx, dy = 37, 23, 2e-5, 3e-5
+    U, aux = _state2d(omech, nx, ny, 3)
+    tc = dict(TRANSPORT["sutherland_pr_le"], **off)
+    ref = jo.Solver(omech, "2D", dx, dy, bc, 0.5, flux_config=LF_VISC, transport_config=tc).flux_func(
+        U, aux, dx, dy, 1e-9, None)
+    assert np.all(np.isfinite(ref))
+    s = Solver(2, nx, ny, dx, dy, bc, precision=prec, flux_config=LF_VISC, transport_config=tc)
+    r = host(s.flux_func(cuda(U), cuda(aux), dx, dy, 1e-9, None))
+    assert np.all(np.isfinite(r))
+    assert field_err(r, ref) < (1e-12 if prec == "fp64_strict" else 1e-11)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("prec", ["fp64_strict", "fp64", "mixed"])
 @pytest.mark.parametrize("tkey", ["sutherland_pr_le", "les_pr_le"])
 def test_viscous_godunov_steps_2d_vs_oracle(omech, prec, tkey):

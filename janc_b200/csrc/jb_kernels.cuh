@@ -2156,8 +2156,7 @@ __device__ __forceinline__ void chem_cell_gen(const MP& m, double rho, const dou
 constexpr int CS_LD = 32, CS_E = JB_GEN_ROWS * 32, CS_B = CS_E + 2 * NR * 32, CS_A = CS_B + NR * CS_LD;
 constexpr int CHEM_SPLIT_SH = CS_A + NR * NR * CS_LD;
 template <int G>
-__device__ __forceinline__ void chem_split_part(const MP& m, const ChemIn& in, double idt, double* sh, int lane) {
-  double* col = sh + lane;
+__device__ __forceinline__ void chem_split_rates(const MP& m, const ChemIn& in, double* col) {
   double E[NR], iE[NR], none[NR];
 #pragma unroll
   for (int k = 0; k < NR; ++k) {
@@ -2165,7 +2164,9 @@ __device__ __forceinline__ void chem_split_part(const MP& m, const ChemIn& in, d
     iE[k] = col[CS_E + (NR + k) * 32];
   }
   chem_rates_gen<G>(m, in.lT, in.invT, in.Tp, in.pT, in.X, in.Xc, E, iE, col, 32, none);
-  __syncthreads();
+}
+template <int G>
+__device__ __forceinline__ void chem_split_cols(const MP& m, const ChemIn& in, double idt, double* col) {
   double rMX[NR], J[NR][NR], w2[2];
 #pragma unroll
   for (int k = 0; k < NR; ++k)
@@ -2198,11 +2199,20 @@ __device__ __forceinline__ void chem_split(const MP& m, double rho, const double
     sh[CS_E + (NR + k) * 32 + lane] = iE;
   }
   __syncthreads();
-  switch (wp) {  // each case holds one more block barrier
-    case 0: chem_split_part<0>(m, in, idt, sh, lane); break;
-    case 1: chem_split_part<1>(m, in, idt, sh, lane); break;
-    case 2: chem_split_part<2>(m, in, idt, sh, lane); break;
-    default: chem_split_part<3>(m, in, idt, sh, lane); break;
+  // the barriers stay outside the switches: every warp meets the same one
+  double* col = sh + lane;
+  switch (wp) {
+    case 0: chem_split_rates<0>(m, in, col); break;
+    case 1: chem_split_rates<1>(m, in, col); break;
+    case 2: chem_split_rates<2>(m, in, col); break;
+    default: chem_split_rates<3>(m, in, col); break;
+  }
+  __syncthreads();
+  switch (wp) {
+    case 0: chem_split_cols<0>(m, in, idt, col); break;
+    case 1: chem_split_cols<1>(m, in, idt, col); break;
+    case 2: chem_split_cols<2>(m, in, idt, col); break;
+    default: chem_split_cols<3>(m, in, idt, col); break;
   }
   __syncthreads();
   if (wp == 0) {

@@ -286,6 +286,9 @@ int jb_kernel_times(jb_handle* h, double* ms, long long* launches);
  * threads, each doing iters*128 float64 FMAs (2 FLOP each), for measuring
  * the device's FP64 peak.  `scratch` is a device buffer of `blocks` doubles. */
 int jb_probe_fp64_fma(int blocks, int iters, double* scratch, void* stream);
+/* y[i] = the kernels' own reciprocal of x[i] (n device doubles; within 2 ulp
+ * where x and 1 / x are normal numbers). */
+int jb_probe_rcp(long long n, const double* x, double* y, void* stream);
 
 /* Human-readable description of the last error on this handle. */
 const char* jb_last_error(const jb_handle* h);

@@ -27,7 +27,7 @@ EXPORTS = ["jb_version", "jb_create", "jb_destroy", "jb_set_theta", "jb_flux_fun
            "jb_workspace_bytes", "jb_set_spacing", "jb_set_flux_scheme", "jb_set_reconstruction", "jb_set_transport", "jb_set_exchange", "jb_set_ghost_cells", "jb_boundary_conditions",
            "jb_sizeof_mech_params",
            "jb_sizeof_grid",
-           "jb_last_error", "jb_probe_fp64_fma", "jb_set_kernel_timing", "jb_kernel_times",
+           "jb_last_error", "jb_probe_fp64_fma", "jb_probe_rcp", "jb_set_kernel_timing", "jb_kernel_times",
            "jb_update_aux_noalloc", "jb_rk3", "jb_u_to_prim",
            "jb_ens_create", "jb_ens_destroy", "jb_ens_instance", "jb_ens_total_cells", "jb_ens_configure",
            "jb_ens_set_back_pressure",
@@ -90,6 +90,7 @@ def lib(path=None):
     L.jb_set_ghost_cells.argtypes = [vp, dp, dp, dp, dp, EXCHANGE_FN, vp]
     L.jb_boundary_conditions.argtypes = [vp, dp, dp, dp, dp, vp]
     L.jb_probe_fp64_fma.argtypes = [i, i, dp, vp]
+    L.jb_probe_rcp.argtypes = [ll, dp, dp, vp]
     L.jb_set_kernel_timing.argtypes = [vp, i]
     L.jb_update_aux_noalloc.argtypes = [ctypes.POINTER(_mech.MechParams), i, i, i, i, dp, dp, dp, vp]
     L.jb_kernel_times.argtypes = [vp, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_longlong)]

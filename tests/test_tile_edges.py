@@ -264,3 +264,37 @@ def test_block_stage_matches_the_strict_build(bx, by):
         for f in range(14):
             assert float((a[:, f] - b[:, f]).abs().max()) <= 1e-12 * float(a[:, f].abs().max()), (stage, f)
     assert s0.status() == s1.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["range", "mantissas", "edges"])
+def test_reciprocal_is_within_two_ulp(kind):
+    """rcp_nr, which the fast builds take for pivots, concentrations,
+    equilibrium factors, Halley steps and float64 WENO weights, against 1 / x
+    (correctly rounded): random numbers over all exponents whose reciprocal is
+    normal, mantissas next to 1, 2 and the approximation's own steps, and the
+    ends of the range; of 0, infinity and NaN it is NaN."""
+    from janc_b200 import _native
+    rng = np.random.default_rng(11)
+    n = 1 << 20
+    sign = rng.choice([-1.0, 1.0], n)
+    if kind == "range":
+        x = sign * np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(-1020, 1021, n))
+    elif kind == "mantissas":
+        at = 1.0 + rng.integers(0, 1 << 20, n) * 2.0 ** -20  # a step of the 20-bit approximation
+        x = sign * np.ldexp(np.nextafter(at, rng.choice([0.0, 3.0], n)), rng.integers(-40, 41, n))
+        x[:3] = 1.0, np.nextafter(1.0, 2.0), np.nextafter(2.0, 1.0)
+    else:
+        x = np.repeat([2.0 ** -1021, 2.0 ** -1021 * (1 + 2.0 ** -52), 1e-300, 1e300, 2.0 ** 1021], 7)
+    y = torch.empty(x.size, dtype=torch.float64, device="cuda")
+    xd = torch.as_tensor(x, device="cuda")
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    L = _native.lib()
+    assert L.jb_probe_rcp(x.size, p(xd), p(y), st) == 0
+    ref = 1.0 / x
+    assert np.all(np.abs(y.cpu().numpy() - ref) <= 2.0 * np.spacing(np.abs(ref)))
+    bad = torch.tensor([0.0, np.inf, -np.inf, np.nan], dtype=torch.float64, device="cuda")
+    out = torch.empty_like(bad)
+    assert L.jb_probe_rcp(4, p(bad), p(out), st) == 0
+    assert bool(torch.isnan(out).all())

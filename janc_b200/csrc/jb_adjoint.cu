@@ -36,8 +36,7 @@
 //   k_init_vjp      initial state from (P, T, Y): T adjoint
 #define JB_NS adj
 #define JB_FAST 1
-#include <atomic>
-
+#include "jb_device.h"
 #include "jb_kernels.cuh"
 
 #include "jb_adjoint.h"
@@ -1484,14 +1483,7 @@ static cudaError_t flux_stage_t(const jb_mech_params& m, const jb_grid& g, const
   // length of 6 .. 48 that takes the fewest waves x (length + 7) over the
   // resident blocks.  200 x 96 cells: 9 (one wave), where a fixed 24 left most
   // of the chip idle (45 us a launch); large grids stay near 24.
-  static std::atomic<int> sm_count{0};
-  int nsm = sm_count.load(std::memory_order_relaxed);
-  if (!nsm) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    sm_count.store(nsm, std::memory_order_relaxed);
-  }
+  const int nsm = sm_count();
   const int nlx = (g.ny + SW_NT - 1) / SW_NT, nly = (g.nx + SW_NT - 1) / SW_NT;
   int sw_r = 24, nbx = 0, nby = 0;
   long long best = -1;

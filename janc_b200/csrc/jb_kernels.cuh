@@ -2348,11 +2348,9 @@ __global__ void __launch_bounds__(JB_CHEM_NT, JB_CHEM_MINB) k_chem(MP m, Grid g,
 
 #if JB_FAST
 // k_chem with four threads a cell (chem_split), 32 cells a block.
+constexpr int CHEM_SPLIT_MINB = 3;
 template <int DIM, bool WRITE_S, bool CELL>
-#ifndef JB_CHEM_SPLIT_MINB
-#define JB_CHEM_SPLIT_MINB 3
-#endif
-__global__ void __launch_bounds__(128, JB_CHEM_SPLIT_MINB) k_chem_split(MP m, Grid g, const double* __restrict__ U,
+__global__ void __launch_bounds__(128, CHEM_SPLIT_MINB) k_chem_split(MP m, Grid g, const double* __restrict__ U,
                                                      const double* __restrict__ aux, double* __restrict__ out,
                                                      jb_fin fin, Slots* slots, double dt_arg) {
   __shared__ double sh[CHEM_SPLIT_SH];

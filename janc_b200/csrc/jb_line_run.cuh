@@ -259,16 +259,14 @@ __global__ void __launch_bounds__(LR_NT, 3)
 // launch), queried once per device.
 template <class V, int S>
 int lr_resident(size_t sm) {
-  static int known[64];
-  int dev = 0, n = 0, nsm = 0, coop = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (known[dev]) return known[dev] - 1;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  cudaFuncSetAttribute(k_line_run<V, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_line_run<V, S>, LR_NT, sm) != cudaSuccess) n = 0;
-  known[dev] = n * nsm + 1;
-  return n * nsm;
+  static PerDevice known;
+  return known.get([sm](int dev) {
+    int n = 0, coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    cudaFuncSetAttribute(k_line_run<V, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_line_run<V, S>, LR_NT, sm) != cudaSuccess) n = 0;
+    return n * sm_count();
+  });
 }
 
 // Launch with tiles of S cells; false, and nothing launched, where their CTAs

@@ -1,8 +1,10 @@
 """The fp64 and mixed builds' own flux kernels (2D x sweep + y runs, 1D line
 tiles) and the register form of the block temperature solve against the
 strict build's general kernels, at the edges of their tiles and segments:
-axes below, at and above the 128-cell y segments, the sweep segments, the 26-
-and 122-cell line tiles, and the 512-cell register slots of a block.
+axes below, at and above the 128-cell y segments, the sweep segments, the
+line tiles (32 cells, above 18944 cells 122; in one-launch runs 32, above 14208
+cells 58, above 25752 122, up to 54168; on 148 SMs), and the 512-cell register
+slots of a block.
 
 The flux bound is relative to dt/dx max(|F| + alpha |U|) of each field, the
 size of the terms whose difference is taken: about 100 roundings of float64
@@ -20,6 +22,7 @@ ND = {"P0": 10 * 101325, "T0": 300, "R0": 369, "x0": 0.08}
 KEYS = ("left_boundary", "right_boundary", "bottom_boundary", "top_boundary")
 BCS = {"walls": ("slip_wall", "zero_gradient", "slip_wall", "no_slip_wall"),
        "outlets": ("pressure_outlet", "no_slip_wall", "zero_gradient", "pressure_outlet"),
+       "ends": ("pressure_outlet", "pressure_outlet"),  # 1D
        "ring": ("periodic", "periodic", "periodic", "periodic"),
        "injector": ("periodic", "periodic", "rdc_injector", "pressure_outlet")}
 
@@ -89,12 +92,15 @@ def test_sweep_flux_matches_the_strict_tiles(nx, ny, bc, prec):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
-@pytest.mark.parametrize("nx,bc", [(4, "ring"), (25, "walls"), (26, "outlets"), (27, "ring"), (53, "walls"),
-                                   (15392, "outlets"), (15393, "walls"), (15494, "ring"), (15495, "outlets")])
+@pytest.mark.parametrize("nx,bc", [(4, "ring"), (31, "walls"), (32, "outlets"), (33, "ends"), (34, "ends"),
+                                   (64, "ring"), (65, "walls"), (18944, "outlets"), (18945, "walls"), (19031, "ends"),
+                                   (19032, "ring"), (19033, "ends"), (19034, "ends"), (19067, "ring")])
 def test_line_flux_matches_the_strict_tiles(nx, bc, prec):
+    """One tile to both sides of the rule's line, and last tiles of one, two, all
+    but one and all cells beside an outlet in either tile."""
     s0, s1 = _pair(1, nx, 1, bc, prec, False, 5e-5)
     U, aux = _state(s0, (nx,))
-    _check_flux(s0, s1, U, aux, {"Pb": 101325.0} if bc == "outlets" else None, 5e-5, prec)
+    _check_flux(s0, s1, U, aux, {"Pb": 101325.0} if bc in ("outlets", "ends") else None, 5e-5, prec)
 
 
 @pytest.mark.gpu
@@ -121,23 +127,23 @@ def test_block_update_matches_the_strict_loop(X, Y):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
-@pytest.mark.parametrize("nx,bc", [(4, "ring"), (26, "outlets"), (27, "outlets"), (54, "outlets"), (131, "walls"),
-                                   (1301, "ring"), (11544, "walls"), (11545, "outlets"), (25753, "outlets"),
-                                   (54169, "walls")])
+@pytest.mark.parametrize("nx,bc", [(4, "ring"), (32, "ends"), (33, "ends"), (34, "ends"), (65, "ends"), (66, "ends"),
+                                   (131, "walls"), (1301, "ring"), (11545, "ends"), (14208, "walls"), (14209, "ends"),
+                                   (14211, "ends"), (20001, "ring"), (20012, "ends"), (25752, "walls"), (25753, "ends"),
+                                   (25865, "ends"), (25866, "ends"), (54168, "walls")])
 def test_line_run_is_the_separate_launches(nx, bc, prec):
     """advance of a 1D line as one persistent launch, bitwise the same steps
     as one launch per phase (the form that per-kernel timing takes): last
-    tiles of one and two cells beside an outlet, one block, the tile sizes'
-    limits, CFL and fixed steps, the launch repeated on its own workspace."""
+    tiles of one and two cells beside an outlet (33, 14211, 25865; 34, 20012,
+    25866), one block, both sides of the tile sizes' limits, CFL and fixed
+    steps, the launch repeated on its own workspace."""
     from janc_b200 import mechanism as jm
     from janc_b200.solver import Solver
     b = dict(zip(KEYS[:2], BCS[bc]))
-    if bc == "outlets":
-        b["right_boundary"] = "pressure_outlet"
     one, sep = [Solver(1, nx, dx=5e-5, boundary_config=b, mechanism=jm.load(), precision=prec) for _ in range(2)]
     sep.set_kernel_timing(True)
     U, aux = _state(one, (nx,))
-    theta = {"Pb": 101325.0} if bc == "outlets" else None
+    theta = {"Pb": 101325.0} if bc == "ends" else None
     for how in ({"cfl": 0.05}, {"dt": 1e-9}, {"cfl": 0.02}):
         a = one.advance(U, aux, 3, theta=theta, **how)
         r = sep.advance(U, aux, 3, theta=theta, **how)
@@ -148,12 +154,13 @@ def test_line_run_is_the_separate_launches(nx, bc, prec):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
-@pytest.mark.parametrize("nx", [20, 500, 15000])
+@pytest.mark.parametrize("nx", [20, 500, 14208, 14209, 25752, 25753, 54168])
 def test_abandoned_line_run_shows_in_its_results(nx, prec):
     """A run whose first wait runs out (it expects a block that is never
-    launched; one block, several, and the longest tiles) returns with NaN in
-    place of the state and the time steps and with the status bit, and the
-    same handle's next run is as if nothing had been."""
+    launched; one block, several, and every tile size to its limits) returns
+    with NaN in place of the state and the time steps and with the status bit,
+    and the same handle's next run is as if nothing had been.  So lines of
+    these sizes do take the one launch."""
     from janc_b200 import _native
     from janc_b200 import mechanism as jm
     from janc_b200.solver import Solver

@@ -80,7 +80,7 @@ def field_err(U, Uref):
     mom = rel_l1(U[1:1 + nmom], Uref[1:1 + nmom])
     errs = [mom] + [rel_l1(U[i], Uref[i]) for i in [0] + list(range(1 + nmom, U.shape[0]))
                     if np.sum(np.abs(Uref[i])) > 1e-30]
-    return max(errs)
+    return float(np.max(errs))  # a NaN anywhere is the result
 
 
 def front(U, aux, nY):

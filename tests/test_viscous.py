@@ -56,7 +56,7 @@ def field_err(a, b):
         den = np.sum(np.abs(b[i]))
         if den > 1e-30:
             errs.append(np.sum(np.abs(a[i] - b[i])) / den)
-    return max(errs)
+    return float(np.max(errs))  # a NaN anywhere is the result
 
 
 # ---------------------------------------------------------------- CPU

@@ -75,8 +75,9 @@ int jb_reaction_source_terms(jb_handle* h, const double* U, const double* aux, d
  * otherwise dt_fixed.  dt_hist (device, nsteps doubles, may be NULL) receives
  * each step's dt.  U/aux are not modified; U_out/aux_out receive the result.
  * Short 1D LF / WENO5-JS lines (fp64, mixed) run all steps in one launch whose
- * blocks wait for one another, each wait at most 2 s (a GPU shared by
- * time slices may take longer); such a run is abandoned with U_out, aux_out
+ * blocks wait for one another: at most 60 s for all of them to start (beside
+ * other streams' kernels), then at most 2 s each (a GPU shared by time slices
+ * may take longer).  A run that waits longer is abandoned with U_out, aux_out
  * and dt_hist filled with NaN and JB_ERR_TIMEOUT in jb_status.  Where such a
  * launch is refused the steps are separate launches. */
 int jb_advance(jb_handle* h, const double* U, const double* aux, double* U_out, double* aux_out,

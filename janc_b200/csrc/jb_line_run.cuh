@@ -19,10 +19,12 @@
 // strip row), so that the CTA that writes one never races with a neighbour
 // still reading another.  The slot sets alternate between even and odd steps.
 //
-// Every wait is bounded (2 s and 2^26 polls), after which the run is
-// abandoned: the last CTA to leave fills the outputs and the time steps with
-// NaN and sets JB_ERR_TIMEOUT.  It clears the barrier words and slot sets for
-// the next launch in any case.
+// Every wait is bounded, after which the run is abandoned.  The first barrier
+// waits for CTAs that may not be resident yet, because other streams' kernels
+// (a long ensemble run, say) hold their places: up to 60 s.  After it every CTA
+// is resident, and a wait is 2 s at most.  Of an abandoned run the last CTA to
+// leave fills the outputs and the time steps with NaN and sets JB_ERR_TIMEOUT;
+// it clears the barrier words and slot sets for the next launch in any case.
 struct LineRun {
   const double *U, *aux;
   double *U_out, *aux_out, *W0, *W1, *A0, *A1, *cand, *strips;
@@ -33,14 +35,15 @@ struct LineRun {
   double* dt_hist;
   unsigned arrivals;             // CTAs that a barrier waits for
   unsigned count0;               // the arrival count before the first
-  unsigned long long limit_ns;   // and how long
+  unsigned long long start_ns;   // how long the first may wait,
+  unsigned long long limit_ns;   // and the others
 };
 
 namespace {
 
 constexpr int LR_NT = 128;
-constexpr unsigned long long LR_LIMIT_NS = 2000000000ull;
-constexpr long long LR_SPIN_MAX = 1LL << 26;
+constexpr unsigned long long LR_START_NS = 60000000000ull, LR_LIMIT_NS = 2000000000ull;
+constexpr long long LR_SPIN_MAX = 1LL << 28;
 
 __device__ __forceinline__ unsigned lr_acquire(const unsigned* p) {
   unsigned v;
@@ -49,7 +52,7 @@ __device__ __forceinline__ unsigned lr_acquire(const unsigned* p) {
 }
 
 // Barrier of all CTAs (every thread calls it); false when the run is abandoned.
-__device__ __forceinline__ bool lr_sync(const LineRun& a, unsigned& target) {
+__device__ __forceinline__ bool lr_sync(const LineRun& a, unsigned& target, unsigned long long limit_ns) {
   __shared__ int s_go;
   __syncthreads();
   if (a.arrivals == 1) return true;
@@ -66,7 +69,7 @@ __device__ __forceinline__ bool lr_sync(const LineRun& a, unsigned& target) {
         unsigned long long now;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
         if (it == 0) t0 = now;
-        if (it >= LR_SPIN_MAX || now - t0 > a.limit_ns) {
+        if (it >= LR_SPIN_MAX || now - t0 > limit_ns) {
           atomicExch(&bar[2], 1u);
           go = 0;
           break;
@@ -127,7 +130,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
       select_cell<1, false, true, true>(m, g, a.U, a.aux, nullptr, nullptr, a.strips, &a.sets[1], 0u, c, amx, amy,
                                         dtm, st);
     block_reduce_store(amx, amy, dtm, st << 16, &a.sets[1], 3, true, use_cfl, -1);
-    go = lr_sync(a, target);
+    go = lr_sync(a, target, a.start_ns);
   }
 #pragma unroll 1
   for (int step = 0; go && step < a.nsteps; ++step) {
@@ -148,7 +151,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
                                        amx, dtm, cur);
       lr_strips(m, g, x0, nin, a.W0, a.A0, a.strips + 1, amx);
       finish_reduce(f1, amx, 0.0, dtm, bits, cur);
-      if (!(go = lr_sync(a, target))) break;
+      if (!(go = lr_sync(a, target, a.limit_ns))) break;
       if (blockIdx.x == 0 && tid == 0) lr_clear(prv);  // every CTA has read it
       // stage 2: U2 = 3/4 U + 1/4 (U1 + L(U1))
       amx = 0.0;
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
                                        smraw, amx, dtm, cur);
       lr_strips(m, g, x0, nin, a.W1, a.A1, a.strips + 2, amx);
       finish_reduce(f2, amx, 0.0, dtm, bits, cur);
-      if (!(go = lr_sync(a, target))) break;
+      if (!(go = lr_sync(a, target, a.limit_ns))) break;
       // stage 3: U3 = 1/3 U + 2/3 (U2 + L(U2)); then the chemistry of the own cells
       amx = 0.0;
       bits = line_tile<3, V, LR_NT, S>(m, g, a.W1, a.A1, U, a.W0, jb_fin_cell(a.A0, nullptr, -1, 0), a.strips + 2,
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
       }
       lr_strips(m, g, x0, nin, a.U_out, a.aux_out, a.strips, amx);
       finish_reduce(f4, amx, 0.0, dtm, bits | (st << 16), cur);
-      go = lr_sync(a, target);
+      go = lr_sync(a, target, a.limit_ns);
     } else {
       unsigned bits = 0, st = 0;
       double amx = 0.0, amy = 0.0, dtm = inf;
@@ -184,26 +187,26 @@ __global__ void __launch_bounds__(LR_NT, 3)
           select_cell<1, true, true, false>(m, g, Us, nullptr, a.cand, As, a.strips, cur, __ldcg(&cur->mask[midx]), c,
                                             amx, amy, dtm, st);
         block_reduce_store(amx, 0.0, inf, st << 16, cur, aidx, true, false, -1);
-        return lr_sync(a, target);
+        return lr_sync(a, target, a.limit_ns);
       };
       // stage 1: U1 = U + L(U)
       bits = line_tile<1, V, LR_NT, S>(m, g, U, aux, U, a.W0, jb_fin_cand(a.cand, 0), a.strips,
                                        bitsd(__ldcg(&prv->ax[3])), dt, x0, smraw, amx, dtm, cur);
       finish_reduce(jb_fin_cand(a.cand, 0), 0.0, 0.0, inf, bits, cur);
-      if (!(go = lr_sync(a, target))) break;
+      if (!(go = lr_sync(a, target, a.limit_ns))) break;
       if (blockIdx.x == 0 && tid == 0) lr_clear(prv);  // every CTA has read it
       if (!(go = select(a.W0, a.A0, 0, 1))) break;
       // stage 2: U2 = 3/4 U + 1/4 (U1 + L(U1))
       bits = line_tile<2, V, LR_NT, S>(m, g, a.W0, a.A0, U, a.W1, jb_fin_cand(a.cand, 1), a.strips,
                                        bitsd(__ldcg(&cur->ax[1])), dt, x0, smraw, amx, dtm, cur);
       finish_reduce(jb_fin_cand(a.cand, 1), 0.0, 0.0, inf, bits, cur);
-      if (!(go = lr_sync(a, target))) break;
+      if (!(go = lr_sync(a, target, a.limit_ns))) break;
       if (!(go = select(a.W1, a.A1, 1, 2))) break;
       // stage 3: U3 = 1/3 U + 2/3 (U2 + L(U2))
       bits = line_tile<3, V, LR_NT, S>(m, g, a.W1, a.A1, U, a.W0, jb_fin_cand(a.cand, 2), a.strips,
                                        bitsd(__ldcg(&cur->ax[2])), dt, x0, smraw, amx, dtm, cur);
       finish_reduce(jb_fin_cand(a.cand, 2), 0.0, 0.0, inf, bits, cur);
-      if (!(go = lr_sync(a, target))) break;
+      if (!(go = lr_sync(a, target, a.limit_ns))) break;
       // chemistry at the selected stage-3 iterate
       bits = st = 0;
       const long long n3 = halley_count(__ldcg(&cur->mask[2])) * nc;
@@ -215,7 +218,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
                                               bits, st, amx, amy, dtm, nullptr);
       }
       finish_reduce(jb_fin_cand(a.cand, 3), 0.0, 0.0, inf, bits | (st << 16), cur);
-      if (!(go = lr_sync(a, target))) break;
+      if (!(go = lr_sync(a, target, a.limit_ns))) break;
       amx = 0.0;
       dtm = inf;
       st = 0;
@@ -223,7 +226,7 @@ __global__ void __launch_bounds__(LR_NT, 3)
         select_cell<1, true, true, true>(m, g, a.U_out, nullptr, a.cand, a.aux_out, a.strips, cur,
                                          __ldcg(&cur->mask[3]), c, amx, amy, dtm, st);
       block_reduce_store(amx, 0.0, dtm, st << 16, cur, 3, true, use_cfl, -1);
-      go = lr_sync(a, target);
+      go = lr_sync(a, target, a.limit_ns);
     }
   }
   __shared__ int s_gone;
@@ -304,7 +307,9 @@ static bool line_run_t(const MP& m, const Grid& g, const jb_line_io& io, cudaStr
   a.slots = io.slots; a.sets = io.slots + 1; a.bar = io.bar;
   a.dt_fixed = io.dt_fixed; a.cfl = io.cfl; a.nsteps = io.nsteps; a.dt_hist = io.dt_hist;
   a.count0 = io.count0;
-  a.limit_ns = io.wait_ms > 0.0 ? (unsigned long long)(io.wait_ms * 1e6) : LR_LIMIT_NS;
+  const unsigned long long ns = (unsigned long long)(io.wait_ms * 1e6);
+  a.start_ns = ns ? ns : LR_START_NS;
+  a.limit_ns = ns ? ns : LR_LIMIT_NS;
   return lr_try<V, 32>(m, g, a, io, st, err) || lr_try<V, 58>(m, g, a, io, st, err) ||
          lr_try<V, 122>(m, g, a, io, st, err);
 }

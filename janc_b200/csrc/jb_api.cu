@@ -181,9 +181,17 @@ int jb_create(const jb_mech_params* mech, int dim, int nx, int ny, double dx, do
   for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&h->auxw[i], bytes_aux);
   // 2D sweeps (jb_sweep.cuh): the primitives of the stage state, float64 in
   // fp64; in mixed float32, and those of the state being written (two buffers
-  // used in turn); behind the iterates in their allocation
-  const size_t bytes_fwork = dim != 2 || precision == JB_PREC_STRICT ? 0 : 24 * nc;
-  if (e == cudaSuccess) e = cudaMalloc(&h->cand, bytes_cand + bytes_fwork);
+  // used in turn); behind the iterates in their allocation.  A grid that fits
+  // the device only without them takes the tile kernels.
+  size_t bytes_fwork = dim != 2 || precision == JB_PREC_STRICT ? 0 : 24 * nc;
+  if (e == cudaSuccess) {
+    e = cudaMalloc(&h->cand, bytes_cand + bytes_fwork);
+    if (e == cudaErrorMemoryAllocation && bytes_fwork) {
+      (void)cudaGetLastError();
+      bytes_fwork = 0;
+      e = cudaMalloc(&h->cand, bytes_cand);
+    }
+  }
   if (bytes_fwork) h->fwork = h->cand + JB_NCAND * nc;
   if (e == cudaSuccess) e = cudaMalloc(&h->strips, bytes_strip);
   const size_t bytes_slots = 3 * sizeof(jb_slots) + 16 * sizeof(unsigned);

@@ -274,6 +274,42 @@ def test_block_stage_matches_the_strict_build(bx, by):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_grid_that_fits_without_the_sweep_scratch(prec):
+    """A handle whose sweep scratch (24 bytes a cell) does not fit the device
+    any more is made without it and takes the tile kernels: the strict build's
+    fluxes and steps all the same.  Torch holds the rest of the memory
+    meanwhile, but for what such a handle takes and half of the scratch."""
+    from janc_b200 import mechanism as jm
+    from janc_b200.solver import Solver
+    nx, ny, d = 1024, 1024, 1e-4
+    b = dict(zip(KEYS, BCS["walls"]))
+    mk = lambda p: Solver(2, nx, ny, d, d, b, jm.load(), precision=p)  # noqa: E731
+    s0 = mk("fp64_strict")
+    U, aux = _state(s0, (nx, ny))
+    ref = s0.advance(U, aux, 1, dt=1e-9)
+    whole = mk(prec)
+    bytes_whole = whole._lib.jb_workspace_bytes(whole._h)
+    del whole
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    keep = bytes_whole - 12 * nx * ny
+    fill = [torch.empty(torch.cuda.mem_get_info()[0] - keep, dtype=torch.uint8, device="cuda")]
+    try:
+        s1 = mk(prec)
+    finally:
+        fill.clear()
+        torch.cuda.empty_cache()
+    assert s1._lib.jb_workspace_bytes(s1._h) == bytes_whole - 24 * nx * ny
+    _check_flux(s0, s1, U, aux, None, d, prec)
+    for x, y in zip(s1.advance(U, aux, 1, dt=1e-9)[:2], ref[:2]):
+        for f in range(x.shape[0]):
+            tol = 1e-11 if prec == "fp64" else 1e-4
+            assert float((x[f] - y[f]).abs().sum()) <= tol * float(y[f].abs().sum()), f
+    assert s1.status() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["range", "mantissas", "edges"])
 def test_reciprocal_is_within_two_ulp(kind):
     """rcp_nr, which the fast builds take for pivots, concentrations,

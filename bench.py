@@ -81,12 +81,15 @@ BYTES_FLUX_STAGE_PER_CELL = 288  # one RK stage of the fused minimum: (224 + 320
 # DRAM bytes per cell measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum,
 # each launch cold) on the 1024x256 channel, mixed precision, with this tree's
 # kernels: one RK stage 2/3 (k_sweep_x 27.35 + 0.00 MB, k_flux_y 67.19 +
-# 0.77 MB) and one chemistry launch (27.37 + 0.73 MB); the capture and its
-# command are in profiles/launches_channel1024x256_mixed.md.  Per cell-step of
+# 0.97 MB) and one chemistry launch (27.37 + 0.92 MB).  Stores that are still
+# in L2 when a launch ends are not in these figures (k_flux_y stores 29 MB);
+# on the 1600x1000 annulus, whose state does not fit L2, a stage moves 509 and
+# the chemistry 226 bytes a cell, stores included.  The captures and their
+# commands are in profiles/launches_channel1024x256_mixed.md.  Per cell-step of
 # the persistent ensemble kernel: profiles/k_ensemble_64tubes.md.
-TRAFFIC_PER_CELL = {"flux": 363.6, "chem": 107.2}
+TRAFFIC_PER_CELL = {"flux": 364.3, "chem": 107.9}
 TRAFFIC_SOURCE = "profiles/launches_channel1024x256_mixed.md"
-TRAFFIC_ENS_PER_CELL_STEP = 764.0
+TRAFFIC_ENS_PER_CELL_STEP = 638.8
 
 
 ENS_N, ENS_SEED, ENS_CFL = 64, 4, 0.1
@@ -620,7 +623,8 @@ def run_ours(args):
                                  args.flux == "LF" and args.recon == "WENO5_JS" and not args.viscous and
                                  args.precision == "mixed" else None),
                      "traffic_source": "ncu dram bytes of one stage's launches on this workload, each "
-                                       "launch cold (mixed precision): " + TRAFFIC_SOURCE,
+                                       "launch cold, without the stores still in L2 at its end (mixed "
+                                       "precision): " + TRAFFIC_SOURCE,
                      "peak_source": hbm_src,
                      "algorithmic_bytes_per_cell": bytes_cell, "launch_ms": launch_ms,
                      "step_achieved_gbs": step_gbs,
